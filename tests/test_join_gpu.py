@@ -278,3 +278,42 @@ def test_star_join_prepared_dimension(cuda, rows):
         assert got[1] == c == want[1]
         assert rel_close(got[0], want[0], 1e-9) or (c == 0 and got[0] is None)
         assert rel_close(got[0], s if c else None, 1e-6) or (c == 0 and got[0] is None)
+
+
+@pytest.mark.parametrize("kind", [A.INT32, A.INT64, A.DATETIME, A.FLOAT32, A.FLOAT64])
+@pytest.mark.parametrize("nullable", [False, True])
+@pytest.mark.parametrize("L,R,distinct", [(1, 8193, 4000), (1025, 8193, 16000), (2049, 12001, 300), (700, 9000, 3)])
+def test_join_long_right_side(cuda, kind, nullable, L, R, distinct):
+    """Right sides beyond the shared-memory table (sorted key + hash of its
+    distinct keys): keys that repeat from never to a few thousand times (runs
+    longer than a warp and than a tile's output chunk), NULLs, NaN (joins
+    nothing) and -0.0 (equals +0.0), one condition and a residual one."""
+    rng = np.random.default_rng(L + R + distinct + kind)
+    dt = {A.INT32: np.int32, A.FLOAT32: np.float32, A.FLOAT64: np.float64}.get(kind, np.int64)
+    values = rng.integers(-distinct, distinct, distinct).astype(dt)
+    if kind in (A.INT64, A.DATETIME):
+        values = values * np.int64(3_000_000_019)
+    if kind in (A.FLOAT32, A.FLOAT64):
+        values[0], values[1 % distinct], values[2 % distinct] = np.nan, -0.0, 0.0
+    side = []
+    for n in (L, R):
+        txt = datagen.text_slots([f"row{i % 7}" for i in range(n)])
+        side.append(([values[rng.integers(0, distinct, n)], rng.integers(-50, 50, n).astype(np.int32), txt],
+                     [(rng.random(n) < 0.1) if nullable else None, None, None]))
+    (lc, ln), (rc, rn) = side
+    lb = ops.DeviceBatch([dev_col(c, kind if i == 0 else None, n) for i, (c, n) in enumerate(zip(lc, ln))])
+    rb = ops.DeviceBatch([dev_col(c, kind if i == 0 else None, n) for i, (c, n) in enumerate(zip(rc, rn))])
+    # a NaN key joins nothing, as a NULL does (the oracle has no rule for NaN conditions)
+    never = [[(n[0] if nullable else np.zeros(len(c[0]), bool)) | (c[0] != c[0]), None, None] for c, n in side]
+    for conds in ([(0, 0, A.EQ)], [(1, 1, A.GT), (0, 0, A.EQ)]):
+        wl, wr = oracle.join_pairs(lc, rc, conds, *never)
+        gl, gr = pairs_np(*ops.join_pairs(lb, rb, conds))
+        np.testing.assert_array_equal(gl, wl)
+        np.testing.assert_array_equal(gr, wr)
+        out = ops.join_project(lb, rb, conds, [(1, 2), (0, 1)])
+        np.testing.assert_array_equal(out.columns[0].data.cpu().numpy(), rc[2][wr])
+        np.testing.assert_array_equal(out.columns[1].data.cpu().numpy(), lc[1][wl])
+        if len(wl) > 1:  # too little room: refused, with the exact count
+            with pytest.raises(A.YQError) as e:
+                ops.join_pairs(lb, rb, conds, capacity=len(wl) - 1)
+            assert e.value.status == A.ERR_CAPACITY

@@ -16,6 +16,8 @@
 //    stably ordered hash table that every block copies into shared memory;
 //    each left row probes its bucket, checks the remaining conditions, counts,
 //    and after a decoupled look-back over tiles writes its pairs;
+//    A longer right side is sorted by its key and probed through a hash table
+//    of its distinct keys in global memory;
 //  - nested-loop path: a warp per left row sweeps the right rows 32 at a time,
 //    ballots the matches and appends them with popc offsets (coalesced);
 //  - no condition: the cross product is written directly, left-major.
@@ -163,6 +165,8 @@ __device__ __forceinline__ void copy_cell_j(char* dst, const char* src, int widt
   else if (width == 8)
     *reinterpret_cast<unsigned long long*>(dst) = __ldg(reinterpret_cast<const unsigned long long*>(src));
   else if (width == 1) *dst = *src;
+  else if (((width | reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src)) & 15) == 0)
+    for (int i = 0; i < width; i += 16) *reinterpret_cast<uint4*>(dst + i) = ldg_nc_v4(src + i);
   else
     for (int i = 0; i < width; i += 4)
       *reinterpret_cast<uint32_t*>(dst + i) = __ldg(reinterpret_cast<const uint32_t*>(src + i));
@@ -355,6 +359,226 @@ __global__ void __launch_bounds__(kJoinBlock) k_join_hash(const __grid_constant_
   if (tile == gridDim.x - 1 && threadIdx.x == 0) *J.total = s_prefix + total;
 }
 
+// --------------------------------------- equality probing, long right sides
+// A right side too long for a shared-memory table is sorted once by its key
+// (the stable radix sort, so rows of one key are contiguous and ascending) and
+// a hash table in global memory maps each distinct key to its first sorted
+// position. A probe costs three dependent reads that L2 serves (slot, key,
+// next key) whatever the right side's length, and a key's repeats are a
+// contiguous run, so the outputs of a tile are written position by position
+// by all its threads (coalesced, and one left row with many matches does not
+// serialise a thread). The nested loop this replaces compares every pair:
+// 2M x 300K INT32 rows took 303 ms, this takes 0.3 ms.
+struct SortedJoin {
+  const uint32_t* perm;           // right rows in key order
+  unsigned long long* skey;       // key of every sorted position
+  uint32_t* slots;                // hash table: first sorted position of a key (kNoSlot: empty)
+  uint32_t* nvalid;               // sorted positions before the NaN and NULL keys (they never join)
+  uint32_t nslots;                // power of two, >= 2 R
+};
+constexpr uint32_t kNoSlot = 0xffffffffu;
+
+__device__ __forceinline__ bool key_joins(const JCol& c, uint32_t row) {
+  if (cell_null(c, row)) return false;
+  if (c.type == YQ_FLOAT32) return !isnan(__uint_as_float((uint32_t)cell_u64(c, row)));
+  if (c.type == YQ_FLOAT64) return !isnan(__longlong_as_double((long long)cell_u64(c, row)));
+  return true;
+}
+
+__global__ void __launch_bounds__(256) k_join_sorted_build(const __grid_constant__ SortedJoin S, const JCol key,
+                                                           uint32_t R, const uint32_t* sort_err, uint32_t* err) {
+  if (blockIdx.x == 0 && threadIdx.x == 0 && *sort_err) atomicOr(err, *sort_err);
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < R; i += gridDim.x * blockDim.x) {
+    const uint32_t row = __ldg(S.perm + i);
+    if (row >= R) {  // a failed sort left no permutation
+      atomicOr(err, kErrBounds);
+      continue;
+    }
+    const uint64_t k = hash_key(key, row);
+    S.skey[i] = k;
+    if (!key_joins(key, row)) continue;
+    if (i + 1 == R || !key_joins(key, min(__ldg(S.perm + i + 1), R - 1u))) *S.nvalid = i + 1;
+    if (i > 0 && hash_key(key, min(__ldg(S.perm + i - 1), R - 1u)) == k) continue;
+    uint32_t h = hash_bucket(k, S.nslots);  // keys are distinct here: the first empty slot is this key's
+    for (uint32_t n = 0; n < S.nslots; ++n, h = (h + 1u) & (S.nslots - 1u))
+      if (atomicCAS(S.slots + h, kNoSlot, i) == kNoSlot) break;
+  }
+}
+
+// First sorted position and run length of the keys equal to left row l's.
+__device__ __forceinline__ uint32_t sorted_matches(const SortedJoin& S, uint32_t nvalid, const JCol& key, uint32_t l,
+                                                   uint32_t& first) {
+  first = 0;
+  if (!key_joins(key, l)) return 0u;
+  const uint64_t k = hash_key(key, l);
+  uint32_t h = hash_bucket(k, S.nslots);
+  uint32_t p = kNoSlot;
+  for (uint32_t n = 0; n < S.nslots; ++n, h = (h + 1u) & (S.nslots - 1u)) {
+    p = __ldg(S.slots + h);
+    if (p == kNoSlot || __ldg(S.skey + p) == k) break;
+  }
+  if (p == kNoSlot || p >= nvalid) return 0u;
+  first = p;
+  uint32_t step = 1;  // run end: doubling steps, then a binary search inside the last one
+  while (p + step < nvalid && __ldg(S.skey + p + step) == k) step <<= 1;
+  uint32_t lo = p + (step >> 1), hi = min(p + step, nvalid);  // key at lo matches; hi is past the run
+  while (lo + 1 < hi) {
+    const uint32_t mid = lo + ((hi - lo) >> 1);
+    if (__ldg(S.skey + mid) == k) lo = mid;
+    else hi = mid;
+  }
+  return lo + 1u - p;
+}
+
+__device__ __forceinline__ void write_col(const JOut& w, unsigned long long pos, uint32_t row) {
+  copy_cell_j(w.dst + (size_t)pos * w.width, w.src + (size_t)row * w.width, w.width);
+  if (w.dst_nulls) w.dst_nulls[pos] = w.src_nulls ? w.src_nulls[row] : 0;
+}
+
+constexpr uint32_t kSortedChunk = 2048;  // outputs resolved to (left, right) rows at a time
+
+// EQ_ONLY: the equality is the only condition, so a left row's matches are its
+// key's run. Otherwise the run's rows are candidates: a lane tests a short run
+// itself, the whole warp a long one.
+template <bool EQ_ONLY>
+__global__ void __launch_bounds__(kJoinBlock) k_join_sorted(const __grid_constant__ JoinParams J,
+                                                            const __grid_constant__ SortedJoin S) {
+  __shared__ uint32_t s_tile;
+  __shared__ uint32_t s_warp[kJoinBlock / 32 + 1];
+  __shared__ unsigned long long s_prefix;
+  __shared__ uint32_t s_off[kJoinTile + 1];
+  __shared__ uint32_t s_first[kJoinTile];
+  __shared__ uint32_t s_l[kSortedChunk], s_r[kSortedChunk];
+  if (threadIdx.x == 0) s_tile = atomicAdd(J.tile_counter, 1u);
+  __syncthreads();
+  const uint32_t tile = s_tile;
+  const uint32_t base = tile * kJoinTile;
+  const uint32_t nvalid = *S.nvalid;
+  const JCond& ec = J.cond[J.eq];
+  const int lane = threadIdx.x & 31;
+  uint32_t first[kJoinItems], run[kJoinItems], cnt[kJoinItems], sum = 0;
+#pragma unroll
+  for (int k = 0; k < kJoinItems; ++k) {
+    const uint32_t l = base + threadIdx.x * kJoinItems + k;
+    first[k] = 0;
+    run[k] = l < J.L ? sorted_matches(S, nvalid, ec.l, l, first[k]) : 0u;
+    cnt[k] = run[k];
+  }
+  if constexpr (!EQ_ONLY) {
+#pragma unroll 1
+    for (int k = 0; k < kJoinItems; ++k) {
+      const uint32_t l = base + threadIdx.x * kJoinItems + k;
+      cnt[k] = 0;
+      if (run[k] <= 32)
+        for (uint32_t x = 0; x < run[k]; ++x) cnt[k] += all_conds(J, l, __ldg(S.perm + first[k] + x), J.eq) ? 1u : 0u;
+      for (uint32_t todo = __ballot_sync(0xffffffffu, run[k] > 32); todo; todo &= todo - 1) {
+        const int src = __ffs(todo) - 1;
+        const uint32_t n = __shfl_sync(0xffffffffu, run[k], src), f = __shfl_sync(0xffffffffu, first[k], src);
+        const uint32_t wl = __shfl_sync(0xffffffffu, l, src);
+        uint32_t c = 0;
+        for (uint32_t x = lane; x < ((n + 31u) & ~31u); x += 32) {
+          const bool m = x < n && all_conds(J, wl, __ldg(S.perm + f + x), J.eq);
+          c += __popc(__ballot_sync(0xffffffffu, m));
+        }
+        if (lane == src) cnt[k] = c;
+      }
+    }
+  }
+  unsigned long long wide = 0;  // the tile's pairs may exceed 32 bits (a hot key on both sides)
+#pragma unroll
+  for (int k = 0; k < kJoinItems; ++k) {
+    wide += cnt[k];
+    sum += cnt[k];
+  }
+  const int huge = __syncthreads_or(wide > 0xfffffu);  // 256 sums below 2^20 fit a 32-bit scan
+  unsigned long long total;
+  unsigned long long excl;
+  if (!huge) {
+    uint32_t t32;
+    excl = block_exclusive_sum<kJoinBlock>(sum, s_warp, t32);
+    total = t32;
+  } else {
+    __shared__ unsigned long long s_wide[2 * (kJoinBlock / 32 + 1)];
+    unsigned long long a = wide, b = 0, tb;
+    block_exclusive_sum2<kJoinBlock>(a, b, s_wide, total, tb);
+    excl = a;
+  }
+  if (threadIdx.x < 32) {
+    const unsigned long long p = tile_lookback(J.status, tile, total, J.err);
+    if (threadIdx.x == 0) s_prefix = p;
+  }
+  __syncthreads();
+  const unsigned long long prefix = s_prefix;
+  if (tile == gridDim.x - 1 && threadIdx.x == 0) *J.total = prefix + total;
+  if (prefix >= J.capacity || total == 0) return;  // nothing of this tile is stored
+  if (EQ_ONLY && !huge) {
+    uint32_t at = (uint32_t)excl;
+#pragma unroll
+    for (int k = 0; k < kJoinItems; ++k) {
+      s_off[threadIdx.x * kJoinItems + k] = at;
+      s_first[threadIdx.x * kJoinItems + k] = first[k];
+      at += cnt[k];
+    }
+    if (threadIdx.x == 0) s_off[kJoinTile] = (uint32_t)total;
+    const unsigned long long room = J.capacity - prefix;
+    const uint32_t n_out = total < room ? (uint32_t)total : (uint32_t)room;
+    for (uint32_t c0 = 0; c0 < n_out; c0 += kSortedChunk) {
+      const uint32_t n = min(kSortedChunk, n_out - c0);
+      __syncthreads();
+      for (uint32_t i = threadIdx.x; i < n; i += kJoinBlock) {
+        uint32_t lo = 0, hi = kJoinTile;  // the left row whose outputs hold position c0 + i
+        while (lo + 1 < hi) {
+          const uint32_t mid = (lo + hi) >> 1;
+          if (s_off[mid] <= c0 + i) lo = mid;
+          else hi = mid;
+        }
+        s_l[i] = base + lo;
+        s_r[i] = __ldg(S.perm + s_first[lo] + (c0 + i - s_off[lo]));
+      }
+      __syncthreads();
+      const unsigned long long p0 = prefix + c0;
+      if (J.nout == 0) {
+        for (uint32_t i = threadIdx.x; i < n; i += kJoinBlock) {
+          J.out_left[p0 + i] = s_l[i];
+          J.out_right[p0 + i] = s_r[i];
+        }
+      } else {
+        for (int o = 0; o < J.nout; ++o) {
+          const JOut& w = J.out[o];
+          const uint32_t* rows = w.side ? s_r : s_l;
+          for (uint32_t i = threadIdx.x; i < n; i += kJoinBlock) write_col(w, p0 + i, rows[i]);
+        }
+      }
+    }
+    return;
+  }
+  unsigned long long pos = prefix + excl;
+#pragma unroll 1
+  for (int k = 0; k < kJoinItems; ++k) {
+    const uint32_t l = base + threadIdx.x * kJoinItems + k;
+    if (run[k] <= 32) {
+      for (uint32_t x = 0; x < run[k]; ++x) {
+        const uint32_t r = __ldg(S.perm + first[k] + x);
+        if (EQ_ONLY || all_conds(J, l, r, J.eq)) emit_pair(J, pos++, l, r);
+      }
+    }
+    for (uint32_t todo = __ballot_sync(0xffffffffu, run[k] > 32); todo; todo &= todo - 1) {
+      const int src = __ffs(todo) - 1;
+      const uint32_t n = __shfl_sync(0xffffffffu, run[k], src), f = __shfl_sync(0xffffffffu, first[k], src);
+      const uint32_t wl = __shfl_sync(0xffffffffu, l, src);
+      unsigned long long wp = __shfl_sync(0xffffffffu, pos, src);
+      for (uint32_t x = lane; x < ((n + 31u) & ~31u); x += 32) {
+        const uint32_t r = x < n ? __ldg(S.perm + f + x) : 0u;
+        const bool m = x < n && (EQ_ONLY || all_conds(J, wl, r, J.eq));
+        const uint32_t bal = __ballot_sync(0xffffffffu, m);
+        if (m) emit_pair(J, wp + __popc(bal & lanemask_lt()), wl, r);
+        wp += __popc(bal);
+      }
+      if (lane == src) pos = wp;
+    }
+  }
+}
+
 // ------------------------------------------------------------ nested loop
 constexpr int kNlRowsPerWarp = 4;
 constexpr uint32_t kNlTile = (kJoinBlock / 32) * kNlRowsPerWarp;  // left rows per block
@@ -475,7 +699,6 @@ __global__ void k_join_count_sorted(const T* __restrict__ lcol, uint32_t L, cons
       else if constexpr (OP == YQ_LE) c = nvalid - lb;
       else if constexpr (OP == YQ_GT) c = lb;
       else if constexpr (OP == YQ_GE) c = ub;
-      else if constexpr (OP == YQ_EQ) c = ub - lb;
       else c = R - (ub - lb);
     }
     counts[l] = c;
@@ -745,11 +968,12 @@ static int build_table(const yq_batch* right, const yq_program* pred, const yq_c
 // binary searches per left row, instead of a comparison pass over L x R.
 constexpr uint32_t kCountFirstRows = 4096;
 
-// Sort workspace for a right side of R rows (an 8-byte key bounds the typed
-// path's 4- and 8-byte keys). Sizing reads no column data: the placeholder
-// pointer only has to be non-null.
-static size_t count_sort_bytes(uint32_t R) {
-  yq_column dummy{reinterpret_cast<void*>(static_cast<uintptr_t>(256)), nullptr, YQ_INT64, 8};
+// Sort workspace for a right side of R rows (an 8-byte key, nullable or not,
+// bounds the 4-byte ones). Sizing reads no column data: the placeholder
+// pointers only have to be non-null.
+static size_t join_sort_bytes(uint32_t R, bool nullable) {
+  const uintptr_t some = 256;
+  yq_column dummy{reinterpret_cast<void*>(some), nullable ? reinterpret_cast<const uint8_t*>(some) : nullptr, YQ_INT64, 8};
   KeyJob j{dummy, 0, 0};
   uint32_t offs[2] = {0, R};
   size_t sb = 0;
@@ -774,6 +998,14 @@ static void count_ws_layout(uint32_t L, uint32_t R, size_t sort_bytes, WsSize& w
   w.add<uint32_t>(L ? L : 1);
 }
 
+static void sorted_ws_layout(uint32_t R, size_t sort_bytes, WsSize& w) {
+  w.add<char>(sort_bytes);
+  w.add<uint32_t>(R);
+  w.add<unsigned long long>(R);
+  w.add<uint32_t>(4);
+  w.add<uint32_t>((size_t)pow2_at_least(R) * 2);
+}
+
 template <typename T>
 static int count_matches_typed(const JoinParams& J, const CountWs& c, cudaStream_t s) {
   const JCond& c0 = J.cond[0];
@@ -795,7 +1027,6 @@ static int count_matches_typed(const JoinParams& J, const CountWs& c, cudaStream
     case YQ_LE: k_join_count_sorted<T, YQ_LE><<<grid, 256, 0, s>>>(lcol, J.L, sorted, c.nvalid, R, c.counts); break;
     case YQ_GT: k_join_count_sorted<T, YQ_GT><<<grid, 256, 0, s>>>(lcol, J.L, sorted, c.nvalid, R, c.counts); break;
     case YQ_GE: k_join_count_sorted<T, YQ_GE><<<grid, 256, 0, s>>>(lcol, J.L, sorted, c.nvalid, R, c.counts); break;
-    case YQ_EQ: k_join_count_sorted<T, YQ_EQ><<<grid, 256, 0, s>>>(lcol, J.L, sorted, c.nvalid, R, c.counts); break;
     default: k_join_count_sorted<T, YQ_NE><<<grid, 256, 0, s>>>(lcol, J.L, sorted, c.nvalid, R, c.counts); break;
   }
   YQ_CHECK_LAUNCH();
@@ -881,51 +1112,56 @@ static int join_impl(const yq_batch* left, const yq_batch* right, const yq_join_
     return n > capacity ? YQ_ERR_CAPACITY : YQ_OK;
   }
 
+  // The sorted table holds any length the sort takes. BOOL keys stay with the
+  // other paths: the sort orders every non-zero byte as one value, a join
+  // compares the bytes.
   const bool use_hash = J.eq >= 0 && J.R <= kHashMaxRows;
+  const size_t eq_sort_bytes =
+      J.eq >= 0 && !use_hash && J.cond[J.eq].r.type != YQ_BOOL ? join_sort_bytes(J.R, J.cond[J.eq].r.nulls != nullptr) : 0;
+  const bool use_sorted = eq_sort_bytes != 0;
   const uint32_t nbuckets = use_hash ? pow2_at_least(J.R) : 0u;
-  const uint32_t ntiles = use_hash ? ceil_div<uint32_t>(J.L, kJoinTile) : ceil_div<uint32_t>(J.L, kNlTile);
+  const uint32_t ntiles = ceil_div<uint32_t>(J.L, use_hash || use_sorted ? kJoinTile : kNlTile);
   const JCond& t0 = J.cond[0];
-  const bool typed = !use_hash && J.ncond == 1 && J.ngroups == 1 && t0.l.type == t0.r.type && !t0.l.nulls &&
+  const bool typed = !use_hash && !use_sorted && J.ncond == 1 && J.ngroups == 1 && t0.l.type == t0.r.type && !t0.l.nulls &&
                      !t0.r.nulls && t0.l.width == t0.r.width &&
                      (t0.l.type == YQ_INT32 || t0.l.type == YQ_FLOAT32 || t0.l.type == YQ_INT64 ||
                       t0.l.type == YQ_DATETIME || t0.l.type == YQ_FLOAT64);
-  const size_t sort_bytes = typed && J.R >= kCountFirstRows ? count_sort_bytes(J.R) : 0;
-  const bool count_first = sort_bytes != 0;  // else (a right side too long to sort) the kernel counts
+  const size_t count_bytes = typed && J.R >= kCountFirstRows ? join_sort_bytes(J.R, false) : 0;
+  const bool count_first = count_bytes != 0;  // else (a right side too long to sort) the kernel counts
   WsSize w;
   w.add<uint32_t>(nbuckets + 1);
   w.add<unsigned long long>(use_hash ? J.R : 1);
   w.add<uint32_t>(use_hash ? J.R : 1);
-  w.add<unsigned long long>((size_t)ntiles + 1);
+  w.add<unsigned long long>((size_t)ntiles + 3);
   w.add<uint32_t>(8);
-  w.add<unsigned long long>(2);
-  if (count_first) count_ws_layout(J.L, J.R, sort_bytes, w);
+  if (count_first) count_ws_layout(J.L, J.R, count_bytes, w);
+  if (use_sorted) sorted_ws_layout(J.R, eq_sort_bytes, w);
   Workspace ws;
   YQ_TRY(ws.acquire(workspace, workspace_bytes, w.total(), s));
   uint32_t* d_bstart = ws.take<uint32_t>(nbuckets + 1);
   unsigned long long* d_hkeys = ws.take<unsigned long long>(use_hash ? J.R : 1);
   uint32_t* d_hrows = ws.take<uint32_t>(use_hash ? J.R : 1);
-  J.status = ws.take<unsigned long long>((size_t)ntiles + 1);
-  uint32_t* d_misc = ws.take<uint32_t>(8);  // [0] tile counter [1] err [2..3] build counts
-  J.total = ws.take<unsigned long long>(2);
-  J.tile_counter = d_misc;
-  J.err = d_misc + 1;
+  J.status = ws.take<unsigned long long>((size_t)ntiles + 3);  // then [total][tile counter, err]
+  uint32_t* d_build = ws.take<uint32_t>(8);                    // [0..1] build counts
+  J.total = J.status + ntiles + 1;
+  J.tile_counter = reinterpret_cast<uint32_t*>(J.total + 1);
+  J.err = J.tile_counter + 1;
   CountWs cw{};
   if (count_first) {
-    cw.sort_ws = ws.take<char>(sort_bytes);
-    cw.sort_bytes = sort_bytes;
+    cw.sort_ws = ws.take<char>(count_bytes);
+    cw.sort_bytes = count_bytes;
     cw.perm = ws.take<uint32_t>(J.R ? J.R : 1);
     cw.sorted = reinterpret_cast<char*>(ws.take<unsigned long long>(J.R ? J.R : 1));
     cw.nvalid = ws.take<uint32_t>(4);
     cw.counts = ws.take<uint32_t>(J.L ? J.L : 1);
   }
-  YQ_TRY_CUDA(cudaMemsetAsync(J.status, 0, ((size_t)ntiles + 1) * sizeof(unsigned long long), s));
-  YQ_TRY_CUDA(cudaMemsetAsync(d_misc, 0, 8 * sizeof(uint32_t), s));
-  YQ_TRY_CUDA(cudaMemsetAsync(J.total, 0, 2 * sizeof(unsigned long long), s));
+  YQ_TRY_CUDA(cudaMemsetAsync(J.status, 0, ((size_t)ntiles + 3) * sizeof(unsigned long long), s));
   double out_row_bytes = nout == 0 ? 8.0 : 0.0;
   for (int o = 0; o < nout; ++o) out_row_bytes += J.out[o].width + (J.out[o].dst_nulls ? 1 : 0);
   if (use_hash) {
-    YQ_TRY(build_table(right, nullptr, nullptr, conds[J.eq].right_col, nbuckets, d_bstart, d_hkeys, d_hrows,
-                       d_misc + 2, s));
+    YQ_TRY_CUDA(cudaMemsetAsync(d_build, 0, 8 * sizeof(uint32_t), s));
+    YQ_TRY(build_table(right, nullptr, nullptr, conds[J.eq].right_col, nbuckets, d_bstart, d_hkeys, d_hrows, d_build,
+                       s));
     J.bstart = d_bstart;
     J.hkeys = d_hkeys;
     J.hrows = d_hrows;
@@ -935,6 +1171,35 @@ static int join_impl(const yq_batch* left, const yq_batch* right, const yq_join_
     YQ_TRY(kernel_allow_smem((const void*)k_join_hash, smem));
     ProfScope ps("join_hash_probe", s, (double)J.L * left->columns[conds[J.eq].left_col].width);
     k_join_hash<<<ntiles, kJoinBlock, smem, s>>>(J);
+    YQ_CHECK_LAUNCH();
+  } else if (use_sorted) {
+    const JCond& ec = J.cond[J.eq];
+    char* sort_ws = ws.take<char>(eq_sort_bytes);
+    uint32_t* perm = ws.take<uint32_t>(J.R);
+    SortedJoin S;
+    S.perm = perm;
+    S.skey = ws.take<unsigned long long>(J.R);
+    S.nvalid = ws.take<uint32_t>(4);
+    S.nslots = pow2_at_least(J.R) * 2u;
+    S.slots = ws.take<uint32_t>(S.nslots);
+    const yq_column rc{const_cast<char*>(ec.r.data), ec.r.nulls, ec.r.type, ec.r.width};
+    KeyJob j{rc, 0, 0};
+    uint32_t offs[2] = {0, J.R};
+    uint32_t* sort_err = nullptr;
+    YQ_TRY(sort_segments_impl(&j, 1, J.R, offs, 1, perm, nullptr, sort_ws, eq_sort_bytes, s, nullptr, nullptr, nullptr,
+                              true, &sort_err));
+    YQ_TRY_CUDA(cudaMemsetAsync(S.nvalid, 0, 4 * sizeof(uint32_t), s));
+    YQ_TRY_CUDA(cudaMemsetAsync(S.slots, 0xff, (size_t)S.nslots * sizeof(uint32_t), s));
+    int grid = (int)ceil_div<uint32_t>(J.R, 256);
+    if (grid > sm_count() * 8) grid = sm_count() * 8;
+    {
+      ProfScope ps("join_sorted_build", s, (double)J.R * ec.r.width);
+      k_join_sorted_build<<<grid, 256, 0, s>>>(S, ec.r, J.R, sort_err, J.err);
+      YQ_CHECK_LAUNCH();
+    }
+    ProfScope ps("join_sorted_probe", s, (double)J.L * ec.l.width);
+    if (J.ncond == 1) k_join_sorted<true><<<ntiles, kJoinBlock, 0, s>>>(J, S);
+    else k_join_sorted<false><<<ntiles, kJoinBlock, 0, s>>>(J, S);
     YQ_CHECK_LAUNCH();
   } else {
     ProfScope ps("join_nested_loop", s, (double)J.L * J.R * 0.0);
@@ -960,12 +1225,16 @@ static int join_impl(const yq_batch* left, const yq_batch* right, const yq_join_
     }
     YQ_CHECK_LAUNCH();
   }
-  unsigned long long h_total = 0;
-  uint32_t h_err = 0;
-  YQ_TRY(d2h_sync(&h_total, J.total, sizeof(h_total), s));
-  YQ_TRY(d2h_sync(&h_err, J.err, sizeof(h_err), s));
+  struct {
+    unsigned long long total;
+    uint32_t counter, err;
+  } h{};
+  YQ_TRY(d2h_sync(&h, J.total, sizeof(h), s));
+  const unsigned long long h_total = h.total;
+  const uint32_t h_err = h.err;
   if (count_host) *count_host = h_total;
   if (h_err & kErrTimeout) return YQ_ERR_TIMEOUT;
+  if (h_err & kErrBounds) return YQ_ERR_INVALID_ARG;
   return h_total > capacity ? YQ_ERR_CAPACITY : YQ_OK;
 }
 
@@ -982,11 +1251,12 @@ size_t yq_join_workspace_size(uint32_t left_rows, uint32_t right_rows) {
   w.add<uint32_t>(nb + 1);
   w.add<unsigned long long>(right_rows ? right_rows : 1);
   w.add<uint32_t>(right_rows ? right_rows : 1);
-  w.add<unsigned long long>((size_t)ntiles + 1);
+  w.add<unsigned long long>((size_t)ntiles + 3);
   w.add<uint32_t>(8);
-  w.add<unsigned long long>(2);
-  if (right_rows >= kCountFirstRows) count_ws_layout(left_rows, right_rows, count_sort_bytes(right_rows), w);
-  return w.total();
+  WsSize sorted = w;
+  if (right_rows >= kCountFirstRows) count_ws_layout(left_rows, right_rows, join_sort_bytes(right_rows, false), w);
+  if (right_rows > kHashMaxRows) sorted_ws_layout(right_rows, join_sort_bytes(right_rows, true), sorted);
+  return w.total() > sorted.total() ? w.total() : sorted.total();
 }
 
 int yq_join_pairs(const yq_batch* left, const yq_batch* right, const yq_join_cond* conds, int32_t ncond,
