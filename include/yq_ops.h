@@ -16,9 +16,10 @@
  *    All work is stream ordered. Calls that must return a host value (a row
  *    count, a status read back from the device) synchronise that stream and say so.
  *  - Scratch: calls that need device scratch take (`workspace`, `workspace_bytes`).
- *    Passing workspace == NULL makes the library allocate it stream-ordered with
- *    cudaMallocAsync on `stream` and release it with cudaFreeAsync after the
- *    launch. The matching `*_workspace_size` function reports the bytes needed.
+ *    Passing workspace == NULL makes the library allocate it stream-ordered on
+ *    `stream`, from a pool of its own per device that keeps at most 1/64 of the
+ *    device's memory between calls (yq_workspace_trim gives it back), and release
+ *    it with cudaFreeAsync after the launch. The matching `*_workspace_size` function reports the bytes needed.
  *  - Every function returns a yq_status; nothing calls exit() (the reference's
  *    CUDA_CHECK exits the process, include/utils/macros.hpp:6-22).
  *  - Every device wait inside a kernel (decoupled look-back, mbarrier waits) is
@@ -692,6 +693,10 @@ int yq_csv_format(const yq_batch* batch, uint8_t* out, uint64_t capacity, uint64
 /* ---------------------------------------------------------------- device */
 /* Number of SMs of the current device (cached per device). */
 int yq_device_sm_count(void);
+/* Gives the memory that the current device's workspace pool keeps and no call
+ * uses back to the driver (the library does so itself when an allocation
+ * fails; a host that allocates elsewhere calls it when it runs out). */
+int yq_workspace_trim(void);
 /* Kernel launches issued by this library on this process (for accounting). */
 uint64_t yq_launch_count(void);
 /* ---- Program-specialised row kernels.

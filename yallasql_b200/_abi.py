@@ -184,6 +184,7 @@ PROTOTYPES = {
     "yq_csv_format": (C.c_int, [P(Batch), vp, u64, P(u64), vp, sz, vp]),
     "yq_device_sm_count": (C.c_int, []),
     "yq_launch_count": (u64, []),
+    "yq_workspace_trim": (i32, []),
     "yq_profile_enable": (C.c_int, [i32]),
     "yq_jit_enable": (C.c_int, [i32]),
     "yq_jit_stats": (C.c_int, [P(i32), P(i32), P(i32), P(C.c_double), C.c_char_p, sz]),

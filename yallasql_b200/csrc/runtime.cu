@@ -151,6 +151,64 @@ int d2h_sync(void* host_dst, const void* dev_src, size_t bytes, cudaStream_t s) 
   return YQ_OK;
 }
 
+// ---------------------------------------------------------- workspace pool
+// Workspaces that the library allocates itself come from a pool of its own.
+// The device's default pool hands every free byte back to the driver at the
+// next synchronisation, so each call that ends with a read-back had its
+// workspace mapped anew: 0.44 ms for a 16K-row filter + aggregate that runs
+// 40 us on the GPU, 13 ms for a 32M-row GROUP BY's 1 GB. This pool keeps up to
+// 1/64 of the device's memory (2.8 GB of 180) across synchronisations, hands
+// back what is above that, and everything when the device runs out or
+// yq_workspace_trim is called. The driver orders reuse between streams.
+namespace {
+constexpr size_t kPoolShare = 64;
+std::mutex g_pool_mu;
+cudaMemPool_t g_pool[64] = {};
+bool g_pool_tried[64] = {};
+
+cudaMemPool_t workspace_pool(int dev) {
+  if (dev < 0 || dev >= 64) return nullptr;
+  std::lock_guard<std::mutex> lk(g_pool_mu);
+  if (g_pool_tried[dev]) return g_pool[dev];
+  g_pool_tried[dev] = true;
+  cudaMemPoolProps props;
+  memset(&props, 0, sizeof(props));
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = dev;
+  cudaDeviceProp prop;
+  cudaMemPool_t pool = nullptr;
+  if (cudaGetDeviceProperties(&prop, dev) == cudaSuccess && cudaMemPoolCreate(&pool, &props) == cudaSuccess) {
+    uint64_t keep = prop.totalGlobalMem / kPoolShare;
+    if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess) g_pool[dev] = pool;
+    else cudaMemPoolDestroy(pool);
+  }
+  if (!g_pool[dev]) cudaGetLastError();  // no pool: allocations take the default one
+  return g_pool[dev];
+}
+}  // namespace
+
+int pool_alloc(void** p, size_t bytes, cudaStream_t s) {
+  int dev = 0;
+  YQ_TRY_CUDA(cudaGetDevice(&dev));
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  YQ_TRY_CUDA(cudaStreamIsCapturing(s, &cap));
+  // a captured allocation belongs to the graph, not to a pool
+  cudaMemPool_t pool = cap == cudaStreamCaptureStatusNone ? workspace_pool(dev) : nullptr;
+  cudaError_t e = pool ? cudaMallocFromPoolAsync(p, bytes, pool, s) : cudaMallocAsync(p, bytes, s);
+  if (e == cudaErrorMemoryAllocation && pool) {
+    cudaGetLastError();
+    // Freed blocks become the driver's again once the work before their free
+    // is done; then the default pool may use them too.
+    if (cudaStreamSynchronize(s) == cudaSuccess && cudaMemPoolTrimTo(pool, 0) == cudaSuccess) e = cudaMallocAsync(p, bytes, s);
+  }
+  if (e != cudaSuccess) {
+    set_cuda_error(e);
+    return YQ_ERR_ALLOC;
+  }
+  return YQ_OK;
+}
+
 // ---------------------------------------------------------------- profiler
 namespace {
 struct ProfRec {
@@ -271,6 +329,13 @@ const char* yq_status_string(int status) {
 int yq_last_cuda_error(void) { return yq::g_last_cuda_error; }
 int yq_abi_version(void) { return YQ_ABI_VERSION; }
 int yq_device_sm_count(void) { return yq::sm_count(); }
+int yq_workspace_trim(void) {
+  int dev = 0;
+  YQ_TRY_CUDA(cudaGetDevice(&dev));
+  if (cudaMemPool_t pool = yq::workspace_pool(dev)) YQ_TRY_CUDA(cudaMemPoolTrimTo(pool, 0));
+  return YQ_OK;
+}
+
 uint64_t yq_launch_count(void) { return yq::g_launches.load(std::memory_order_relaxed); }
 
 int yq_profile_enable(int32_t on) {

@@ -97,6 +97,10 @@ __host__ __device__ inline T ceil_div(T a, T b) { return (a + b - 1) / b; }
 
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
+// Stream-ordered allocation from the library's workspace pool of the current
+// device (runtime.cu); freed with cudaFreeAsync on the same stream.
+int pool_alloc(void** p, size_t bytes, cudaStream_t s);
+
 // Bump allocator over one workspace region. When the caller passes no
 // workspace, `Workspace::acquire` allocates it stream-ordered and the
 // destructor frees it stream-ordered (cudaFreeAsync), so a call never blocks
@@ -118,11 +122,8 @@ struct Workspace {
     }
     if (need == 0) return YQ_OK;
     void* p = nullptr;
-    cudaError_t e = cudaMallocAsync(&p, need, s);
-    if (e != cudaSuccess) {
-      set_cuda_error(e);
-      return YQ_ERR_ALLOC;
-    }
+    const int st = pool_alloc(&p, need, s);
+    if (st != YQ_OK) return st;
     base = static_cast<char*>(p);
     bytes = need;
     owned = true;

@@ -24,6 +24,17 @@ static int32_t width_of(int32_t type, int32_t text_width = 16) {
   }
 }
 
+// Device allocation on the default pool; when the device is full, the operator
+// library's idle workspaces go back to the driver first.
+static cudaError_t device_alloc(void** p, size_t bytes, cudaStream_t s) {
+  cudaError_t e = cudaMallocAsync(p, bytes, s);
+  if (e == cudaErrorMemoryAllocation && yq_workspace_trim() == YQ_OK) {
+    cudaGetLastError();
+    e = cudaMallocAsync(p, bytes, s);
+  }
+  return e;
+}
+
 // ------------------------------------------------------------------ Batch
 Batch::Batch(std::vector<ColumnPtr> cols, uint64_t n, cudaStream_t s, bool with_nulls)
     : columns(std::move(cols)), rows(n), location(Device::GPU), stream(s) {
@@ -31,8 +42,8 @@ Batch::Batch(std::vector<ColumnPtr> cols, uint64_t n, cudaStream_t s, bool with_
   nulls.resize(columns.size(), nullptr);
   for (size_t c = 0; c < columns.size(); ++c) {
     const size_t b = std::max<uint64_t>(1, n) * columns[c]->width;
-    check_cuda(cudaMallocAsync(&data[c], b, s), "Batch alloc");
-    if (with_nulls) check_cuda(cudaMallocAsync(reinterpret_cast<void**>(&nulls[c]), std::max<uint64_t>(1, n), s),
+    check_cuda(device_alloc(&data[c], b, s), "Batch alloc");
+    if (with_nulls) check_cuda(device_alloc(reinterpret_cast<void**>(&nulls[c]), std::max<uint64_t>(1, n), s),
                                "Batch nulls alloc");
   }
 }
@@ -94,10 +105,10 @@ void Batch::cpuToGpu() {
     const size_t nb = std::max<uint64_t>(1, rows);
     void* p = nullptr;
     void* q = nullptr;
-    check_cuda(cudaMallocAsync(&p, b, stream), "reload alloc");
+    check_cuda(device_alloc(&p, b, stream), "reload alloc");
     check_cuda(cudaMemcpyAsync(p, data[c], b, cudaMemcpyHostToDevice, stream), "reload copy");
     if (nulls[c]) {
-      check_cuda(cudaMallocAsync(&q, nb, stream), "reload alloc");
+      check_cuda(device_alloc(&q, nb, stream), "reload alloc");
       check_cuda(cudaMemcpyAsync(q, nulls[c], nb, cudaMemcpyHostToDevice, stream), "reload copy");
     }
     check_cuda(cudaStreamSynchronize(stream), "reload sync");
