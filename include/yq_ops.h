@@ -336,21 +336,24 @@ int yq_merge_pass(const yq_column* cols, int32_t ncols, int32_t key_col,
  * (include/engine/operators/order_operator.hpp:89-193,
  *  src/engine/operators/order_operator.cpp:14-220): the rows of `in` arrive as
  * nruns sorted-on-arrival batches (run r = rows [run_offsets[r],
- * run_offsets[r+1]), host array). Every run is sorted by the segmented radix
- * sort, whose last pass also leaves each row's order-preserving key words;
- * the runs are then merged pairwise, level by level, as (key words, row id)
- * pairs by a persistent merge-path kernel that stages both windows of the
- * tiles ahead with 1-D bulk copies; finally every column is gathered once by
- * the merged row ids into `out` (same schema, at least in->rows rows).
- * Stable: equal keys keep their input order. The call waits for the device
- * once, at the end, to report errors.
+ * run_offsets[r+1]), host array). The runs lie back to back in device memory,
+ * so one stable radix sort of the whole table gives the order that sorting each
+ * run and merging the runs (ties to the earlier run) would give, without the
+ * merge levels; its last pass also leaves each row's order-preserving key
+ * words, from which the key column is written, and every other column is
+ * gathered once by the sorted row ids into `out` (same schema, at least
+ * in->rows rows). yq_order_by_tiled with a merge tile sorts the runs and merges
+ * them pairwise, level by level, as (key words, row id) pairs by a persistent
+ * merge-path kernel that stages both windows of the tiles ahead with 1-D bulk
+ * copies. Stable: equal keys keep their input order. The call waits for the
+ * device once, at the end, to report errors.
  *
- * With many runs over a table larger than L2 the gather goes in two levels
- * when the workspace allows (or the library allocates it): the columns are
- * first gathered run by run into sorted-run order, and the final gather then
- * reads every run's rows in increasing order. yq_order_by_workspace_size is
- * the least workspace (one-level gather); yq_order_by_batch_workspace_size
- * includes the sorted-run copy of the batch's columns. */
+ * On a table larger than L2 the gather goes through packed rows when the
+ * workspace allows (or the library allocates it): the narrow columns are first
+ * copied side by side into one record per row, so a row costs one random read
+ * instead of one per column. yq_order_by_workspace_size is the least workspace
+ * (columns gathered one by one); yq_order_by_batch_workspace_size includes the
+ * packed rows of the batch's columns. */
 size_t yq_order_by_workspace_size(const yq_column* key, uint32_t rows, const uint32_t* run_offsets,
                                   int32_t nruns);
 size_t yq_order_by_batch_workspace_size(const yq_batch* in, int32_t key_col, const uint32_t* run_offsets,
@@ -360,18 +363,18 @@ int yq_order_by(const yq_batch* in, int32_t key_col, int32_t descending, int32_t
                 size_t workspace_bytes, void* stream);
 /* yq_order_by with the merge-path tile given: merge_items outputs per
  * thread (4, 8 or 16; 16 needs a key of at most two words, else
- * YQ_ERR_UNSUPPORTED; 0 = the tuned or default choice). */
+ * YQ_ERR_UNSUPPORTED; 0 = no merge, as yq_order_by). */
 int yq_order_by_tiled(const yq_batch* in, int32_t key_col, int32_t descending, int32_t nulls_first,
                       const uint32_t* run_offsets, int32_t nruns, yq_batch* out, int32_t merge_items,
                       void* workspace, size_t workspace_bytes, void* stream);
-/* Tunes yq_order_by for this input: the run-formation sort through
- * yq_sort_autotune (digit bits, items per thread, block threads; returned in
- * *best_sort) and the merge-path tile (outputs per thread, 4, 8 or 16; 16 for
- * keys of up to two words) by timing the whole ORDER BY once per tile; the
- * fastest tile is remembered for this key width and row count (log2) and
- * used by later yq_order_by calls. The reference fixes the merge tile at
- * compile time (ELE_PER_TH 6, src/kernels/merge_batchs.cu:8). Allocates its
- * own output and workspace (stream-ordered) and synchronises `stream`. */
+/* Tunes yq_order_by for this input: its sort through yq_sort_autotune (digit
+ * bits, items per thread, block threads; returned in *best_sort and used by
+ * later calls on inputs of this key width and size), and the merge-path tile of
+ * yq_order_by_tiled (outputs per thread, 4, 8 or 16; 16 for keys of up to two
+ * words) by timing the whole ORDER BY once per tile. The reference fixes the
+ * merge tile at compile time (ELE_PER_TH 6, src/kernels/merge_batchs.cu:8).
+ * Allocates its own output and workspace (stream-ordered) and synchronises
+ * `stream`. */
 int yq_order_by_autotune(const yq_batch* in, int32_t key_col, int32_t descending, int32_t nulls_first,
                          const uint32_t* run_offsets, int32_t nruns, yq_sort_config* best_sort,
                          int32_t* best_merge_items, void* stream);

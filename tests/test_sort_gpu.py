@@ -155,3 +155,36 @@ def test_long_text_keys_sort_in_chunks(cuda, width, desc, with_nulls):
     perm = ops.sort_indices(col, descending=desc).cpu().numpy()
     want = oracle.sort_perm(k, desc=desc, nulls=nulls)
     np.testing.assert_array_equal(perm.astype(np.int64), want.astype(np.int64))
+
+
+@pytest.mark.parametrize("n", [2_000_003, 3_000_001])
+def test_gather_of_large_tables(cuda, n):
+    """Tables around and above the packed-row threshold: every cell width the
+    records hold, null bytes on both or one side, a wide text column that moves
+    by itself, and a permutation that is not one (its bad rows are skipped)."""
+    rng = np.random.default_rng(n)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(n)
+    perm = torch.randperm(n, generator=g, device="cuda", dtype=torch.int32)
+    cols = []
+    for type_, width in ((A.INT64, 8), (A.TEXT, 16), (A.INT32, 4), (A.TEXT, 12), (A.BOOL, 1), (A.TEXT, 64), (A.FLOAT64, 8)):
+        d = torch.randint(0, 256, (n, width), generator=g, device="cuda", dtype=torch.uint8)
+        data = d if type_ == A.TEXT else d.view(ops.TORCH_DTYPE[type_]).flatten()
+        nulls = (torch.rand(n, generator=g, device="cuda") < 0.1).to(torch.uint8) if width in (4, 12) else None
+        cols.append(ops.DeviceColumn(data, type_, nulls))
+    out = ops.gather(ops.DeviceBatch(cols), perm)
+    idx = perm.long()
+    for c, o in zip(cols, out.columns):
+        assert torch.equal(o.data.view(torch.uint8), c.data[idx].view(torch.uint8))
+        if c.nulls is not None:
+            assert torch.equal(o.nulls, c.nulls[idx])
+    bad = perm.clone()
+    bad[5], bad[n - 1] = n, -1
+    for o in out.columns:
+        o.data.zero_()
+    ops.gather(ops.DeviceBatch(cols), bad, out=out)
+    keep = torch.ones(n, dtype=torch.bool, device="cuda")
+    keep[5] = keep[n - 1] = False
+    for c, o in zip(cols, out.columns):
+        assert torch.equal(o.data[keep].view(torch.uint8), c.data[idx[keep]].view(torch.uint8))
+        assert not o.data[~keep].view(torch.uint8).any()

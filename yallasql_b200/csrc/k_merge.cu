@@ -13,8 +13,6 @@
 //      on an mbarrier, merges there (ties take run A, so the merge is stable),
 //      and moves every payload column with coalesced writes.
 #include <string.h>
-#include <map>
-#include <mutex>
 #include <vector>
 #include "yq_sort.cuh"
 
@@ -450,7 +448,6 @@ __global__ void k_merge_raw_partition(const __grid_constant__ RawLevel L) {
 struct RawSlot {
   uint32_t na, nb, cnt, out0;
   uint32_t ka, kb, ia, ib;  // byte offsets of the first A / B key and id in the slot
-  uint32_t a_row, b_row;    // first A / B row (the ids themselves when the level has no id input)
 };
 
 // ITEMS outputs per thread: a tile of kMergeBlock * ITEMS outputs. Variants
@@ -496,27 +493,19 @@ __device__ __forceinline__ void raw_issue(const RawLevel& L, const RawTile& d, i
   r.nb = d.nb;
   r.cnt = d.cnt;
   r.out0 = d.out0;
-  r.a_row = d.a_row;
-  r.b_row = d.b_row;
   {
     uint32_t k2 = 0, i2 = 0, b2 = 0;
     r.ka = raw_window(kreg, k2, L.keys_in, d.a_row, d.na, G::W, bar, b2, false);
     r.kb = raw_window(kreg, k2, L.keys_in, d.b_row, d.nb, G::W, bar, b2, false);
-    if (L.ids_in) {  // no id input: every row's id is its row number
-      r.ia = raw_window(ireg, i2, L.ids_in, d.a_row, d.na, 4u, bar, b2, false);
-      r.ib = raw_window(ireg, i2, L.ids_in, d.b_row, d.nb, 4u, bar, b2, false);
-    } else {
-      r.ia = r.ib = 0u;
-    }
+    r.ia = raw_window(ireg, i2, L.ids_in, d.a_row, d.na, 4u, bar, b2, false);
+    r.ib = raw_window(ireg, i2, L.ids_in, d.b_row, d.nb, 4u, bar, b2, false);
     mbar_arrive_expect_tx(bar, b2);
   }
   s_slot[slot] = r;
   raw_window(kreg, ko, L.keys_in, d.a_row, d.na, G::W, bar, bytes, true);
   raw_window(kreg, ko, L.keys_in, d.b_row, d.nb, G::W, bar, bytes, true);
-  if (L.ids_in) {
-    raw_window(ireg, io, L.ids_in, d.a_row, d.na, 4u, bar, bytes, true);
-    raw_window(ireg, io, L.ids_in, d.b_row, d.nb, 4u, bar, bytes, true);
-  }
+  raw_window(ireg, io, L.ids_in, d.a_row, d.na, 4u, bar, bytes, true);
+  raw_window(ireg, io, L.ids_in, d.b_row, d.nb, 4u, bar, bytes, true);
 }
 
 template <int KW>
@@ -666,13 +655,13 @@ __global__ void __launch_bounds__(kMergeBlock) k_merge_raw_tiles(const __grid_co
         if (takeA) {
 #pragma unroll
           for (int j = 0; j < KW; ++j) okey[x][j] = ka[j];
-          oid[x] = L.ids_in ? idA[ia] : r.a_row + ia;
+          oid[x] = idA[ia];
           ++ia;
           if (ia < r.na) raw_key_s<KW>(kA + (size_t)ia * G::W, ka);
         } else {
 #pragma unroll
           for (int j = 0; j < KW; ++j) okey[x][j] = kb[j];
-          oid[x] = L.ids_in ? idB[jb] : r.b_row + jb;
+          oid[x] = idB[jb];
           ++jb;
           if (jb < r.nb) raw_key_s<KW>(kB + (size_t)jb * G::W, kb);
         }
@@ -729,6 +718,68 @@ static int launch_raw_level(const RawLevel& L, cudaStream_t s, double bytes) {
   return YQ_OK;
 }
 
+// The key column from the sorted key words (no merge level to write it).
+// TYPE: one value class per kernel, so that a thread's eight loads are in
+// flight before its first store.
+template <int KW, int TYPE>
+__global__ void __launch_bounds__(256) k_decode_keys(const uint32_t* __restrict__ keys, const KeyDecode dec, uint32_t rows) {
+  constexpr int ROWS = 8;
+  const uint32_t inv = dec.desc ? 0xffffffffu : 0u;
+  for (unsigned long long r0 = blockIdx.x * 256ull * ROWS; r0 < rows; r0 += gridDim.x * 256ull * ROWS) {
+    uint32_t lo[ROWS], hi[ROWS];
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i) {
+      const unsigned long long r = min(r0 + i * 256 + threadIdx.x, (unsigned long long)rows - 1);
+      if (KW == 1) {
+        lo[i] = __ldg(keys + r);
+        hi[i] = dec.high[0];
+      } else {
+        const uint2 q = __ldg(reinterpret_cast<const uint2*>(keys) + r);
+        lo[i] = q.x;
+        hi[i] = q.y;
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i) {
+      const unsigned long long r = r0 + i * 256 + threadIdx.x;
+      if (r >= rows) break;
+      const uint32_t a = lo[i] ^ inv, b = hi[i] ^ inv;
+      if (TYPE == YQ_INT32) reinterpret_cast<uint32_t*>(dec.out)[r] = a ^ 0x80000000u;
+      else if (TYPE == YQ_FLOAT32) reinterpret_cast<uint32_t*>(dec.out)[r] = (a & 0x80000000u) ? (a & 0x7fffffffu) : ~a;
+      else if (TYPE == YQ_BOOL) reinterpret_cast<uint8_t*>(dec.out)[r] = (uint8_t)(a & 1u);
+      else if (TYPE == YQ_INT64) reinterpret_cast<uint2*>(dec.out)[r] = make_uint2(a, b ^ 0x80000000u);
+      else reinterpret_cast<uint2*>(dec.out)[r] = (b & 0x80000000u) ? make_uint2(a, b & 0x7fffffffu) : make_uint2(~a, ~b);
+    }
+  }
+}
+
+template <int KW>
+static int launch_decode_type(const uint32_t* keys, const KeyDecode& dec, uint32_t rows, int grid, cudaStream_t s) {
+  switch (dec.type) {
+    case YQ_INT32: k_decode_keys<KW, YQ_INT32><<<grid, 256, 0, s>>>(keys, dec, rows); break;
+    case YQ_FLOAT32: k_decode_keys<KW, YQ_FLOAT32><<<grid, 256, 0, s>>>(keys, dec, rows); break;
+    case YQ_BOOL: k_decode_keys<KW, YQ_BOOL><<<grid, 256, 0, s>>>(keys, dec, rows); break;
+    case YQ_INT64:
+    case YQ_DATETIME: k_decode_keys<KW, YQ_INT64><<<grid, 256, 0, s>>>(keys, dec, rows); break;
+    case YQ_FLOAT64: k_decode_keys<KW, YQ_FLOAT64><<<grid, 256, 0, s>>>(keys, dec, rows); break;
+    default: return YQ_ERR_UNSUPPORTED;
+  }
+  YQ_CHECK_LAUNCH();
+  return YQ_OK;
+}
+
+static int launch_decode_keys(int kw, const uint32_t* keys, const KeyDecode& dec, uint32_t rows, cudaStream_t s) {
+  const int cap = sm_count() * 8;
+  const uint32_t need = ceil_div<uint32_t>(rows, 256 * 8);
+  const int grid = need < (uint32_t)cap ? (int)need : cap;
+  ProfScope ps("decode_keys", s, (double)rows * (4.0 * kw + dec.width));
+  switch (kw) {  // a decodable key has at most two words
+    case 1: return launch_decode_type<1>(keys, dec, rows, grid, s);
+    case 2: return launch_decode_type<2>(keys, dec, rows, grid, s);
+    default: return YQ_ERR_UNSUPPORTED;
+  }
+}
+
 static bool merge_items_ok(int kw, int items) {
   return items == 4 || items == 8 || (items == 16 && kw <= 2);
 }
@@ -747,26 +798,6 @@ static int launch_raw_level_items(int kw, int items, const RawLevel& L, cudaStre
     case 808: return launch_raw_level<8, 8>(L, s, bytes);
     default: return YQ_ERR_UNSUPPORTED;
   }
-}
-
-// Merge-path tile (outputs per thread) per (key words, log2 of rows), set by
-// yq_order_by_autotune; kMergeItems where none was tuned.
-static std::mutex g_merge_tune_mu;
-static std::map<std::pair<int, int>, int> g_merge_tuned;
-
-static int log2_rows(uint32_t rows) {
-  int b = 0;
-  while (rows > 1) {
-    rows >>= 1;
-    ++b;
-  }
-  return b;
-}
-
-static int merge_items_for(int kw, uint32_t rows) {
-  std::lock_guard<std::mutex> lk(g_merge_tune_mu);
-  auto it = g_merge_tuned.find({kw, log2_rows(rows)});
-  return it == g_merge_tuned.end() ? kMergeItems : it->second;
 }
 
 // Merge levels of one ORDER BY: host plan of every level's pairs.
@@ -813,33 +844,10 @@ struct OrderWs {
   size_t npairs = 0;
 };
 
-// Two-level gather: with many runs over a table larger than L2, one gather by
-// the merged row ids reads every cell at a random row of the whole table
-// (each 4-16-byte cell costs a DRAM sector or more). Instead every column is
-// first gathered run by run into sorted-run order (the rows a run reads lie
-// within that run, so the in-flight window stays in L2), the row ids become
-// positions in that layout, and after the merges the final gather reads each
-// run's rows in increasing order: hundreds of sequential streams whose
-// sectors L2 serves until every cell of them is used.
-constexpr double kTwoLevelGatherBytes = 64.0 * 1024 * 1024;
-
-static bool two_level_gather(const yq_batch& in, int nruns) {
-  if (nruns < 2) return false;
-  double b = 0;
-  for (int c = 0; c < in.ncols; ++c) b += (double)in.rows * (in.columns[c].width + (in.columns[c].nulls ? 1 : 0));
-  return b >= kTwoLevelGatherBytes;
-}
-
-// The sorted-run copy of every column (same widths, nulls where the input has them).
-static void stage_ws_layout(const yq_batch& in, WsSize& w) {
-  for (int c = 0; c < in.ncols; ++c) {
-    w.add<char>((size_t)in.rows * in.columns[c].width + 16);
-    if (in.columns[c].nulls) w.add<uint8_t>((size_t)in.rows + 16);
-  }
-}
-
-__global__ void k_iota(uint32_t* __restrict__ ids, uint32_t n) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) ids[i] = i;
+// Null bytes and values of a batch as the gather of an ORDER BY sees them (the
+// outputs have the inputs' columns).
+static size_t order_record_bytes(const yq_batch& in) {
+  return packed_gather_bytes(in.columns, in.ncols, in.columns, nullptr, in.rows);
 }
 
 static int order_ws_layout(const yq_column& key, uint32_t rows, const uint32_t* offsets, int nruns, OrderWs& o,
@@ -880,7 +888,7 @@ extern "C" size_t yq_order_by_batch_workspace_size(const yq_batch* in, int32_t k
   OrderWs o;
   WsSize w;
   if (order_ws_layout(in->columns[key_col], in->rows, run_offsets, nruns, o, w) != YQ_OK) return 0;
-  if (two_level_gather(*in, nruns)) stage_ws_layout(*in, w);
+  if (const size_t rec = order_record_bytes(*in)) w.add<char>(rec);
   return w.total();
 }
 
@@ -932,7 +940,10 @@ static int order_by_segments_impl(const yq_batch* in, int32_t key_col, int32_t d
                             nullptr, true, &sort_err));
   yq_column outs[YQ_MAX_BATCH_COLUMNS];
   for (int c = 0; c < in->ncols; ++c) outs[c] = out->columns[c];
-  YQ_TRY(yq_gather(in->columns, in->ncols, perm, rows, outs, s));
+  // column by column: a task's rows lie within its own rows, which L2 holds
+  // for tasks of up to a few million rows, and packing them first costs what
+  // the records save (26M rows in 64 tasks: 1.32 ms against 0.65 + 0.91)
+  YQ_TRY(gather_impl(in->columns, in->ncols, perm, rows, outs, nullptr, s));
   YQ_TRY_CUDA(cudaMemcpyAsync(d_err, sort_err, sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
   if (no_wait) return YQ_OK;
   uint32_t e = 0;
@@ -959,11 +970,11 @@ extern "C" int yq_order_by_segments_perm(const yq_batch* in, int32_t key_col, in
                                 workspace, workspace_bytes, stream);
 }
 
-// merge_items: outputs per thread of the merge tiles (0 = the tuned or default
-// choice); *kw_used (optional): the key words the merge levels compared.
+// merge_items: outputs per thread of the merge tiles (0 = no merge: one sort of
+// the whole table).
 static int order_by_run(const yq_batch* in, int32_t key_col, int32_t descending, int32_t nulls_first,
                         const uint32_t* run_offsets, int32_t nruns, yq_batch* out, void* workspace,
-                        size_t workspace_bytes, void* stream, int merge_items, int* kw_used = nullptr) {
+                        size_t workspace_bytes, void* stream, int merge_items) {
   if (!in || !out || !run_offsets || nruns <= 0 || key_col < 0 || key_col >= in->ncols || out->ncols != in->ncols ||
       in->ncols > YQ_MAX_BATCH_COLUMNS)
     return YQ_ERR_INVALID_ARG;
@@ -983,32 +994,33 @@ static int order_by_run(const yq_batch* in, int32_t key_col, int32_t descending,
   WsSize wsz;
   YQ_TRY(order_ws_layout(key, rows, run_offsets, nruns, o, wsz));
   const size_t base_bytes = wsz.total();
-  // The sorted-run copy needs more workspace: used when the caller's holds it
-  // (yq_order_by_batch_workspace_size) or the library allocates.
-  bool staged = two_level_gather(*in, nruns);
-  if (staged) {
-    stage_ws_layout(*in, wsz);
-    if (workspace && workspace_bytes < wsz.total()) staged = false;
+  // The gather's packed rows need more workspace: used when the caller's holds
+  // them (yq_order_by_batch_workspace_size) or the library allocates.
+  size_t rec_bytes = order_record_bytes(*in);
+  if (rec_bytes) {
+    wsz.add<char>(rec_bytes);
+    if (workspace && workspace_bytes < wsz.total()) rec_bytes = 0;
   }
   Workspace ws;
-  YQ_TRY(ws.acquire(workspace, workspace_bytes, staged ? wsz.total() : base_bytes, s));
+  YQ_TRY(ws.acquire(workspace, workspace_bytes, rec_bytes ? wsz.total() : base_bytes, s));
   char* sort_ws = ws.take<char>(o.sort_bytes);
   uint32_t* keys[2] = {ws.take<uint32_t>((size_t)rows * o.kw_max + 16), ws.take<uint32_t>((size_t)rows * o.kw_max + 16)};
   uint32_t* ids[2] = {ws.take<uint32_t>((size_t)rows + 16), ws.take<uint32_t>((size_t)rows + 16)};
   RawPair* d_pairs = ws.take<RawPair>(o.npairs);
   RawTile* d_tiles = ws.take<RawTile>(o.max_tiles);
   uint32_t* d_err = ws.take<uint32_t>(4);
-  yq_column stage[YQ_MAX_BATCH_COLUMNS];
-  if (staged)
-    for (int c = 0; c < in->ncols; ++c) {
-      stage[c] = in->columns[c];
-      stage[c].data = ws.take<char>((size_t)rows * in->columns[c].width + 16);
-      stage[c].nulls = in->columns[c].nulls ? ws.take<uint8_t>((size_t)rows + 16) : nullptr;
-    }
+  char* records = rec_bytes ? ws.take<char>(rec_bytes) : nullptr;
   YQ_TRY_CUDA(cudaMemsetAsync(d_err, 0, 4 * sizeof(uint32_t), s));
 
-  // 1. every run sorted; the sort hands over its key words and row ids, and
-  // its histogram pass flags key values the key words cannot restore
+  // 1. the table sorted by one stable sort, as the runs sorted and merged with
+  // ties to the earlier run would leave it: the passes over the whole table
+  // cost 15 % more than within its runs (64M rows, f32 key: 2.5 against 2.2 ms)
+  // and the merge levels they save cost more than the sort does (550 runs: ten
+  // levels, 2.6 ms). A call that names a merge tile sorts the runs and merges.
+  // The sort hands over its key words and row ids, and its histogram pass
+  // flags key values the key words cannot restore.
+  const bool by_runs = merge_items != 0 && nruns > 1;
+  const uint32_t whole[2] = {0, rows};
   const bool may_decode = nruns > 1 && !key.nulls && key.type != YQ_TEXT;
   uint32_t* d_lossy = d_err + 1;
   KeyJob job{key, descending != 0, nulls_first != 0};
@@ -1016,32 +1028,31 @@ static int order_by_run(const yq_batch* in, int32_t key_col, int32_t descending,
   int kw = 0;
   uint32_t* sort_err = nullptr;
   uint32_t high[8];
-  YQ_TRY(sort_segments_impl(&job, 1, rows, run_offsets, nruns, ids[0], nullptr, sort_ws, o.sort_bytes, s, nullptr,
-                            keys[0], &kw, true, &sort_err, high));
-  // The last merge level writes the key column itself when the key has no
+  YQ_TRY(sort_segments_impl(&job, 1, rows, by_runs ? run_offsets : whole, by_runs ? nruns : 1, ids[0], nullptr, sort_ws,
+                            o.sort_bytes, s, nullptr, keys[0], &kw, true, &sort_err, high));
+  // The key column is written from the sorted key words when the key has no
   // nulls; the gather then moves the key column only if some value would not
   // round-trip through its key words (flag set on the device).
   const bool decode = kw > 0 && may_decode;
   const uint32_t* only_if[YQ_MAX_BATCH_COLUMNS] = {nullptr};
-  if (decode) only_if[key_col] = d_lossy;  // zero unless a value would not round-trip
-  // 1b. two-level gather, first level: every column into sorted-run order;
-  // the row ids become positions in that copy, so the first merge level
-  // reads no ids (a row's id is its position)
-  const bool merged = kw > 0 && nruns > 1;
-  staged = staged && merged;
-  bool ids_are_positions = false;
-  if (staged) {
-    YQ_TRY(gather_impl(in->columns, in->ncols, ids[0], rows, stage, only_if, s));
-    ids_are_positions = true;
+  KeyDecode dec;
+  memset(&dec, 0, sizeof(dec));
+  if (decode) {
+    only_if[key_col] = d_lossy;  // zero unless a value would not round-trip
+    dec.out = static_cast<char*>(out->columns[key_col].data);
+    dec.type = key.type;
+    dec.vwords = key.type == YQ_INT32 || key.type == YQ_FLOAT32 || key.type == YQ_BOOL ? 1 : 2;
+    dec.width = key.width;
+    dec.desc = descending != 0;
+    memcpy(dec.high, high, sizeof(high));
   }
   // 2. merge levels over (key words, row id)
   int cur = 0;
-  if (merged) {
-    if (kw_used) *kw_used = kw;
-    const int mi = merge_items ? merge_items : merge_items_for(kw, rows);
-    if (!merge_items_ok(kw, mi)) return YQ_ERR_UNSUPPORTED;
+  bool merged = false;
+  if (by_runs && kw > 0) {
+    if (!merge_items_ok(kw, merge_items)) return YQ_ERR_UNSUPPORTED;
     OrderPlan P;
-    plan_order_levels(run_offsets, nruns, kMergeBlock * (uint32_t)mi, P);
+    plan_order_levels(run_offsets, nruns, kMergeBlock * (uint32_t)merge_items, P);
     if (P.pairs.size() > o.npairs) return YQ_ERR_UNSUPPORTED;
     YQ_TRY(h2d_async(d_pairs, P.pairs.data(), P.pairs.size() * sizeof(RawPair), s));
     const int levels = (int)P.level_tiles.size();
@@ -1049,17 +1060,10 @@ static int order_by_run(const yq_batch* in, int32_t key_col, int32_t descending,
       const bool last = l + 1 == levels;
       RawLevel L;
       L.keys_in = keys[cur];
-      L.ids_in = ids_are_positions ? nullptr : ids[cur];
+      L.ids_in = ids[cur];
       L.keys_out = last ? nullptr : keys[cur ^ 1];
       memset(&L.dec, 0, sizeof(L.dec));
-      if (last && decode) {
-        L.dec.out = static_cast<char*>(out->columns[key_col].data);
-        L.dec.type = key.type;
-        L.dec.vwords = key.type == YQ_INT32 || key.type == YQ_FLOAT32 || key.type == YQ_BOOL ? 1 : 2;
-        L.dec.width = key.width;
-        L.dec.desc = descending != 0;
-        memcpy(L.dec.high, high, sizeof(high));
-      }
+      if (last) L.dec = dec;
       L.ids_out = ids[cur ^ 1];
       L.pairs = d_pairs + P.level_first[l];
       L.npairs = P.level_first[l + 1] - P.level_first[l];
@@ -1068,25 +1072,20 @@ static int order_by_run(const yq_batch* in, int32_t key_col, int32_t descending,
       L.err = d_err;
       if (L.ntiles > o.max_tiles) return YQ_ERR_UNSUPPORTED;
       if (L.ntiles == 0) continue;
-      // algorithmic bytes: key words + id in and out (ids only out on the
-      // last level; no ids in when they are the row positions)
-      const double bytes =
-          (double)rows * (4.0 * kw + (L.ids_in ? 4.0 : 0.0) + (last ? 4.0 : 4.0 * kw + 4.0));
-      YQ_TRY(launch_raw_level_items(kw, mi, L, s, bytes));
-      ids_are_positions = false;
+      // algorithmic bytes: key words + id in and out (ids only out on the last level)
+      const double bytes = (double)rows * (4.0 * kw + 4.0 + (last ? 4.0 : 4.0 * kw + 4.0));
+      YQ_TRY(launch_raw_level_items(kw, merge_items, L, s, bytes));
+      merged = true;
       cur ^= 1;
     }
   }
-  if (ids_are_positions) {  // no level ran: the final gather still needs the positions written out
-    k_iota<<<sm_count() * 4, 256, 0, s>>>(ids[cur], rows);
-    YQ_CHECK_LAUNCH();
-  }
+  if (decode && !merged) YQ_TRY(launch_decode_keys(kw, keys[cur], dec, rows, s));
   // 3. every column (the key included) gathered once by the final row ids
-  YQ_TRY(gather_impl(staged ? stage : in->columns, in->ncols, ids[cur], rows, out->columns, only_if, s));
-  uint32_t err[2] = {0, 0};
-  YQ_TRY(d2h_sync(&err[0], sort_err, sizeof(uint32_t), s));
-  YQ_TRY(d2h_sync(&err[1], d_err, sizeof(uint32_t), s));
-  const uint32_t e = err[0] | err[1];
+  YQ_TRY(gather_impl(in->columns, in->ncols, ids[cur], rows, out->columns, only_if, s, records, rec_bytes));
+  YQ_TRY_CUDA(cudaMemcpyAsync(d_err + 2, sort_err, sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
+  uint32_t err[3] = {0, 0, 0};  // merge, lossy flag, sort
+  YQ_TRY(d2h_sync(err, d_err, sizeof(err), s));
+  const uint32_t e = err[0] | err[2];
   if (e & kErrTimeout) return YQ_ERR_TIMEOUT;
   if (e & kErrBounds) return YQ_ERR_INVALID_ARG;
   return YQ_OK;
@@ -1114,8 +1113,9 @@ extern "C" int yq_order_by_autotune(const yq_batch* in, int32_t key_col, int32_t
       !best_sort || !best_merge_items)
     return YQ_ERR_INVALID_ARG;
   cudaStream_t s = as_stream(stream);
-  // run formation: the sort's own tuner over the runs as segments
-  YQ_TRY(yq_sort_autotune(&in->columns[key_col], in->rows, run_offsets, nruns, descending, best_sort, stream));
+  // the sort's own tuner over the whole table, as yq_order_by sorts it
+  const uint32_t whole[2] = {0, in->rows};
+  YQ_TRY(yq_sort_autotune(&in->columns[key_col], in->rows, whole, 1, descending, best_sort, stream));
   *best_merge_items = kMergeItems;
   const int kw = sort_key_words_max(in->columns[key_col]);
   if (nruns < 2 || in->rows == 0 || kw <= 0) return YQ_OK;
@@ -1147,12 +1147,10 @@ extern "C" int yq_order_by_autotune(const yq_batch* in, int32_t key_col, int32_t
     status = YQ_ERR_CUDA;
   float best_ms = 1e30f;
   int pick = kMergeItems;
-  int kw_merge = 0;
   for (int items : {8, 4, 16}) {
     if (status != YQ_OK) break;
     if (!merge_items_ok(kw, items)) continue;
-    status = order_by_run(in, key_col, descending, nulls_first, run_offsets, nruns, &out, ws, wsb, stream, items,
-                          &kw_merge);
+    status = order_by_run(in, key_col, descending, nulls_first, run_offsets, nruns, &out, ws, wsb, stream, items);
     if (status != YQ_OK) break;
     cudaEventRecord(e0, s);
     for (int r = 0; r < 2 && status == YQ_OK; ++r)
@@ -1171,10 +1169,6 @@ extern "C" int yq_order_by_autotune(const yq_batch* in, int32_t key_col, int32_t
   for (int i = 0; i < nb; ++i)
     if (bufs[i]) cudaFreeAsync(bufs[i], s);
   if (status != YQ_OK) return status;
-  if (kw_merge > 0) {  // keyed by the key words the merge levels compare
-    std::lock_guard<std::mutex> lk(g_merge_tune_mu);
-    g_merge_tuned[{kw_merge, log2_rows(in->rows)}] = pick;
-  }
   *best_merge_items = pick;
   return YQ_OK;
 }

@@ -1047,37 +1047,53 @@ int sort_segments_impl(const KeyJob* jobs, int njobs, uint32_t rows, const uint3
 
 // Gather used by yq_gather and yq_order_by (see yq_sort.cuh).
 int gather_impl(const yq_column* in, int32_t ncols, const uint32_t* perm, uint32_t rows, const yq_column* out,
-                const uint32_t* const* only_if, cudaStream_t s) {
+                const uint32_t* const* only_if, cudaStream_t s, void* records, size_t record_bytes, bool may_alloc) {
   if (ncols < 0 || ncols > YQ_MAX_BATCH_COLUMNS || (ncols > 0 && (!in || !out)) || (rows > 0 && !perm))
     return YQ_ERR_INVALID_ARG;
   if (rows == 0 || ncols == 0) return YQ_OK;
-  GatherParams G;
-  memset(&G, 0, sizeof(G));
-  G.ncols = ncols;
   for (int c = 0; c < ncols; ++c) {
     if (!in[c].data || !out[c].data || in[c].width != out[c].width || in[c].width <= 0) return YQ_ERR_INVALID_ARG;
     if (in[c].width != 1 && in[c].width % 4 != 0) return YQ_ERR_INVALID_ARG;
-    G.c[c].src = static_cast<const char*>(in[c].data);
-    G.c[c].src_nulls = in[c].nulls;
-    G.c[c].dst = static_cast<char*>(out[c].data);
-    G.c[c].dst_nulls = const_cast<uint8_t*>(out[c].nulls);
-    G.c[c].width = in[c].width;
-    G.c[c].only_if = only_if ? only_if[c] : nullptr;
   }
+  uint32_t moved = 0;
+  if (const size_t need = packed_gather_bytes(in, ncols, out, only_if, rows)) {
+    Workspace ws;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    YQ_TRY_CUDA(cudaStreamIsCapturing(s, &cap));
+    if (records ? record_bytes < need
+                : !may_alloc || cap != cudaStreamCaptureStatusNone || need > pool_kept_bytes()) {
+      records = nullptr;
+    } else if (!records && ws.acquire(nullptr, 0, need, s) == YQ_OK) {  // no memory: column by column
+      records = ws.base;
+    }
+    if (records) YQ_TRY(packed_gather(in, ncols, out, only_if, perm, rows, records, s, &moved));
+  }
+  GatherParams G;
+  memset(&G, 0, sizeof(G));
+  double row_bytes = 4.0;  // permutation
+  for (int c = 0; c < ncols; ++c) {
+    if (moved >> c & 1u) continue;
+    GatherCol& g = G.c[G.ncols++];
+    g.src = static_cast<const char*>(in[c].data);
+    g.src_nulls = in[c].nulls;
+    g.dst = static_cast<char*>(out[c].data);
+    g.dst_nulls = const_cast<uint8_t*>(out[c].nulls);
+    g.width = in[c].width;
+    g.only_if = only_if ? only_if[c] : nullptr;
+    if (!g.only_if) row_bytes += 2.0 * in[c].width + (out[c].nulls ? 2.0 : 0.0);
+  }
+  if (G.ncols == 0) return YQ_OK;
   // Aligned columns (16-byte text slots, 4/8-byte values) take the
   // column-parallel kernel; others the row-parallel one.
   bool aligned = true;
-  for (int c = 0; c < ncols; ++c)
+  for (int c = 0; c < G.ncols; ++c)
     aligned &= ((reinterpret_cast<uintptr_t>(G.c[c].src) | reinterpret_cast<uintptr_t>(G.c[c].dst)) &
                 (uintptr_t)(G.c[c].width >= 16 ? 15 : (G.c[c].width >= 8 ? 7 : (G.c[c].width >= 4 ? 3 : 0)))) == 0;
-  double row_bytes = 4.0;  // permutation
-  for (int c = 0; c < ncols; ++c)
-    if (!only_if || !only_if[c]) row_bytes += 2.0 * in[c].width + (out[c].nulls ? 2.0 : 0.0);
   ProfScope ps("gather", s, (double)rows * row_bytes);
   if (aligned) {
     const uint32_t tiles = ceil_div<uint32_t>(rows, 256u * kGatherItems);
     const uint32_t cap = (uint32_t)sm_count() * 8;
-    dim3 grid(tiles < cap ? tiles : cap, (unsigned)ncols);
+    dim3 grid(tiles < cap ? tiles : cap, (unsigned)G.ncols);
     k_gather_cols<<<grid, 256, 0, s>>>(G, perm, rows);
   } else {
     int grid = (int)ceil_div<uint32_t>(rows, 256);
@@ -1208,7 +1224,7 @@ int yq_sort_autotune(const yq_column* key, uint32_t rows, const uint32_t* seg_of
 }
 
 int yq_gather(const yq_column* in, int32_t ncols, const uint32_t* perm, uint32_t rows, yq_column* out, void* stream) {
-  return gather_impl(in, ncols, perm, rows, out, nullptr, as_stream(stream));
+  return gather_impl(in, ncols, perm, rows, out, nullptr, as_stream(stream), nullptr, 0, true);
 }
 
 }  // extern "C"

@@ -523,14 +523,14 @@ class PreparedDim:
 
 
 def order_by_workspace_bytes(col: DeviceColumn, offsets: list[int]) -> int:
-    """Least workspace of yq_order_by (one-level gather)."""
+    """Least workspace of yq_order_by (columns gathered one by one)."""
     offs = (C.c_uint32 * len(offsets))(*offsets)
     cc = col.c()
     return int(lib().yq_order_by_workspace_size(C.byref(cc), col.rows, offs, len(offsets) - 1))
 
 
 def order_by_batch_workspace_bytes(batch: DeviceBatch, key: int, offsets: list[int]) -> int:
-    """Workspace of yq_order_by including the sorted-run copy of the columns."""
+    """Workspace of yq_order_by including the packed rows of the columns."""
     offs = (C.c_uint32 * len(offsets))(*offsets)
     b, _keep = batch.c()
     return int(lib().yq_order_by_batch_workspace_size(C.byref(b), key, offs, len(offsets) - 1))
@@ -538,13 +538,12 @@ def order_by_batch_workspace_bytes(batch: DeviceBatch, key: int, offsets: list[i
 
 class OrderByRuns:
     """Out-of-core ORDER BY of one key over a batch made of runs (4 MB
-    batches), through yq_order_by: the runs are sorted by the segmented radix
-    sort, merged level by level as (key words, row id) pairs, and every column
-    is gathered once by the merged row ids (OrderOperator::firstPass +
+    batches), through yq_order_by: one stable radix sort of the whole table
+    (the order that sorted and merged runs would have), then every column
+    gathered once by the sorted row ids (OrderOperator::firstPass +
     merge_all_sorted, order_operator.hpp:89-193 / order_operator.cpp:14-220).
     The workspace is allocated once and reused across calls; `two_level`
-    sizes it for the sorted-run copy that the two-level gather uses on large
-    tables."""
+    sizes it for the packed rows through which large tables are gathered."""
 
     def __init__(self, batch: DeviceBatch, key: int, offsets: list[int], two_level: bool = True):
         self.key, self.offsets, self.n = key, list(offsets), batch.rows
@@ -620,9 +619,10 @@ def sort_autotune(col: DeviceColumn, offsets, descending=False, stream=None) -> 
 
 def order_by_autotune(batch: DeviceBatch, key: int, descending: bool, offsets, nulls_first=False,
                       stream=None) -> tuple["A.SortConfig", int]:
-    """Tune yq_order_by for this input (yq_order_by_autotune): the run sort's
-    (digit bits, items per thread, block threads) and the merge tile's outputs
-    per thread, remembered for later calls on inputs of this shape."""
+    """Tune yq_order_by for this input (yq_order_by_autotune): the sort's
+    (digit bits, items per thread, block threads), remembered for later calls
+    on inputs of this shape, and the outputs per thread of the merge tile for
+    `order_by(..., merge_items=...)`."""
     offs = offsets if isinstance(offsets, C.Array) else (C.c_uint32 * len(offsets))(*offsets)
     ib, _ia = batch.c()
     best = A.SortConfig()
