@@ -157,6 +157,25 @@ def test_long_text_keys_sort_in_chunks(cuda, width, desc, with_nulls):
     np.testing.assert_array_equal(perm.astype(np.int64), want.astype(np.int64))
 
 
+@pytest.mark.parametrize("words", ["low", "high", "both", "none"])
+@pytest.mark.parametrize("nulls_first", [False, True])
+@pytest.mark.parametrize("n", [33, 4097, 123_457])
+def test_nullable_wide_keys(cuda, words, nulls_first, n):
+    """Nullable 8-byte keys of which one value word, the other, both or none is
+    the same in every row: the passes carry the words that differ."""
+    rng = np.random.default_rng(n + len(words))
+    lo = rng.integers(0, 1 << 32, n) if words in ("low", "both") else np.full(n, 77)
+    hi = rng.integers(-(1 << 31), 1 << 31, n) if words in ("high", "both") else np.full(n, -5)
+    k = (hi.astype(np.int64) << 32) | lo.astype(np.int64)
+    nulls = rng.random(n) < 0.2
+    for desc in (False, True):
+        perm = gpu_perm(dev_col(k, A.INT64, nulls), descending=desc, nulls_first=nulls_first)
+        rank = np.where(nulls, 0 if nulls_first else 2, 1)
+        # value order (reversed by DESC), NULLs at their end, ties in input order
+        want = np.lexsort((np.arange(n), np.where(nulls, 0, ~k if desc else k), rank))
+        np.testing.assert_array_equal(perm, want.astype(np.uint32))
+
+
 @pytest.mark.parametrize("n", [2_000_003, 3_000_001])
 def test_gather_of_large_tables(cuda, n):
     """Tables around and above the packed-row threshold: every cell width the

@@ -1232,6 +1232,7 @@ int yq_merge_pass(const yq_column* cols, int32_t ncols, int32_t key_col, int32_t
   M.key.desc = descending != 0;
   M.key.nulls_first = nulls_first != 0;
   M.key.null_word = kc.nulls != nullptr;
+  M.key.nsel = 0;
   M.staged = (kc.width <= 32 && (kc.width == 4 || kc.width == 8 || kc.width % 16 == 0) &&
               (reinterpret_cast<uintptr_t>(kc.data) & 15u) == 0);
 

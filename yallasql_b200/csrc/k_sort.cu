@@ -40,6 +40,7 @@ struct SegInfo {
 
 template <int KW, int D>
 __device__ __forceinline__ uint32_t digit_of(const uint32_t (&k)[KW], int shift) {
+  if (KW == 1 && 32 % D == 0) return (k[0] >> shift) & ((1u << D) - 1u);
   const int w = shift >> 5, o = shift & 31;
   uint32_t lo = 0u, hi = 0u;
 #pragma unroll
@@ -48,8 +49,62 @@ __device__ __forceinline__ uint32_t digit_of(const uint32_t (&k)[KW], int shift)
     if (j == w + 1) hi = k[j];
   }
   uint32_t v = lo >> o;
-  if (o + D > 32) v |= hi << (32 - o);
+  if (32 % D != 0 && o + D > 32) v |= hi << (32 - o);
   return v & ((1u << D) - 1u);
+}
+
+// Keys of N rows `rows[i]` (where `ok` has bit i) straight from the key column.
+// Fixed-width numeric columns without nulls, the common case, load every value
+// before any is transformed, so a thread keeps N reads in flight; a type switch
+// around each load would wait for one before it issues the next.
+template <int KW, int N>
+__device__ __forceinline__ void load_keys(const KeySrc& s, const uint32_t (&rows)[N], uint32_t ok, uint32_t (&k)[N][KW]) {
+  if (KW == 1 && !s.null_word && (s.type == YQ_INT32 || s.type == YQ_FLOAT32)) {
+    uint32_t v[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) v[i] = (ok >> i & 1u) ? __ldg(reinterpret_cast<const uint32_t*>(s.data) + rows[i]) : 0u;
+    const uint32_t inv = s.desc ? 0xffffffffu : 0u;
+    if (s.type == YQ_INT32) {
+#pragma unroll
+      for (int i = 0; i < N; ++i) k[i][0] = v[i] ^ 0x80000000u ^ inv;
+    } else {
+#pragma unroll
+      for (int i = 0; i < N; ++i) k[i][0] = float_key(v[i]) ^ inv;
+    }
+  } else if (KW == 2 && !s.null_word && (s.type == YQ_INT64 || s.type == YQ_DATETIME)) {
+    uint2 v[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+      v[i] = (ok >> i & 1u) ? __ldg(reinterpret_cast<const uint2*>(s.data) + rows[i]) : make_uint2(0u, 0u);
+    const uint32_t inv = s.desc ? 0xffffffffu : 0u;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      k[i][0] = v[i].x ^ inv;
+      k[i][KW > 1 ? 1 : 0] = v[i].y ^ 0x80000000u ^ inv;
+    }
+  } else if (KW == 2 && s.nsel) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      uint32_t f[4] = {0u, 0u, 0u, 0u};
+      if (ok >> i & 1u) make_key<4>(s, rows[i], f);
+#pragma unroll
+      for (int j = 0; j < KW; ++j) {
+        k[i][j] = 0u;
+#pragma unroll
+        for (int w = 0; w < 4; ++w)
+          if (j < s.nsel && s.sel[j] == w) k[i][j] = f[w];
+      }
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      if (ok >> i & 1u) make_key<KW>(s, rows[i], k[i]);
+      else {
+#pragma unroll
+        for (int j = 0; j < KW; ++j) k[i][j] = 0u;
+      }
+    }
+  }
 }
 
 __device__ __forceinline__ int find_segment(const SegInfo& g, uint32_t tile) {
@@ -66,15 +121,36 @@ __device__ __forceinline__ int find_segment(const SegInfo& g, uint32_t tile) {
 // ------------------------------------------------------------- histogram
 // Each block owns a contiguous range of tiles; per-segment counts for every
 // pass accumulate in shared memory and are flushed when the segment changes.
+// Bound by the latency of its loads and by shared-memory atomics on one
+// address: a thread loads kHistItems keys before it counts any, and one-word
+// keys count into four copies of the bins (lanes modulo 4), since the leading
+// digit of floats takes only a few values.
+template <int KW>
+constexpr int kHistCopies = KW == 1 ? 4 : (KW == 2 ? 2 : 1);
+template <int KW>
+constexpr int kHistItems = KW <= 2 ? 8 : (KW == 4 ? 4 : 2);
 template <int KW, int D>
 __global__ void __launch_bounds__(kSortBlock) k_sort_histogram(const KeySrc src, const SegInfo seg, uint32_t tile_rows,
                                                                uint32_t ntiles, uint32_t* __restrict__ hist) {
   constexpr int RADIX = 1 << D;
   constexpr int P = (KW * 32 + D - 1) / D;
-  extern __shared__ uint32_t s_hist[];  // [P][RADIX]
-  const int lane = threadIdx.x & 31;
-  for (int i = threadIdx.x; i < P * RADIX; i += kSortBlock) s_hist[i] = 0u;
+  constexpr int C = kHistCopies<KW>, N = kHistItems<KW>;
+  extern __shared__ uint32_t s_hist[];  // [P][RADIX][C]
+  const int lane = threadIdx.x & 31, copy = lane & (C - 1);
+  for (int i = threadIdx.x; i < P * RADIX * C; i += kSortBlock) s_hist[i] = 0u;
   __syncthreads();
+  auto flush = [&](int sg) {
+    uint32_t* h = hist + (size_t)sg * P * RADIX;
+    for (int i = threadIdx.x; i < P * RADIX; i += kSortBlock) {
+      uint32_t n = 0u;
+#pragma unroll
+      for (int c = 0; c < C; ++c) {
+        n += s_hist[i * C + c];
+        s_hist[i * C + c] = 0u;
+      }
+      if (n) atomicAdd(h + i, n);
+    }
+  };
   const uint32_t per = ceil_div<uint32_t>(ntiles, gridDim.x);
   const uint32_t t0 = blockIdx.x * per;
   const uint32_t t1 = min(ntiles, t0 + per);
@@ -84,11 +160,7 @@ __global__ void __launch_bounds__(kSortBlock) k_sort_histogram(const KeySrc src,
     if (sg != cur) {
       if (cur >= 0) {
         __syncthreads();
-        uint32_t* h = hist + (size_t)cur * P * RADIX;
-        for (int i = threadIdx.x; i < P * RADIX; i += kSortBlock) {
-          if (s_hist[i]) atomicAdd(h + i, s_hist[i]);
-          s_hist[i] = 0u;
-        }
+        flush(cur);
         __syncthreads();
       }
       cur = sg;
@@ -96,49 +168,49 @@ __global__ void __launch_bounds__(kSortBlock) k_sort_histogram(const KeySrc src,
     const uint32_t lt = t - __ldg(seg.tile_start + sg);
     const uint32_t r0 = __ldg(seg.seg_start + sg) + lt * tile_rows;
     const uint32_t r1 = min(__ldg(seg.seg_start + sg + 1), r0 + tile_rows);
-    for (uint32_t base = r0; base < r1; base += kSortBlock) {
-      const uint32_t e = base + threadIdx.x;
-      const bool valid = e < r1;
-      uint32_t k[KW];
-      const uint32_t row = valid ? (src.in_perm ? __ldg(src.in_perm + e) : e) : 0u;
-      if (valid) make_key<KW>(src, row, k);
-      else {
+    for (uint32_t base = r0; base < r1; base += kSortBlock * N) {
+      uint32_t row[N], k[N][KW], ok = 0u;
 #pragma unroll
-        for (int j = 0; j < KW; ++j) k[j] = 0u;
+      for (int i = 0; i < N; ++i) {
+        const uint32_t e = base + i * kSortBlock + threadIdx.x;
+        if (e < r1) ok |= 1u << i;
+        row[i] = e < r1 ? (src.in_perm ? __ldg(src.in_perm + e) : e) : 0u;
       }
-      if (src.lossy) {  // the key column is read here anyway: flag values the key words cannot restore
-        const bool l = valid && !(src.nulls && src.nulls[row]) &&
-                       key_value_lossy(src.type, src.data + (size_t)row * src.width);
-        if (__any_sync(0xffffffffu, l) && lane == 0) atomicOr(src.lossy, 1u);
-      }
-      const uint32_t vb = __ballot_sync(0xffffffffu, valid);
-      const int first = __ffs(vb) - 1;
-      // One vote per key: when every valid lane of the warp holds the same key
-      // (all-equal columns, heavy Zipf heads) lane `first` counts them all.
-      // Every lane executes the shuffle (full mask), valid or not.
-      bool same = true;
+      load_keys<KW, N>(src, row, ok, k);
 #pragma unroll
-      for (int j = 0; j < KW; ++j) {
-        const uint32_t kf = __shfl_sync(0xffffffffu, k[j], first < 0 ? 0 : first);
-        same &= (!valid || k[j] == kf);
-      }
-      if (__all_sync(0xffffffffu, same)) {
-        if (lane == first) {
-#pragma unroll
-          for (int p = 0; p < P; ++p) atomicAdd(&s_hist[p * RADIX + digit_of<KW, D>(k, p * D)], (uint32_t)__popc(vb));
+      for (int i = 0; i < N; ++i) {
+        const bool valid = ok >> i & 1u;
+        if (src.lossy) {  // the key column is read here anyway: flag values the key words cannot restore
+          const bool l = valid && !(src.nulls && src.nulls[row[i]]) &&
+                         key_value_lossy(src.type, src.data + (size_t)row[i] * src.width);
+          if (__any_sync(0xffffffffu, l) && lane == 0) atomicOr(src.lossy, 1u);
         }
-      } else if (valid) {
+        const uint32_t vb = __ballot_sync(0xffffffffu, valid);
+        const int first = __ffs(vb) - 1;
+        // One vote per key: when every valid lane of the warp holds the same key
+        // (all-equal columns, heavy Zipf heads) lane `first` counts them all.
+        // Every lane executes the shuffle (full mask), valid or not.
+        bool same = true;
 #pragma unroll
-        for (int p = 0; p < P; ++p) atomicAdd(&s_hist[p * RADIX + digit_of<KW, D>(k, p * D)], 1u);
+        for (int j = 0; j < KW; ++j) {
+          const uint32_t kf = __shfl_sync(0xffffffffu, k[i][j], first < 0 ? 0 : first);
+          same &= (!valid || k[i][j] == kf);
+        }
+        if (__all_sync(0xffffffffu, same)) {
+          if (lane == first) {
+#pragma unroll
+            for (int p = 0; p < P; ++p)
+              atomicAdd(&s_hist[(p * RADIX + digit_of<KW, D>(k[i], p * D)) * C + copy], (uint32_t)__popc(vb));
+          }
+        } else if (valid) {
+#pragma unroll
+          for (int p = 0; p < P; ++p) atomicAdd(&s_hist[(p * RADIX + digit_of<KW, D>(k[i], p * D)) * C + copy], 1u);
+        }
       }
     }
   }
   __syncthreads();
-  if (cur >= 0) {
-    uint32_t* h = hist + (size_t)cur * P * RADIX;
-    for (int i = threadIdx.x; i < P * RADIX; i += kSortBlock)
-      if (s_hist[i]) atomicAdd(h + i, s_hist[i]);
-  }
+  if (cur >= 0) flush(cur);
 }
 
 // --------------------------------------------------------------- onesweep
@@ -153,7 +225,8 @@ struct SweepParams {
   uint32_t* status;      // [ntiles][RADIX], zero on entry
   uint32_t* tile_counter;
   uint32_t* err;
-  int32_t pass;          // index of this pass's digit (bit offset = pass * D)
+  int32_t pass;          // index of this pass's digit in the histogram
+  int32_t shift;         // bit offset of the digit in the pass's key words
   int32_t npass;         // P
 };
 
@@ -168,48 +241,92 @@ constexpr int sweep_min_blocks(int kw, int d, int items, int block) {
                       : (block > 256 ? (sweep_min_blocks(kw, d, items) + 1) / 2 : 2 * sweep_min_blocks(kw, d, items));
 }
 
-// BLOCK threads, ITEMS keys per thread: a tile of BLOCK * ITEMS rows. Every
-// digit has its own thread in the per-digit steps (RADIX <= BLOCK).
-template <int KW, int D, int ITEMS, int BLOCK>
-__global__ void __launch_bounds__(BLOCK, sweep_min_blocks(KW, D, ITEMS, BLOCK)) k_sort_onesweep(const __grid_constant__ SweepParams S) {
+// Exclusive count of one digit over the segment's tiles before this one, from
+// their status words (p = the nearest predecessor's, `back` of them). The first
+// read takes one word: behind a full pipeline of tiles the nearest predecessor
+// that has published anything usually holds its inclusive count. While words
+// hold only their tile's own count the walk reads eight at a time, so a sort
+// whose tiles all start together (up to a few hundred) is not a chain of
+// dependent L2 reads, one a tile.
+template <int RADIX>
+__device__ __forceinline__ uint32_t sweep_lookback(const uint32_t* p, uint32_t back, uint32_t* err) {
+  constexpr int W = 8;
+  uint32_t excl = 0u, spins = 0u;
+  auto wait = [&]() {
+    if (++spins > kSpinLimit || ((spins & 63u) == 0u && ld_relaxed_u32(err) != 0u)) {
+      atomicOr(err, kErrTimeout);
+      return false;
+    }
+    __nanosleep(spins < 64 ? 32 : 128);
+    return true;
+  };
+  bool wide = false;
+  while (back > 0) {
+    if (!wide || back < W) {
+      const uint32_t v = ld_relaxed_u32(p), f = v & ~kStatMask;
+      if (f == 0u) {
+        if (!wait()) break;
+        continue;
+      }
+      excl += v & kStatMask;
+      if (f == kStatIncl) break;
+      p -= RADIX;
+      --back;
+      wide = true;
+    } else {
+      uint32_t v[W];
+#pragma unroll
+      for (int i = 0; i < W; ++i) v[i] = ld_relaxed_u32(p - (ptrdiff_t)i * RADIX);
+      uint32_t used = 0u;
+      bool done = false;
+#pragma unroll
+      for (int i = 0; i < W; ++i) {
+        const uint32_t f = v[i] & ~kStatMask;
+        if (used == (uint32_t)i && !done && f != 0u) {
+          excl += v[i] & kStatMask;
+          ++used;
+          done = f == kStatIncl;
+        }
+      }
+      if (done) break;
+      if (used == 0u && !wait()) break;
+      p -= (ptrdiff_t)used * RADIX;
+      back -= used;
+    }
+  }
+  return excl;
+}
+
+// One tile of the pass. FULL: every position holds a row (all tiles but the
+// last of a segment), so the position checks fall away.
+template <int KW, int D, int ITEMS, int BLOCK, bool FULL>
+__device__ __forceinline__ void sweep_tile(const SweepParams& S, uint32_t* smem, uint32_t tile, int sg, uint32_t lt,
+                                           uint32_t seg0, uint32_t seg1, uint32_t r0, uint32_t tile_n) {
   constexpr int RADIX = 1 << D;
   constexpr int NW = BLOCK / 32;
   constexpr uint32_t TILE = BLOCK * ITEMS;
-  static_assert(RADIX <= BLOCK, "one digit per thread");
-
-  extern __shared__ uint32_t smem[];
   uint32_t* s_whist = smem;                       // [NW][RADIX]
-  uint32_t* s_tile_base = s_whist + NW * RADIX;   // [RADIX]
-  uint32_t* s_glob = s_tile_base + RADIX;         // [RADIX]
+  uint32_t* s_glob = s_whist + NW * RADIX;        // [RADIX] output position of staged position 0
   uint32_t* s_scan = s_glob + RADIX;              // [NW + 1]
-  uint32_t* s_misc = s_scan + NW + 1;             // [4]
-  uint32_t* s_keys = s_misc + 4;                  // [TILE][KW]
+  uint32_t* s_keys = s_scan + NW + 1 + 4;         // [TILE][KW]
   uint32_t* s_vals = s_keys + TILE * KW;          // [TILE]
-
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (threadIdx.x == 0) s_misc[0] = atomicAdd(S.tile_counter, 1u);
-  for (int i = threadIdx.x; i < NW * RADIX; i += BLOCK) s_whist[i] = 0u;
-  __syncthreads();
-  const uint32_t tile = s_misc[0];
-  const int sg = find_segment(S.seg, tile);
-  const uint32_t lt = tile - __ldg(S.seg.tile_start + sg);
-  const uint32_t seg0 = __ldg(S.seg.seg_start + sg);
-  const uint32_t seg1 = __ldg(S.seg.seg_start + sg + 1);
-  const uint32_t r0 = seg0 + lt * TILE;
-  const uint32_t tile_n = min(TILE, seg1 - r0);
-  const int shift = S.pass * D;
+  const int shift = S.shift;
 
   // 1. load (warp-striped: element = r0 + warp*ITEMS*32 + k*32 + lane)
+  // Row ids are not needed before the staging: they are read behind the ranking,
+  // which keeps its registers to the keys and ranks.
   uint32_t key[ITEMS][KW];
-  uint32_t val[ITEMS];
   uint32_t rank[ITEMS];
+  const uint32_t off0 = (uint32_t)(warp * ITEMS * 32 + lane);
+  auto valid = [&](int k) { return FULL || off0 + k * 32 < tile_n; };
+  if (S.keys_in) {
 #pragma unroll
-  for (int k = 0; k < ITEMS; ++k) {
-    const uint32_t off = (uint32_t)(warp * ITEMS * 32 + k * 32 + lane);
-    const uint32_t e = r0 + off;
-    const bool valid = off < tile_n;
-    if (valid) {
-      if (S.keys_in) {
+    for (int k = 0; k < ITEMS; ++k) {
+      const uint32_t e = r0 + off0 + k * 32;
+#pragma unroll
+      for (int j = 0; j < KW; ++j) key[k][j] = 0u;
+      if (valid(k)) {
         if (KW == 1) {
           key[k][0] = __ldg(S.keys_in + e);
         } else if (KW == 2) {
@@ -226,26 +343,25 @@ __global__ void __launch_bounds__(BLOCK, sweep_min_blocks(KW, D, ITEMS, BLOCK)) 
             key[k][j + 3 < KW ? j + 3 : 0] = q.w;
           }
         }
-        val[k] = __ldg(S.vals_in + e);
-      } else {
-        const uint32_t row = S.src.in_perm ? __ldg(S.src.in_perm + e) : e;
-        make_key<KW>(S.src, row, key[k]);
-        val[k] = row;
       }
-    } else {
-#pragma unroll
-      for (int j = 0; j < KW; ++j) key[k][j] = 0u;
-      val[k] = 0u;
     }
+  } else {
+    uint32_t ok = 0u, row[ITEMS];
+#pragma unroll
+    for (int k = 0; k < ITEMS; ++k) {
+      const uint32_t e = r0 + off0 + k * 32;
+      if (valid(k)) ok |= 1u << k;
+      row[k] = valid(k) ? (S.src.in_perm ? __ldg(S.src.in_perm + e) : e) : 0u;
+    }
+    load_keys<KW, ITEMS>(S.src, row, FULL ? 0xffffffffu : ok, key);
   }
 
   // 2. warp-level stable ranking (order within a warp = (k, lane))
   const uint32_t lt_mask = lanemask_lt();
+  uint32_t* const whist = s_whist + warp * RADIX;
 #pragma unroll
   for (int k = 0; k < ITEMS; ++k) {
-    const uint32_t off = (uint32_t)(warp * ITEMS * 32 + k * 32 + lane);
-    const bool valid = off < tile_n;
-    uint32_t peers = __ballot_sync(0xffffffffu, valid);
+    uint32_t peers = FULL ? 0xffffffffu : __ballot_sync(0xffffffffu, valid(k));
     const uint32_t dk = digit_of<KW, D>(key[k], shift);
 #pragma unroll
     for (int b = 0; b < D; ++b) {
@@ -253,15 +369,22 @@ __global__ void __launch_bounds__(BLOCK, sweep_min_blocks(KW, D, ITEMS, BLOCK)) 
       const uint32_t bb = __ballot_sync(0xffffffffu, bit);
       peers &= bit ? bb : ~bb;
     }
-    const int leader = __ffs(peers) - 1;
+    const int leader = FULL ? 31 - __clz(peers) : (peers ? 31 - __clz(peers) : 0);
     uint32_t old = 0u;
-    if (valid && lane == leader) {
-      old = s_whist[warp * RADIX + dk];
-      s_whist[warp * RADIX + dk] = old + __popc(peers);
+    if (valid(k) && lane == leader) {
+      old = whist[dk];
+      whist[dk] = old + __popc(peers);
     }
-    old = __shfl_sync(0xffffffffu, old, leader < 0 ? 0 : leader);
+    old = __shfl_sync(0xffffffffu, old, leader);
     rank[k] = old + __popc(peers & lt_mask);
     __syncwarp();
+  }
+  uint32_t val[ITEMS];
+  const uint32_t* const ids = S.keys_in ? S.vals_in : S.src.in_perm;  // null: a row's id is its position
+#pragma unroll
+  for (int k = 0; k < ITEMS; ++k) {
+    const uint32_t e = r0 + off0 + k * 32;
+    val[k] = ids && valid(k) ? __ldg(ids + e) : e;
   }
   __syncthreads();
 
@@ -269,77 +392,59 @@ __global__ void __launch_bounds__(BLOCK, sweep_min_blocks(KW, D, ITEMS, BLOCK)) 
   const int t = threadIdx.x;
   uint32_t tile_count = 0u, seg_count = 0u;
   if (t < RADIX) {
-    for (int w = 0; w < NW; ++w) {
-      const uint32_t c = s_whist[w * RADIX + t];
-      s_whist[w * RADIX + t] = tile_count;
-      tile_count += c;
-    }
     seg_count = __ldg(S.hist + ((size_t)sg * S.npass + S.pass) * RADIX + t);
+#pragma unroll
+    for (int w = 0; w < NW; ++w) tile_count += s_whist[w * RADIX + t];
+    st_relaxed_u32(S.status + (size_t)tile * RADIX + t, (lt == 0 ? kStatIncl : kStatAgg) | tile_count);
   }
   uint32_t total;
   const uint32_t tile_excl = block_exclusive_sum<BLOCK>(t < RADIX ? tile_count : 0u, s_scan, total);
   const uint32_t seg_excl = block_exclusive_sum<BLOCK>(t < RADIX ? seg_count : 0u, s_scan, total);
-
-  // 4. decoupled look-back per digit over the segment's earlier tiles
-  if (t < RADIX) {
-    s_tile_base[t] = tile_excl;
-    uint32_t* st = S.status + (size_t)tile * RADIX + t;
-    uint32_t excl = 0u;
-    if (lt == 0) {
-      st_relaxed_u32(st, kStatIncl | tile_count);
-    } else {
-      st_relaxed_u32(st, kStatAgg | tile_count);
-      const uint32_t* p = st - RADIX;
-      uint32_t back = lt;
-      uint32_t spins = 0;
-      while (back > 0) {
-        const uint32_t v = ld_relaxed_u32(p);
-        const uint32_t f = v & ~kStatMask;
-        if (f == 0u) {
-          if (++spins > kSpinLimit || ((spins & 63u) == 0u && ld_relaxed_u32(S.err) != 0u)) {
-            atomicOr(S.err, kErrTimeout);
-            break;
-          }
-          __nanosleep(spins < 64 ? 32 : 128);
-          continue;
-        }
-        excl += v & kStatMask;
-        if (f == kStatIncl) break;
-        p -= RADIX;
-        --back;
-      }
-      st_relaxed_u32(st, kStatIncl | ((excl + tile_count) & kStatMask));
+  if (t < RADIX) {  // a warp's counts become the staged position of its first key of the digit
+    uint32_t at = tile_excl;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) {
+      const uint32_t c = s_whist[w * RADIX + t];
+      s_whist[w * RADIX + t] = at;
+      at += c;
     }
-    s_glob[t] = seg0 + seg_excl + excl;
   }
   __syncthreads();
 
-  // 5. stage the tile in shared memory in digit order
+  // 4. stage the tile in shared memory in digit order (every position is one
+  // of the tile's: the counts are those of the very keys staged)
 #pragma unroll
   for (int k = 0; k < ITEMS; ++k) {
-    const uint32_t off = (uint32_t)(warp * ITEMS * 32 + k * 32 + lane);
-    if (off < tile_n) {
-      const uint32_t dk = digit_of<KW, D>(key[k], shift);
-      const uint32_t lp = s_tile_base[dk] + s_whist[warp * RADIX + dk] + rank[k];
-      if (lp >= tile_n) {
-        atomicOr(S.err, kErrBounds);
-        continue;
-      }
+    if (valid(k)) {
+      const uint32_t lp = whist[digit_of<KW, D>(key[k], shift)] + rank[k];
 #pragma unroll
       for (int j = 0; j < KW; ++j) s_keys[lp * KW + j] = key[k][j];
       s_vals[lp] = val[k];
     }
   }
+
+  // 5. decoupled look-back per digit over the segment's earlier tiles
+  if (t < RADIX) {
+    uint32_t excl = 0u;
+    if (lt != 0) {
+      uint32_t* st = S.status + (size_t)tile * RADIX + t;
+      excl = sweep_lookback<RADIX>(st - RADIX, lt, S.err);
+      st_relaxed_u32(st, kStatIncl | ((excl + tile_count) & kStatMask));
+    }
+    s_glob[t] = seg0 + seg_excl + excl - tile_excl;
+  }
   __syncthreads();
 
   // 6. contiguous scatter per digit run
-  for (uint32_t i = threadIdx.x; i < tile_n; i += BLOCK) {
+#pragma unroll
+  for (int x = 0; x < ITEMS; ++x) {
+    const uint32_t i = threadIdx.x + x * BLOCK;
+    if (!FULL && i >= tile_n) break;
     uint32_t kk[KW];
 #pragma unroll
     for (int j = 0; j < KW; ++j) kk[j] = s_keys[i * KW + j];
-    const uint32_t d = digit_of<KW, D>(kk, shift);
-    const uint32_t g = s_glob[d] + (i - s_tile_base[d]);
-    if (g < seg0 || g >= seg1) {  // offsets inconsistent with the histogram: skip, report
+    const uint32_t g = s_glob[digit_of<KW, D>(kk, shift)] + i;
+    if (g - seg0 >= seg1 - seg0) {  // offsets inconsistent with the histogram: skip, report
       atomicOr(S.err, kErrBounds);
       continue;
     }
@@ -357,6 +462,29 @@ __global__ void __launch_bounds__(BLOCK, sweep_min_blocks(KW, D, ITEMS, BLOCK)) 
     }
     S.vals_out[g] = s_vals[i];
   }
+}
+
+// BLOCK threads, ITEMS keys per thread: a tile of BLOCK * ITEMS rows. Every
+// digit has its own thread in the per-digit steps (RADIX <= BLOCK).
+template <int KW, int D, int ITEMS, int BLOCK>
+__global__ void __launch_bounds__(BLOCK, sweep_min_blocks(KW, D, ITEMS, BLOCK)) k_sort_onesweep(const __grid_constant__ SweepParams S) {
+  constexpr int RADIX = 1 << D;
+  constexpr int NW = BLOCK / 32;
+  constexpr uint32_t TILE = BLOCK * ITEMS;
+  static_assert(RADIX <= BLOCK, "one digit per thread");
+  extern __shared__ uint32_t smem[];
+  uint32_t* s_misc = smem + NW * RADIX + RADIX + NW + 1;  // [4]
+  if (threadIdx.x == 0) s_misc[0] = atomicAdd(S.tile_counter, 1u);
+  for (int i = threadIdx.x; i < NW * RADIX; i += BLOCK) smem[i] = 0u;
+  __syncthreads();
+  const uint32_t tile = s_misc[0];
+  const int sg = find_segment(S.seg, tile);
+  const uint32_t lt = tile - __ldg(S.seg.tile_start + sg);
+  const uint32_t seg0 = __ldg(S.seg.seg_start + sg);
+  const uint32_t seg1 = __ldg(S.seg.seg_start + sg + 1);
+  const uint32_t r0 = seg0 + lt * TILE;
+  if (seg1 - r0 >= TILE) sweep_tile<KW, D, ITEMS, BLOCK, true>(S, smem, tile, sg, lt, seg0, seg1, r0, TILE);
+  else sweep_tile<KW, D, ITEMS, BLOCK, false>(S, smem, tile, sg, lt, seg0, seg1, r0, seg1 - r0);
 }
 
 // Which passes change the order, decided on the device so the host reads 16
@@ -572,7 +700,7 @@ template <int KW, int D, int ITEMS, int BLOCK>
 static size_t sweep_smem() {
   constexpr int RADIX = 1 << D;
   constexpr int NW = BLOCK / 32;
-  return sizeof(uint32_t) * ((size_t)NW * RADIX + 2 * RADIX + NW + 1 + 4 + (size_t)BLOCK * ITEMS * (KW + 1));
+  return sizeof(uint32_t) * ((size_t)NW * RADIX + RADIX + NW + 1 + 4 + (size_t)BLOCK * ITEMS * (KW + 1));
 }
 
 template <int KW, int D, int ITEMS, int BLOCK>
@@ -588,7 +716,7 @@ template <int KW, int D>
 static int launch_hist(const KeySrc& src, const SegInfo& seg, uint32_t tile_rows, uint32_t ntiles, uint32_t* hist,
                        cudaStream_t s) {
   constexpr int P = (KW * 32 + D - 1) / D;
-  const size_t smem = sizeof(uint32_t) * P * (1 << D);
+  const size_t smem = sizeof(uint32_t) * P * (1 << D) * kHistCopies<KW>;
   YQ_TRY(kernel_allow_smem((const void*)k_sort_histogram<KW, D>, smem));
   int grid = sm_count() * 4;
   if ((uint32_t)grid > ntiles) grid = (int)ntiles;
@@ -914,6 +1042,7 @@ int sort_segments_impl(const KeyJob* jobs, int njobs, uint32_t rows, const uint3
     YQ_TRY_CUDA(cudaMemsetAsync(d_misc, 0, 64 * sizeof(uint32_t), s));
 
     KeySrc src;
+    src.nsel = 0;
     src.data = static_cast<const char*>(cc.data);
     src.nulls = c.nulls;
     src.in_perm = perm_in;
@@ -986,6 +1115,28 @@ int sort_segments_impl(const KeyJob* jobs, int njobs, uint32_t rows, const uint3
         } else {
           kq = kp;
         }
+        // A nullable 8-byte key has three words, which take the four-word
+        // kernels; when one value word is the same in every row (dates, ids
+        // below 2^32) two words are left, and a pass moves 12 bytes a row
+        // instead of 20. Only nullable keys: their sorted key words are
+        // compared, never decoded.
+        if (c.nulls && kp.sh.kw == 4 && kq.sh.kw == 4) {
+          std::vector<int> kept_words, kept;
+          for (int w = 0; w < 4; ++w) {
+            bool all = true;
+            for (int q = 0; q < ppw && all; ++q) all = common[w * ppw + q] >= 0;
+            if (!all) kept_words.push_back(w);
+          }
+          if (kept_words.size() <= 2 && pick_kernels(2, kp.D, 0, kq.K)) {
+            kq.sh.kw = 2;
+            kq.P = 2 * ppw;
+            kq.tile_rows = kq.K.tile_rows();
+            src.nsel = (int)kept_words.size();
+            for (int j = 0; j < src.nsel; ++j) src.sel[j] = (int8_t)kept_words[j];
+          } else {
+            kq = kp;
+          }
+        }
       }
     }
     if (keys_out) *kw_out = kq.sh.kw;
@@ -1015,6 +1166,13 @@ int sort_segments_impl(const KeyJob* jobs, int njobs, uint32_t rows, const uint3
       Sp.tile_counter = d_misc + i;
       Sp.err = d_err;
       Sp.pass = passes[i];
+      int word = passes[i] * kq.D / 32, bit = passes[i] * kq.D % 32;
+      for (int j = 0; j < src.nsel; ++j)
+        if (src.sel[j] == word) {
+          word = j;
+          break;
+        }
+      Sp.shift = word * 32 + bit;
       Sp.npass = kp.P;
       // algorithmic bytes: keys + row ids in, keys + row ids out (the first
       // pass reads the raw key (+ incoming permutation), the last writes ids only)

@@ -19,6 +19,8 @@ struct KeySrc {
   int32_t desc;
   int32_t nulls_first;
   int32_t null_word;    // 1: word `vwords` is the null flag
+  int32_t nsel;         // non-zero: the passes' key is words sel[0], sel[1] of a four-word key
+  int8_t sel[4];        // (the other words are the same in every row)
   uint32_t* lossy;      // optional: the histogram sets it when a value would not survive the key words
 };
 
@@ -41,21 +43,30 @@ __device__ __forceinline__ bool key_value_lossy(int type, const char* p) {
 
 __device__ __forceinline__ uint32_t bswap(uint32_t x) { return __byte_perm(x, 0, 0x0123); }
 
+// Order-preserving word of a float's bits: -0.0 ties +0.0, NaN above +inf.
+__device__ __forceinline__ uint32_t float_key(uint32_t b) {
+  if ((b & 0x7fffffffu) == 0u) b = 0u;
+  else if ((b & 0x7fffffffu) > 0x7f800000u) b = 0x7fc00000u;
+  return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+}
+
 // Key words of the value stored at `p` (generic pointer: global or shared).
 template <int KW>
 __device__ __forceinline__ void make_key_ptr(const KeySrc& s, const char* p, bool is_null, uint32_t (&k)[KW]) {
 #pragma unroll
   for (int j = 0; j < KW; ++j) k[j] = 0u;
+  // Every NULL has one key, below its null word any: for 8-byte integers that
+  // of 0, so that a high word the values share (dates, ids below 2^32) is
+  // shared by all rows and takes no pass.
+  if (is_null && s.null_word && KW > 1 && (s.type == YQ_INT64 || s.type == YQ_DATETIME)) {
+    const uint32_t inv = s.desc ? 0xffffffffu : 0u;
+    k[0] = inv;
+    k[KW > 1 ? 1 : 0] = 0x80000000u ^ inv;
+  }
   if (!is_null) {
     switch (s.type) {
       case YQ_INT32: k[0] = *reinterpret_cast<const uint32_t*>(p) ^ 0x80000000u; break;
-      case YQ_FLOAT32: {
-        uint32_t b = *reinterpret_cast<const uint32_t*>(p);
-        if ((b & 0x7fffffffu) == 0u) b = 0u;                                               // -0.0 ties +0.0
-        else if ((b & 0x7f800000u) == 0x7f800000u && (b & 0x007fffffu)) b = 0x7fc00000u;  // NaN above +inf
-        k[0] = (b & 0x80000000u) ? ~b : (b | 0x80000000u);
-        break;
-      }
+      case YQ_FLOAT32: k[0] = float_key(*reinterpret_cast<const uint32_t*>(p)); break;
       case YQ_INT64:
       case YQ_DATETIME: {
         const uint2 v = *reinterpret_cast<const uint2*>(p);
