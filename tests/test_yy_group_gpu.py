@@ -125,3 +125,32 @@ def test_tiles_inside_one_group(cuda, layout):
     q = rng.integers(-1000, 1000, n).astype(np.int64)
     check([(k, A.INT32, None), (v, A.FLOAT32, vn), (q, A.INT64, None)], 0,
           ALL_AGGS([1]) + [(A.AGG_SUM, 2), (A.AGG_MIN, 2)])  # eight aggregates, the most a call takes
+
+
+@pytest.mark.parametrize("ktype", [A.INT32, A.INT64, A.DATETIME])
+@pytest.mark.parametrize("rows,distinct", [(100_000, 1), (100_001, 50), (131_073, 96), (262_147, 97), (300_007, 511)])
+def test_few_distinct_keys(cuda, ktype, rows, distinct):
+    """Around the limits of the sort-free path (100,000 rows, 96 keys, the
+    accumulators' room): keys at the type's ends and -1, key null bytes with
+    and without a NULL, inputs with and without NULLs, all numeric types."""
+    rng = np.random.default_rng(rows + distinct)
+    dt = np.int32 if ktype == A.INT32 else np.int64
+    pool = np.unique(np.concatenate([np.array([-1, np.iinfo(dt).min, np.iinfo(dt).max, 0], dt),
+                                     rng.integers(-1000, 1000, 2000).astype(dt) * dt(7)]))
+    pool = rng.permutation(pool)[:distinct]
+    k = pool[rng.integers(0, distinct, rows)]
+    k[:distinct] = pool
+    no_null, one_null = np.zeros(rows, bool), np.zeros(rows, bool)
+    one_null[rows // 2] = True
+    i32 = rng.integers(-(1 << 31), 1 << 31, rows).astype(np.int32)
+    f32 = rng.normal(0, 100, rows).astype(np.float32)
+    i64 = rng.integers(-(1 << 50), 1 << 50, rows).astype(np.int64)
+    f64 = rng.normal(0, 1e6, rows)
+    f32n = rng.random(rows) < 0.5
+    f32n[k == pool[0]] = True  # a group without a value
+    inputs = [(i32, A.INT32, None), (f32, A.FLOAT32, f32n), (i64, A.INT64, None), (f64, A.FLOAT64, None)]
+    for kn in (None, no_null, one_null):
+        cols = [(k, ktype, kn)] + inputs
+        check(cols, 0, [(A.AGG_COUNT_STAR, 0), (A.AGG_SUM, 1), (A.AGG_SUM, 2), (A.AGG_MIN, 1), (A.AGG_COUNT, 2),
+                        (A.AGG_MAX, 2), (A.AGG_AVG, 4), (A.AGG_AVG, 1)])
+        check(cols, 0, [(A.AGG_MIN, 4), (A.AGG_MAX, 3), (A.AGG_SUM, 3), (A.AGG_MIN, 2)])

@@ -22,9 +22,18 @@
 //   k_group_span      each group that crosses tiles, from the tile where it
 //                     starts: its tiles' partial records folded in tile order
 //                     (fixed tree), output row written
-// No atomics: every floating-point sum is added in an order fixed by the
+// No floating-point atomics: every sum is added in an order fixed by the
 // data's sorted layout, so a query gives the same bits on every run.
+//
+// Integer keys of few distinct values (up to kFewGroups) skip the sort:
+//   k_few_find        the distinct keys, through a hash table per block (a NULL
+//                     key or too many keys send the call to the sort)
+//   k_few_order       their ascending order = the group indices
+//   k_few_accumulate  one pass over the input columns into accumulators that
+//                     each thread owns in shared memory
+//   k_few_finish      each group's partials folded in block order
 #include <climits>
+#include <cstring>
 
 #include "yq_common.cuh"
 #include "yq_sort.cuh"
@@ -469,6 +478,344 @@ __global__ void __launch_bounds__(kGroupThreads) k_group_span(const __grid_const
   }
 }
 
+// ------------------------------------------------------- few distinct keys
+// With few groups the sort, its permutation and the reads through it are most
+// of the work (32M rows, 11 groups, five aggregates: 1.63 ms of kernels for
+// 384 MB of input). Here the input is read once to find the keys and once to
+// accumulate. Each thread owns an accumulator per group and aggregate in
+// shared memory (element [group][thread], so a warp's 32 updates hit 32
+// banks whatever groups its rows belong to) and adds its rows in row order;
+// threads, then blocks, fold in a fixed tree. So sums need no atomics and the
+// bits do not depend on scheduling. Latency-bound on the shared-memory
+// read-modify-writes; eight rows a thread are loaded ahead.
+// The group limit is the accumulators': at 28 bytes a thread and group, 50
+// groups leave one block of 128 threads on an SM.
+constexpr int kFewThreads = 128;
+constexpr int kFewItems = 8;
+constexpr uint32_t kFewGroups = 96;
+constexpr uint32_t kFewSlots = 512;          // hash slots, at most a fifth full
+constexpr int kFewFindThreads = 256;
+constexpr unsigned long long kNoKey = ~0ull;  // empty slot; the key of that value has a flag of its own
+
+struct FewTable {
+  unsigned long long keys[kFewSlots];  // kNoKey on entry
+  uint32_t count, has_last, overflow, ngroups;  // zero on entry, as all below
+  uint32_t last_gid, pad;
+  uint32_t gid[kFewSlots];
+  unsigned long long group_key[kFewGroups];
+};
+
+// 4-byte keys zero-extended (never kNoKey), 8-byte keys as they are.
+__device__ __forceinline__ unsigned long long few_key(const yq_column& k, uint32_t r) {
+  return k.width == 4 ? (unsigned long long)__ldg(static_cast<const uint32_t*>(k.data) + r)
+                      : __ldg(static_cast<const unsigned long long*>(k.data) + r);
+}
+__device__ __forceinline__ uint32_t few_hash(unsigned long long k) {
+  return (uint32_t)((k * 0x9e3779b97f4a7c15ull) >> 55);  // the top 9 bits
+}
+static_assert(kFewSlots == 512, "few_hash gives nine bits");
+
+// Puts `key` into the table; false when it holds too many keys.
+__device__ __forceinline__ bool few_insert(unsigned long long* keys, uint32_t* count, unsigned long long key) {
+  uint32_t h = few_hash(key);
+  for (uint32_t n = 0; n < kFewSlots; ++n, h = (h + 1) & (kFewSlots - 1)) {
+    unsigned long long cur = *reinterpret_cast<volatile unsigned long long*>(keys + h);
+    if (cur == key) return true;
+    if (cur != kNoKey) continue;
+    cur = atomicCAS(keys + h, kNoKey, key);
+    if (cur == kNoKey) return atomicAdd(count, 1u) < kFewGroups;
+    if (cur == key) return true;
+  }
+  return false;
+}
+
+__global__ void __launch_bounds__(kFewFindThreads) k_few_find(const yq_column key, uint32_t rows, FewTable* T) {
+  __shared__ unsigned long long s_keys[kFewSlots];
+  __shared__ uint32_t s_count, s_last, s_over;
+  for (uint32_t i = threadIdx.x; i < kFewSlots; i += kFewFindThreads) s_keys[i] = kNoKey;
+  if (threadIdx.x == 0) s_count = s_last = s_over = 0u;
+  __syncthreads();
+  constexpr uint32_t STEP = kFewFindThreads * kFewItems;
+  bool ok = true;
+  for (unsigned long long base = (unsigned long long)blockIdx.x * STEP; base < rows;
+       base += (unsigned long long)gridDim.x * STEP) {
+    // another thread or block has found too many keys: the table is not used
+    if (*reinterpret_cast<volatile uint32_t*>(&s_over) || ld_relaxed_u32(&T->overflow)) break;
+    unsigned long long k[kFewItems];
+    bool in[kFewItems];
+#pragma unroll
+    for (int q = 0; q < kFewItems; ++q) {
+      const unsigned long long r = base + q * kFewFindThreads + threadIdx.x;
+      in[q] = r < rows;
+      k[q] = in[q] ? few_key(key, (uint32_t)r) : 0ull;
+      if (in[q] && key.nulls && key.nulls[r]) ok = false;  // a NULL group's key cell is its first row's: the sort finds it
+    }
+#pragma unroll
+    for (int q = 0; q < kFewItems; ++q) {
+      if (!in[q]) continue;
+      if (k[q] == kNoKey) s_last = 1u;
+      else if (ok && !few_insert(s_keys, &s_count, k[q])) ok = false;
+    }
+    if (!ok) s_over = 1u;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    if (s_last) atomicOr(&T->has_last, 1u);
+    if (s_over) atomicOr(&T->overflow, 1u);
+  }
+  if (s_over) return;
+  for (uint32_t i = threadIdx.x; i < kFewSlots; i += kFewFindThreads)
+    if (s_keys[i] != kNoKey && !few_insert(T->keys, &T->count, s_keys[i])) atomicOr(&T->overflow, 1u);
+}
+
+// Group index of every key: ascending signed order.
+__global__ void __launch_bounds__(kFewSlots) k_few_order(FewTable* T, int width) {
+  __shared__ unsigned long long s_keys[kFewSlots];
+  const uint32_t i = threadIdx.x;
+  const unsigned long long mine = T->keys[i];
+  s_keys[i] = mine;
+  __syncthreads();
+  const uint32_t n = T->count + (T->has_last ? 1u : 0u);
+  if (T->overflow || n > kFewGroups) {
+    if (i == 0) T->overflow = 1u;
+    return;
+  }
+  auto value = [width](unsigned long long k) { return width == 4 ? (long long)(int32_t)(uint32_t)k : (long long)k; };
+  const bool has_last = T->has_last != 0u;  // the key ~0: signed -1
+  if (mine != kNoKey) {
+    uint32_t rank = has_last && -1ll < value(mine) ? 1u : 0u;
+    for (uint32_t j = 0; j < kFewSlots; ++j)
+      if (s_keys[j] != kNoKey && value(s_keys[j]) < value(mine)) ++rank;
+    T->gid[i] = rank;
+    T->group_key[rank] = mine;
+  }
+  if (i == 0) {
+    if (has_last) {
+      uint32_t rank = 0;
+      for (uint32_t j = 0; j < kFewSlots; ++j)
+        if (s_keys[j] != kNoKey && value(s_keys[j]) < -1ll) ++rank;
+      T->last_gid = rank;
+      T->group_key[rank] = kNoKey;
+    }
+    T->ngroups = n;
+  }
+}
+
+// What a thread keeps per group, [group][thread] arrays one after another:
+// its rows, per nullable input its non-NULL values, per aggregate its value.
+struct FewAcc {
+  int32_t cnt_off;  // count array of the aggregate (0: the row counts)
+  int32_t val_off;  // value array (-1: a count)
+  int32_t val_size;
+};
+struct FewParams {
+  GroupParams P;
+  yq_column key;
+  FewAcc acc[YQ_MAX_AGGREGATES];
+  int32_t bytes;      // of all arrays, for one group and thread
+  uint32_t ngroups;
+  uint32_t rows_per_block;
+  const FewTable* T;
+  GPart* part;        // [blocks][groups][nagg]
+  yq_column out_key;
+};
+
+__device__ __forceinline__ int32_t ordered32(float f) {
+  uint32_t u = f != f ? 0x7fc00000u : __float_as_uint(f);
+  u = (u >> 31) ? ~u : (u | 0x80000000u);
+  return (int32_t)(u ^ 0x80000000u);
+}
+// ordered32's keys as ordered() gives them for the same value in double.
+__device__ __forceinline__ long long widen_ordered32(int32_t k) {
+  uint32_t u = (uint32_t)k ^ 0x80000000u;
+  u = (u >> 31) ? (u & 0x7fffffffu) : ~u;
+  return ordered((double)__uint_as_float(u));
+}
+
+template <typename T>
+__device__ __forceinline__ void few_load(const GAgg& a, const uint32_t (&row)[kFewItems], uint32_t use,
+                                         T (&v)[kFewItems]) {
+#pragma unroll
+  for (int q = 0; q < kFewItems; ++q) v[q] = (use >> q & 1u) ? __ldg(static_cast<const T*>(a.data) + row[q]) : T(0);
+}
+
+// One aggregate over a thread's rows: F folds a value into the accumulator.
+template <typename T, typename A, typename F>
+__device__ __forceinline__ void few_fold(const GAgg& a, A* acc, const uint32_t (&row)[kFewItems],
+                                         const uint32_t (&g)[kFewItems], uint32_t use, F f) {
+  T v[kFewItems];
+  few_load<T>(a, row, use, v);
+#pragma unroll
+  for (int q = 0; q < kFewItems; ++q)
+    if (use >> q & 1u) {
+      A* p = acc + g[q] * kFewThreads + threadIdx.x;
+      *p = f(*p, v[q]);
+    }
+}
+
+__global__ void __launch_bounds__(kFewThreads) k_few_accumulate(const __grid_constant__ FewParams F) {
+  extern __shared__ __align__(16) char s_few[];
+  unsigned long long* s_keys = reinterpret_cast<unsigned long long*>(s_few);
+  uint32_t* s_gid = reinterpret_cast<uint32_t*>(s_keys + kFewSlots);
+  char* s_acc = reinterpret_cast<char*>(s_gid + kFewSlots);
+  const uint32_t G = F.ngroups, tid = threadIdx.x;
+  const size_t unit = (size_t)G * kFewThreads;  // elements of one array
+  for (uint32_t i = tid; i < kFewSlots; i += kFewThreads) {
+    s_keys[i] = F.T->keys[i];
+    s_gid[i] = F.T->gid[i];
+  }
+  for (size_t i = tid * 4; i < unit * F.bytes; i += kFewThreads * 4) *reinterpret_cast<uint32_t*>(s_acc + i) = 0u;
+  __syncthreads();
+  for (int j = 0; j < F.P.nagg; ++j) {  // MIN / MAX start at their identity
+    const int kind = F.P.a[j].kind;
+    if (kind != YQ_AGG_MIN && kind != YQ_AGG_MAX) continue;
+    for (uint32_t g = 0; g < G; ++g) {
+      char* p = s_acc + unit * F.acc[j].val_off + (size_t)(g * kFewThreads + tid) * F.acc[j].val_size;
+      if (F.acc[j].val_size == 4) *reinterpret_cast<int32_t*>(p) = kind == YQ_AGG_MIN ? INT_MAX : INT_MIN;
+      else *reinterpret_cast<long long*>(p) = kind == YQ_AGG_MIN ? LLONG_MAX : LLONG_MIN;
+    }
+  }
+  uint32_t* const rows_acc = reinterpret_cast<uint32_t*>(s_acc);
+  const unsigned long long r_begin = (unsigned long long)blockIdx.x * F.rows_per_block;
+  const unsigned long long r_end = min((unsigned long long)F.P.rows, r_begin + F.rows_per_block);
+  const uint32_t last_gid = F.T->last_gid;
+  for (unsigned long long base = r_begin; base < r_end; base += kFewThreads * kFewItems) {
+    uint32_t row[kFewItems], g[kFewItems], in = 0u;
+    unsigned long long k[kFewItems];
+#pragma unroll
+    for (int q = 0; q < kFewItems; ++q) {
+      const unsigned long long r = base + q * kFewThreads + tid;
+      row[q] = r < r_end ? (uint32_t)r : 0u;
+      if (r < r_end) in |= 1u << q;
+      k[q] = few_key(F.key, row[q]);
+    }
+#pragma unroll
+    for (int q = 0; q < kFewItems; ++q) {
+      if (k[q] == kNoKey) {
+        g[q] = last_gid;
+      } else {
+        uint32_t h = few_hash(k[q]);
+        for (uint32_t n = 0; n < kFewSlots && s_keys[h] != k[q]; ++n) h = (h + 1) & (kFewSlots - 1);
+        g[q] = s_gid[h];
+      }
+      if (g[q] >= G) {  // cannot be: k_few_find saw every key
+        in &= ~(1u << q);
+        g[q] = 0u;
+        atomicOr(F.P.err, kErrBounds);
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < kFewItems; ++q)
+      if (in >> q & 1u) ++rows_acc[g[q] * kFewThreads + tid];
+    for (int j = 0; j < F.P.nagg; ++j) {
+      const GAgg& a = F.P.a[j];
+      const FewAcc& A = F.acc[j];
+      uint32_t use = in;
+      if (a.kind == YQ_AGG_COUNT_STAR) continue;
+      if (a.nulls) {
+        uint32_t* cnt = reinterpret_cast<uint32_t*>(s_acc + unit * A.cnt_off);
+#pragma unroll
+        for (int q = 0; q < kFewItems; ++q)
+          if (use >> q & 1u) {
+            if (a.nulls[row[q]]) use &= ~(1u << q);
+            else ++cnt[g[q] * kFewThreads + tid];
+          }
+      }
+      if (A.val_off < 0) continue;
+      char* const val = s_acc + unit * A.val_off;
+      if (a.kind == YQ_AGG_SUM || a.kind == YQ_AGG_AVG) {
+        if (a.type == YQ_FLOAT32)
+          few_fold<float>(a, reinterpret_cast<double*>(val), row, g, use, [](double x, float v) { return x + (double)v; });
+        else if (a.type == YQ_FLOAT64)
+          few_fold<double>(a, reinterpret_cast<double*>(val), row, g, use, [](double x, double v) { return x + v; });
+        else if (a.type == YQ_INT32)
+          few_fold<int32_t>(a, reinterpret_cast<long long*>(val), row, g, use,
+                            [](long long x, int32_t v) { return (long long)((unsigned long long)x + (unsigned long long)(long long)v); });
+        else
+          few_fold<long long>(a, reinterpret_cast<long long*>(val), row, g, use,
+                              [](long long x, long long v) { return (long long)((unsigned long long)x + (unsigned long long)v); });
+      } else {
+        const bool lo = a.kind == YQ_AGG_MIN;
+        if (a.type == YQ_FLOAT32)
+          few_fold<float>(a, reinterpret_cast<int32_t*>(val), row, g, use, [lo](int32_t x, float v) {
+            const int32_t o = ordered32(v);
+            return lo ? min(x, o) : max(x, o);
+          });
+        else if (a.type == YQ_INT32)
+          few_fold<int32_t>(a, reinterpret_cast<int32_t*>(val), row, g, use,
+                            [lo](int32_t x, int32_t v) { return lo ? min(x, v) : max(x, v); });
+        else if (a.type == YQ_FLOAT64)
+          few_fold<double>(a, reinterpret_cast<long long*>(val), row, g, use, [lo](long long x, double v) {
+            const long long o = ordered(v);
+            return lo ? min(x, o) : max(x, o);
+          });
+        else
+          few_fold<long long>(a, reinterpret_cast<long long*>(val), row, g, use,
+                              [lo](long long x, long long v) { return lo ? min(x, v) : max(x, v); });
+      }
+    }
+  }
+  __syncthreads();
+  // each (group, aggregate): the block's threads folded by one warp, a lane's
+  // threads in order and then the lanes pairwise
+  const int lane = tid & 31, warp = tid >> 5;
+  for (uint32_t x = warp; x < G * (uint32_t)F.P.nagg; x += kFewThreads / 32) {
+    const uint32_t g = x / F.P.nagg;
+    const int j = (int)(x % F.P.nagg);
+    const GAgg& a = F.P.a[j];
+    const FewAcc& A = F.acc[j];
+    const bool flt = is_float(a.type);
+    GPart acc = part_identity(a.kind);
+#pragma unroll
+    for (int t = 0; t < kFewThreads / 32; ++t) {
+      const size_t e = (size_t)g * kFewThreads + t * 32 + lane;
+      GPart p;
+      p.cnt = reinterpret_cast<const uint32_t*>(s_acc + unit * A.cnt_off)[e];
+      p.v = 0ull;
+      if (A.val_off >= 0) {
+        const char* val = s_acc + unit * A.val_off;
+        if (A.val_size == 8) p.v = reinterpret_cast<const unsigned long long*>(val)[e];
+        else {
+          const int32_t v = reinterpret_cast<const int32_t*>(val)[e];
+          p.v = p.cnt == 0 ? part_identity(a.kind).v
+                           : (unsigned long long)(a.type == YQ_FLOAT32 ? widen_ordered32(v) : (long long)v);
+        }
+      }
+      acc = part_combine(a.kind, flt, acc, p);
+    }
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const GPart o{__shfl_down_sync(0xffffffffu, acc.cnt, d), __shfl_down_sync(0xffffffffu, acc.v, d)};
+      if ((lane & (2 * d - 1)) == 0) acc = part_combine(a.kind, flt, acc, o);
+    }
+    if (lane == 0) F.part[((size_t)blockIdx.x * G + g) * F.P.nagg + j] = acc;
+  }
+}
+
+// One warp per (group, aggregate): the blocks' partials in block order.
+__global__ void __launch_bounds__(32) k_few_finish(const __grid_constant__ FewParams F, uint32_t nblocks) {
+  const uint32_t g = blockIdx.x;
+  const int j = blockIdx.y, lane = threadIdx.x;
+  if (j == 0 && lane == 0) {
+    const unsigned long long k = F.T->group_key[g];
+    if (F.out_key.width == 4) static_cast<uint32_t*>(F.out_key.data)[g] = (uint32_t)k;
+    else static_cast<unsigned long long*>(F.out_key.data)[g] = k;
+    if (F.out_key.nulls) const_cast<uint8_t*>(F.out_key.nulls)[g] = 0;
+  }
+  if (j >= F.P.nagg) return;
+  const GAgg& a = F.P.a[j];
+  const bool flt = is_float(a.type);
+  GPart acc = part_identity(a.kind);
+  for (uint32_t b = lane; b < nblocks; b += 32)
+    acc = part_combine(a.kind, flt, acc, F.part[((size_t)b * F.ngroups + g) * F.P.nagg + j]);
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const GPart o{__shfl_down_sync(0xffffffffu, acc.cnt, d), __shfl_down_sync(0xffffffffu, acc.v, d)};
+    if ((lane & (2 * d - 1)) == 0) acc = part_combine(a.kind, flt, acc, o);
+  }
+  if (lane == 0) part_write(a, F.P.out[j], g, acc);
+}
+
 int out_type(int32_t kind, int32_t in) {
   switch (kind) {
     case YQ_AGG_COUNT:
@@ -484,6 +831,116 @@ int type_width(int32_t t) { return (t == YQ_INT32 || t == YQ_FLOAT32) ? 4 : 8; }
 unsigned grid_for(uint64_t n, unsigned per_block) {
   const uint64_t g = (n + per_block - 1) / per_block;
   return (unsigned)(g < 1 ? 1 : (g > 65535 ? 65535 : g));
+}
+
+// Blocks the accumulation runs at most (its partials are sized for them).
+constexpr int kFewBlocksPerSm = 8;
+
+size_t few_workspace_bytes(int32_t nagg) {
+  WsSize w;
+  w.add<FewTable>(1);
+  w.add<GPart>((size_t)sm_count() * kFewBlocksPerSm * kFewGroups * (nagg > 0 ? nagg : 1));
+  w.add<uint32_t>(4);
+  return w.total();
+}
+
+// Rows from which the search for few distinct keys pays for itself when it
+// fails (a search that meets too many keys stops within its first steps, but
+// its launches and its read-back take about 25 us).
+constexpr uint32_t kFewMinRows = 100000;
+
+bool few_applies(const yq_column& key, uint32_t rows) {
+  return rows >= kFewMinRows && (key.type == YQ_INT32 || key.type == YQ_INT64 || key.type == YQ_DATETIME);
+}
+
+// The sort-free path. *done = false: the keys are too many (or one is NULL)
+// and nothing was written.
+int group_by_few(const GroupParams& P, const yq_column& key, const yq_column& out_key, uint32_t capacity,
+                 uint32_t* groups, void* few_ws, size_t few_bytes, cudaStream_t s, bool* done) {
+  *done = false;
+  Workspace ws;
+  YQ_TRY(ws.acquire(few_ws, few_bytes, few_workspace_bytes(P.nagg), s));
+  FewTable* T = ws.take<FewTable>(1);
+  GPart* part = ws.take<GPart>((size_t)sm_count() * kFewBlocksPerSm * kFewGroups * (P.nagg > 0 ? P.nagg : 1));
+  uint32_t* d_err = ws.take<uint32_t>(4);
+  YQ_TRY_CUDA(cudaMemsetAsync(T->keys, 0xff, sizeof(T->keys), s));
+  YQ_TRY_CUDA(cudaMemsetAsync(&T->count, 0, sizeof(FewTable) - sizeof(T->keys), s));
+  const unsigned step = kFewFindThreads * kFewItems;
+  unsigned grid = grid_for(P.rows, step);
+  if (grid > (unsigned)sm_count() * 8) grid = (unsigned)sm_count() * 8;
+  {
+    ProfScope ps("group_few_find", s, (double)P.rows * key.width);
+    k_few_find<<<grid, kFewFindThreads, 0, s>>>(key, P.rows, T);
+    YQ_CHECK_LAUNCH();
+  }
+  k_few_order<<<1, kFewSlots, 0, s>>>(T, key.width);
+  YQ_CHECK_LAUNCH();
+  uint32_t head[4];  // count, has_last, overflow, ngroups
+  YQ_TRY(d2h_sync(head, &T->count, sizeof(head), s));
+  const uint32_t G = head[3];
+  if (head[2] || G == 0) return YQ_OK;
+  FewParams F;
+  F.P = P;
+  F.P.err = d_err;
+  F.key = key;
+  F.out_key = out_key;
+  F.ngroups = G;
+  F.T = T;
+  F.part = part;
+  // arrays in descending element size, so each stays aligned
+  int off = 0;
+  auto value_size = [&](int j) {
+    const GAgg& a = P.a[j];
+    if (a.kind == YQ_AGG_COUNT || a.kind == YQ_AGG_COUNT_STAR) return 0;
+    return a.kind == YQ_AGG_SUM || a.kind == YQ_AGG_AVG || type_width(a.type) == 8 ? 8 : 4;
+  };
+  off = 4;  // the row counts; padded to 8 with the 4-byte arrays placed first
+  for (int j = 0; j < P.nagg; ++j) {
+    F.acc[j] = FewAcc{0, -1, 0};
+    if (P.a[j].kind != YQ_AGG_COUNT_STAR && P.a[j].nulls) {
+      F.acc[j].cnt_off = off;
+      off += 4;
+    }
+  }
+  for (const int size : {4, 8}) {
+    for (int j = 0; j < P.nagg; ++j) {
+      if (value_size(j) != size) continue;
+      F.acc[j].val_off = off;
+      F.acc[j].val_size = size;
+      off += size;
+    }
+  }
+  F.bytes = off;
+  const size_t smem = kFewSlots * 12 + (size_t)G * kFewThreads * off;
+  if (smem > 220 * 1024) return YQ_OK;  // too many accumulators for one block
+  if (G > capacity) {
+    *groups = G;
+    *done = true;
+    return YQ_ERR_CAPACITY;
+  }
+  YQ_TRY(kernel_allow_smem((const void*)k_few_accumulate, smem));
+  int per_sm = kernel_blocks_per_sm((const void*)k_few_accumulate, kFewThreads, smem);
+  if (per_sm > kFewBlocksPerSm) per_sm = kFewBlocksPerSm;
+  unsigned blocks = grid_for(P.rows, kFewThreads * kFewItems);
+  if (blocks > (unsigned)(sm_count() * per_sm)) blocks = (unsigned)(sm_count() * per_sm);
+  F.rows_per_block = (uint32_t)align_up(((size_t)P.rows + blocks - 1) / blocks, kFewThreads * kFewItems);
+  blocks = (P.rows + F.rows_per_block - 1) / F.rows_per_block;
+  YQ_TRY_CUDA(cudaMemsetAsync(d_err, 0, 4 * sizeof(uint32_t), s));
+  double in_bytes = (double)P.rows * key.width;
+  for (int j = 0; j < P.nagg; ++j)
+    if (P.a[j].data) in_bytes += (double)P.rows * (type_width(P.a[j].type) + (P.a[j].nulls ? 1 : 0));
+  {
+    ProfScope ps("group_few_accumulate", s, in_bytes);
+    k_few_accumulate<<<blocks, kFewThreads, smem, s>>>(F);
+    YQ_CHECK_LAUNCH();
+  }
+  k_few_finish<<<dim3(G, (unsigned)(P.nagg > 0 ? P.nagg : 1)), 32, 0, s>>>(F, blocks);
+  YQ_CHECK_LAUNCH();
+  uint32_t err = 0;
+  YQ_TRY(d2h_sync(&err, d_err, sizeof(err), s));
+  *groups = G;
+  *done = true;
+  return err ? YQ_ERR_INVALID_ARG : YQ_OK;
 }
 
 }  // namespace
@@ -515,6 +972,7 @@ size_t yq_group_by_workspace_size(const yq_column* key, uint32_t rows, int32_t n
   w.add<uint8_t>(tile_order_sort_bytes((uint32_t)tiles));
   w.add<uint32_t>(tiles);                     // tile flags
   w.add<uint32_t>(4);                         // error word
+  if (few_applies(*key, rows)) w.add<char>(few_workspace_bytes(nagg));
   return w.total();
 }
 
@@ -574,6 +1032,13 @@ int yq_group_by(const yq_batch* batch, int32_t key_col, const yq_group_agg* aggs
   void* order_ws = ws.take<uint8_t>(order_ws_bytes);
   uint32_t* tile_flags = ws.take<uint32_t>((size_t)ntiles + 1);
   uint32_t* d_err = ws.take<uint32_t>(4);
+  if (few_applies(key, rows)) {
+    const size_t few_bytes = few_workspace_bytes(nagg);
+    char* few_ws = ws.take<char>(few_bytes);
+    bool done = false;
+    const int st = group_by_few(P, key, out[0], capacity, groups, few_ws, few_bytes, s, &done);
+    if (done || st != YQ_OK) return st;
+  }
   // The sort skips the passes whose digit every key shares (a key of few
   // distinct values sorts in one or two passes) and hands over its key words
   // in sorted order; a text key too long for one pass's words sorts without
