@@ -219,6 +219,27 @@ def test_writer_unaligned_output_and_capacity(cuda, yq):
     assert host[3:3 + len(want)] == want and host[:3] == bytes(3) and host[3 + len(want):] == bytes(61)
 
 
+@pytest.mark.parametrize("rows", [1, 127, 128, 129, 4099])
+@pytest.mark.parametrize("offset", [0, 3, 8])
+def test_writer_one_pass(cuda, yq, rows, offset):
+    """Room for the longest text the rows can have: written in one pass, at any
+    output alignment, and nothing beyond the text."""
+    rng = np.random.default_rng(rows + offset)
+    cols = random_batch(rng, rows)
+    want = oracle.csv_format(cols, rows)
+    b = device_batch(cols)
+    bc, keep = b.c()
+    n = C.c_uint64(0)
+    room = rows * 1024
+    out = torch.full((room + 64,), 0x7f, dtype=torch.uint8, device="cuda")
+    assert yq.yq_csv_format(C.byref(bc), out.data_ptr() + offset, room, C.byref(n), None, 0, None) == A.OK
+    torch.cuda.synchronize()
+    host = out.cpu().numpy().tobytes()
+    assert n.value == len(want)
+    assert host[offset:offset + len(want)] == want
+    assert set(host[:offset] + host[offset + len(want):]) <= {0x7f}
+
+
 def test_scan_then_write_round_trip(cuda):
     """Sales CSV text -> device scan -> device writer equals the oracle writer
     over the oracle scan (1M rows, bit-exact text)."""

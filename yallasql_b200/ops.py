@@ -752,6 +752,11 @@ def read_csv(data: bytes, project: list[str] | None = None, text_width: int = 25
     return [schema[f] for f in fields], batch
 
 
+# Longest text of a cell by type (TEXT: its slot and two quotes).
+_CSV_MAX_CELL = {A.INT32: 11, A.INT64: 20, A.FLOAT32: 46, A.DATETIME: 29}
+_CSV_ONE_PASS_BYTES = 1 << 30
+
+
 def csv_format(batch: DeviceBatch, stream=None) -> torch.Tensor:
     """The rows of a device batch as CSV text on the device (uint8 tensor),
     formatted as the reference's CsvWriter::batchToCsv formats them
@@ -760,6 +765,14 @@ def csv_format(batch: DeviceBatch, stream=None) -> torch.Tensor:
     s = _stream(stream)
     cols, keep = batch.c()
     n = C.c_uint64(0)
+    # with room for the longest text these rows can have one call counts and
+    # writes; otherwise a first call only counts
+    bound = batch.rows * sum(_CSV_MAX_CELL.get(c.type, c.width + 2) + 1 for c in batch.columns)
+    if 0 < bound <= _CSV_ONE_PASS_BYTES:
+        out = torch.empty(bound, dtype=torch.uint8, device="cuda")
+        _check(L.yq_csv_format(C.byref(cols), out.data_ptr(), bound, C.byref(n), None, 0, s), "yq_csv_format")
+        out = out[: int(n.value)]
+        return out.clone() if bound > 4 * int(n.value) else out
     st = L.yq_csv_format(C.byref(cols), None, 0, C.byref(n), None, 0, s)
     if st not in (A.OK, A.ERR_CAPACITY):
         _check(st, "yq_csv_format")
