@@ -317,3 +317,34 @@ def test_join_long_right_side(cuda, kind, nullable, L, R, distinct):
             with pytest.raises(A.YQError) as e:
                 ops.join_pairs(lb, rb, conds, capacity=len(wl) - 1)
             assert e.value.status == A.ERR_CAPACITY
+
+
+@pytest.mark.parametrize("kind", [A.INT32, A.INT64])
+@pytest.mark.parametrize("spread", [1, 3, 70, 100_000])
+def test_star_aggregate_key_ranges(cuda, kind, spread):
+    """Dimension keys dense (a bitmap of their range), around the bitmap's room
+    and sparse (the hash table), negative ones among them; fact keys beyond
+    both ends, and no dimension row kept."""
+    rng = np.random.default_rng(spread + kind)
+    dt = np.int32 if kind == A.INT32 else np.int64
+    dk = ((np.arange(3000) - 1200) * spread).astype(dt)
+    year = rng.integers(0, 4, 3000).astype(np.int32)
+    fk = rng.integers(-1300 * spread, 1900 * spread, 200_003).astype(dt)
+    fk[:3000] = dk
+    v = rng.integers(-1000, 1000, len(fk)).astype(np.int32)
+    fb = ops.DeviceBatch([dev_col(fk, kind), dev_col(v)])
+    db = ops.DeviceBatch([dev_col(rng.permutation(dk), kind), dev_col(year)])
+    keys = db.columns[0].data.cpu().numpy()
+    aggs = [Aggregate(A.AGG_SUM, ColumnRef(1, A.INT32)), Aggregate(A.AGG_COUNT_STAR)]
+    for y in (2, 9):
+        plan = ops.JoinAggPlan([kind, A.INT32], [kind, A.INT32], None, 0,
+                               Compare(A.EQ, ColumnRef(1, A.INT32), Constant(y, A.INT32)), 0, aggs)
+        hit = np.isin(fk, keys[year == y])
+        want = [int(v[hit].sum()) if hit.any() else None, int(hit.sum())]
+        for prepared in (False, True):
+            st = ops.AggState(aggs)
+            if prepared:
+                plan.run_prepared(fb, plan.prepare(db), st)
+            else:
+                plan.run(fb, db, st)
+            assert st.read() == want

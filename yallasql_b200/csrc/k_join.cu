@@ -21,6 +21,7 @@
 //  - nested-loop path: a warp per left row sweeps the right rows 32 at a time,
 //    ballots the matches and appends them with popc offsets (coalesced);
 //  - no condition: the cross product is written directly, left-major.
+#include <limits.h>
 #include <string.h>
 #include <type_traits>
 #include <vector>
@@ -201,7 +202,7 @@ struct BuildParams {
   uint32_t* bstart;   // [nbuckets + 1]
   unsigned long long* hkeys;
   uint32_t* hrows;
-  uint32_t* counts;   // [0] rows kept, [1] duplicate keys seen
+  uint32_t* counts;   // [0] rows kept, [1] duplicate keys seen, [2..3] least and [4..5] greatest key (signed)
 };
 
 
@@ -250,20 +251,43 @@ __global__ void __launch_bounds__(kBuildBlock) k_hash_build(const __grid_constan
     __syncthreads();
   }
   const uint32_t kept = min(s_kept, kHashMaxRows);
-  // 2. bucket counts and starts
-  for (uint32_t i = threadIdx.x; i < kept; i += kBuildBlock)
-    atomicAdd(&s_cnt[hash_bucket(hash_key(B.key, s_rows[i]), B.nbuckets)], 1u);
-  __syncthreads();
+  // 2. bucket counts and starts, key range
+  __shared__ long long s_min, s_max;
   if (threadIdx.x == 0) {
-    uint32_t run = 0;
-    for (uint32_t b = 0; b < B.nbuckets; ++b) {
-      const uint32_t c = s_cnt[b];
-      B.bstart[b] = run;
-      s_cnt[b] = run;  // becomes the insertion cursor
-      run += c;
+    s_min = LLONG_MAX;
+    s_max = LLONG_MIN;
+  }
+  __syncthreads();
+  {
+    long long lo = LLONG_MAX, hi = LLONG_MIN;
+    for (uint32_t i = threadIdx.x; i < kept; i += kBuildBlock) {
+      const long long k = (long long)hash_key(B.key, s_rows[i]);
+      atomicAdd(&s_cnt[hash_bucket((uint64_t)k, B.nbuckets)], 1u);
+      lo = min(lo, k);
+      hi = max(hi, k);
     }
+    if (lo <= hi) {
+      atomicMin(&s_min, lo);
+      atomicMax(&s_max, hi);
+    }
+  }
+  __syncthreads();
+  uint32_t run = 0;
+  for (uint32_t b0 = 0; b0 < B.nbuckets; b0 += kBuildBlock) {
+    const uint32_t b = b0 + threadIdx.x;
+    uint32_t total;
+    const uint32_t at = run + block_exclusive_sum<kBuildBlock>(b < B.nbuckets ? s_cnt[b] : 0u, s_warp, total);
+    if (b < B.nbuckets) {
+      B.bstart[b] = at;
+      s_cnt[b] = at;  // becomes the insertion cursor
+    }
+    run += total;
+  }
+  if (threadIdx.x == 0) {
     B.bstart[B.nbuckets] = run;
     B.counts[0] = s_kept;
+    *reinterpret_cast<long long*>(B.counts + 2) = s_min;
+    *reinterpret_cast<long long*>(B.counts + 4) = s_max;
   }
   __syncthreads();
   // 3. stable scatter: rows in ascending order, one warp at a time
@@ -378,6 +402,8 @@ struct SortedJoin {
   uint32_t nslots;                // power of two, >= 2 R
 };
 constexpr uint32_t kNoSlot = 0xffffffffu;
+constexpr uint32_t kSortedMinRows = 1024;  // right rows from which a sorted table may be chosen, and from
+constexpr uint32_t kTableRows = 4096;      // which it always is
 
 __device__ __forceinline__ bool key_joins(const JCol& c, uint32_t row) {
   if (cell_null(c, row)) return false;
@@ -703,20 +729,24 @@ __global__ void k_join_count_sorted(const T* __restrict__ lcol, uint32_t L, cons
 // Same tiles, look-back and output order (left row major, right rows
 // ascending) as k_join_nested.
 //
-// Each left row's matches are compacted into a shared-memory run that starts
-// at its output position's place in a 16-byte word and leaves in full runs of
-// 512 bytes, 16 a lane. Storing each match as it is found (64 unaligned bytes
-// a store for a comparison that half the pairs pass) held the kernel to
-// 2.3 TB/s of output: 20K x 20K INT32 rows under <, 199M pairs, 677 us for the
-// writing alone; with the runs 0.59 ms, the counting pass included. The right column is read through L1 (80 KB at 20K rows)
-// rather than staged, so warps never wait for one another; blocks of four
-// warps keep the last wave short (1,250 blocks at 20K left rows).
+// Each left row's matches are compacted into a shared-memory ring of two runs
+// of 512 bytes, whose entries sit where their output positions lie in a 16-byte
+// word; a full run leaves 16 bytes a lane. Storing each match as it is found
+// (64 unaligned bytes a store for a comparison that half the pairs pass) held
+// the kernel to 2.3 TB/s of output: 20K x 20K INT32 rows under <, 199M pairs,
+// 677 us for the writing alone. A row's ring is looked at once for kNtUnroll
+// right values a lane (they cross at most one run), which keeps the run writer
+// out of the unrolled comparisons: with a look after every value the kernel
+// waited for its instructions. The right column is read through L1 (80 KB at
+// 20K rows) rather than staged, so warps never wait for one another; blocks of
+// four warps keep the last wave short (1,250 blocks at 20K left rows).
 constexpr int kNtBlock = 128;
 constexpr int kNtRows = 4;
 constexpr uint32_t kNtTile = (kNtBlock / 32) * kNtRows;  // left rows per block
-constexpr int kNtUnroll = 4;                              // right values a lane loads ahead
+constexpr int kNtCountUnroll = 16;  // right values a lane loads ahead while counting,
+constexpr int kNtUnroll = 4;        // and while it writes
 
-// Outputs [pb + i0, pb + i1) of left row l: right rows rows[i0 .. i1).
+// Outputs [pb + i0, pb + i1) of left row l: right rows rows[i0 .. i1) of a run.
 __device__ __noinline__ void write_rows(const JoinParams& J, uint32_t l, unsigned long long pb, uint32_t i0,
                                         uint32_t i1, const uint32_t* rows) {
   const uint32_t lane = threadIdx.x & 31;
@@ -741,7 +771,9 @@ __global__ void __launch_bounds__(kNtBlock) k_join_nested_typed(const __grid_con
   using B = typename std::conditional<VALUES, T, uint32_t>::type;
   constexpr uint32_t VEC = 16 / sizeof(B);
   constexpr uint32_t RUN = 32 * VEC;
-  __shared__ __align__(16) B s_buf[kNtBlock / 32][kNtRows][RUN + 32];
+  constexpr uint32_t RING = RUN * (RUN < 32u * kNtUnroll ? 4 : 2);  // a batch of matches crosses less than half of it
+  static_assert(RING >= RUN + 32 * kNtUnroll, "a batch must not overtake the run being written");
+  __shared__ __align__(16) B s_buf[kNtBlock / 32][kNtRows][RING];
   __shared__ uint32_t s_tile;
   __shared__ uint32_t s_cnt[kNtTile];
   __shared__ uint32_t s_warp[kNtBlock / 32 + 1];
@@ -771,17 +803,22 @@ __global__ void __launch_bounds__(kNtBlock) k_join_nested_typed(const __grid_con
     uint32_t cnt[kNtRows];
 #pragma unroll
     for (int i = 0; i < kNtRows; ++i) cnt[i] = 0;
-    // per-lane counts (one predicated add a comparison), summed over the warp below
-    for (uint32_t r0 = lane; r0 < J.R; r0 += 32 * kNtUnroll) {
-      T rv[kNtUnroll];
+    // per-lane counts (a compare and an add a comparison), summed over the warp below
+    constexpr uint32_t STEP = 32 * kNtCountUnroll;
+    const uint32_t whole = J.R / STEP * STEP;
+    for (uint32_t r0 = lane; r0 < whole; r0 += STEP) {
+      T rv[kNtCountUnroll];
 #pragma unroll
-      for (int u = 0; u < kNtUnroll; ++u) rv[u] = r0 + u * 32 < J.R ? __ldg(rcol + r0 + u * 32) : T(0);
+      for (int u = 0; u < kNtCountUnroll; ++u) rv[u] = __ldg(rcol + r0 + u * 32);
 #pragma unroll
-      for (int u = 0; u < kNtUnroll; ++u)
-        if (r0 + u * 32 < J.R) {
+      for (int u = 0; u < kNtCountUnroll; ++u)
 #pragma unroll
-          for (int i = 0; i < kNtRows; ++i) cnt[i] += nl_cmp<T, OP>(lv[i], rv[u]) ? 1u : 0u;
-        }
+        for (int i = 0; i < kNtRows; ++i) cnt[i] += nl_cmp<T, OP>(lv[i], rv[u]) ? 1u : 0u;
+    }
+    for (uint32_t r = whole + lane; r < J.R; r += 32) {
+      const T rv = __ldg(rcol + r);
+#pragma unroll
+      for (int i = 0; i < kNtRows; ++i) cnt[i] += nl_cmp<T, OP>(lv[i], rv) ? 1u : 0u;
     }
 #pragma unroll
     for (int i = 0; i < kNtRows; ++i)
@@ -820,70 +857,73 @@ __global__ void __launch_bounds__(kNtBlock) k_join_nested_typed(const __grid_con
   // every pair of this tile fits and the outputs take 16-byte stores
   const bool whole = prefix + total <= J.capacity &&
                      ((reinterpret_cast<uintptr_t>(vl) | reinterpret_cast<uintptr_t>(vr)) & 15) == 0;
-  unsigned long long pb[kNtRows];  // output position of the run's entry 0
-  uint32_t head[kNtRows], fill[kNtRows];
+  unsigned long long p0[kNtRows];  // output position of ring entry 0 (a whole 16-byte word)
+  uint32_t head[kNtRows];          // first entry of the run that is not yet written
+  uint32_t fill[kNtRows];          // entries so far, the head's empty ones included
   bool any = false;
 #pragma unroll
   for (int i = 0; i < kNtRows; ++i) {
     const unsigned long long p = prefix + s_off[warp * kNtRows + i];
     head[i] = fill[i] = (uint32_t)(p & (VEC - 1));
-    pb[i] = p - head[i];
-    lok[i] = lok[i] && s_cnt[warp * kNtRows + i] > 0;
+    p0[i] = p - head[i];
+    lok[i] = lok[i] && s_cnt[warp * kNtRows + i] > 0 && p < J.capacity;
     any |= lok[i];
   }
   if (!any) return;
-  auto flush = [&](int i, uint32_t n) {  // entries [head, n) of row i's run
+  // entries [head, n) of row i, all within one run
+  auto flush = [&](int i, uint32_t n) {
     __syncwarp();
-    const B* buf = s_buf[warp][i];
+    const uint32_t r0 = head[i] & ~(RUN - 1u);  // the run's first entry
+    const B* buf = s_buf[warp][i] + (r0 & (RING - 1u));
+    const unsigned long long pos = p0[i] + r0;
     if constexpr (VALUES) {
-      if (whole && n == RUN && head[i] == 0) {
+      if (whole && head[i] == r0 && n == r0 + RUN) {
         if (vl) {
           T x[VEC];
 #pragma unroll
           for (uint32_t v = 0; v < VEC; ++v) x[v] = lv[i];
-          *reinterpret_cast<uint4*>(vl + pb[i] + lane * VEC) = *reinterpret_cast<const uint4*>(x);
+          *reinterpret_cast<uint4*>(vl + pos + lane * VEC) = *reinterpret_cast<const uint4*>(x);
         }
-        if (vr) *reinterpret_cast<uint4*>(vr + pb[i] + lane * VEC) = *reinterpret_cast<const uint4*>(buf + lane * VEC);
+        if (vr) *reinterpret_cast<uint4*>(vr + pos + lane * VEC) = *reinterpret_cast<const uint4*>(buf + lane * VEC);
       } else {
-        for (uint32_t x = head[i] + lane; x < n; x += 32)
-          if (pb[i] + x < J.capacity) {
-            if (vl) vl[pb[i] + x] = lv[i];
-            if (vr) vr[pb[i] + x] = buf[x];
+        for (uint32_t x = head[i] - r0 + lane; x < n - r0; x += 32)
+          if (pos + x < J.capacity) {
+            if (vl) vl[pos + x] = lv[i];
+            if (vr) vr[pos + x] = buf[x];
           }
       }
     } else {
-      write_rows(J, l0 + i, pb[i], head[i], n, buf);
+      write_rows(J, l0 + i, pos, head[i] - r0, n - r0, buf);
     }
+    __syncwarp();
+    head[i] = n;
   };
-  for (uint32_t r0 = lane; r0 < ((J.R + 31u) & ~31u); r0 += 32 * kNtUnroll) {
+  // kNtUnroll right values a lane against every row; FULL: all of them exist
+  auto batch = [&](uint32_t r0, auto full) {
+    constexpr bool FULL = decltype(full)::value;
     T rv[kNtUnroll];
 #pragma unroll
-    for (int u = 0; u < kNtUnroll; ++u) rv[u] = r0 + u * 32 < J.R ? __ldg(rcol + r0 + u * 32) : T(0);
+    for (int u = 0; u < kNtUnroll; ++u) rv[u] = FULL || r0 + u * 32 < J.R ? __ldg(rcol + r0 + u * 32) : T(0);
 #pragma unroll
-    for (int u = 0; u < kNtUnroll; ++u) {
-      const uint32_t r = r0 + u * 32;
-      const bool ok = r < J.R;
+    for (int i = 0; i < kNtRows; ++i) {
+      const uint32_t before = fill[i];
 #pragma unroll
-      for (int i = 0; i < kNtRows; ++i) {
-        const bool m = ok && lok[i] && nl_cmp<T, OP>(lv[i], rv[u]);
+      for (int u = 0; u < kNtUnroll; ++u) {
+        const bool m = (FULL || r0 + u * 32 < J.R) && lok[i] && nl_cmp<T, OP>(lv[i], rv[u]);
         const uint32_t bal = __ballot_sync(0xffffffffu, m);
         if (m) {
-          if constexpr (VALUES) s_buf[warp][i][fill[i] + __popc(bal & lt)] = rv[u];
-          else s_buf[warp][i][fill[i] + __popc(bal & lt)] = r;
+          const uint32_t at = (fill[i] + __popc(bal & lt)) & (RING - 1u);
+          if constexpr (VALUES) s_buf[warp][i][at] = rv[u];
+          else s_buf[warp][i][at] = r0 + u * 32;
         }
         fill[i] += __popc(bal);
-        if (fill[i] >= RUN) {
-          flush(i, RUN);
-          const B rest = s_buf[warp][i][RUN + lane];
-          __syncwarp();
-          s_buf[warp][i][lane] = rest;
-          fill[i] -= RUN;
-          head[i] = 0;
-          pb[i] += RUN;
-        }
       }
+      for (uint32_t run = (before | (RUN - 1u)) + 1u; run <= fill[i]; run += RUN) flush(i, run);
     }
-  }
+  };
+  uint32_t r0 = lane;
+  for (; r0 - lane + 32 * kNtUnroll <= J.R; r0 += 32 * kNtUnroll) batch(r0, std::true_type{});
+  if (r0 - lane < J.R) batch(r0, std::false_type{});
 #pragma unroll
   for (int i = 0; i < kNtRows; ++i)
     if (lok[i] && fill[i] > head[i]) flush(i, fill[i]);
@@ -1149,13 +1189,22 @@ static int join_impl(const yq_batch* left, const yq_batch* right, const yq_join_
     return n > capacity ? YQ_ERR_CAPACITY : YQ_OK;
   }
 
-  // The sorted table holds any length the sort takes. BOOL keys stay with the
-  // other paths: the sort orders every non-zero byte as one value, a join
-  // compares the bytes.
-  const bool use_hash = J.eq >= 0 && J.R <= kHashMaxRows;
-  const size_t eq_sort_bytes =
-      J.eq >= 0 && !use_hash && J.cond[J.eq].r.type != YQ_BOOL ? join_sort_bytes(J.R, J.cond[J.eq].r.nulls != nullptr) : 0;
+  // The sorted table holds any length the sort takes; the shared-memory table is
+  // built by one block and copied by every block of the probe. Its build is the
+  // longer one from about 4,096 rows on (20K left rows to 8,000 right ones:
+  // 0.30 ms against 0.16), its copies cost more than the sort's launches from
+  // about 2^32 pairs on (2M to 4,000: 0.36 ms against 0.23; 2M to 2,000: 0.23
+  // both; 20K to 2,000: 0.15 against 0.18). BOOL keys stay with the other paths
+  // (the sort orders every non-zero byte as one value, a join compares the
+  // bytes), and float keys as long as the shared-memory table holds them (it
+  // joins equal NaN bit patterns).
+  const bool eq_float = J.eq >= 0 && (J.cond[J.eq].r.type == YQ_FLOAT32 || J.cond[J.eq].r.type == YQ_FLOAT64);
+  const uint32_t table_rows =
+      eq_float ? kHashMaxRows : ((unsigned long long)J.L * J.R > (1ull << 32) ? kSortedMinRows : kTableRows);
+  const size_t eq_sort_bytes = J.eq >= 0 && J.R > table_rows && J.cond[J.eq].r.type != YQ_BOOL
+                                   ? join_sort_bytes(J.R, J.cond[J.eq].r.nulls != nullptr) : 0;
   const bool use_sorted = eq_sort_bytes != 0;
+  const bool use_hash = J.eq >= 0 && !use_sorted && J.R <= kHashMaxRows;
   const uint32_t nbuckets = use_hash ? pow2_at_least(J.R) : 0u;
   const JCond& t0 = J.cond[0];
   const bool typed = !use_hash && !use_sorted && J.ncond == 1 && J.ngroups == 1 && t0.l.type == t0.r.type && !t0.l.nulls &&
@@ -1292,7 +1341,7 @@ size_t yq_join_workspace_size(uint32_t left_rows, uint32_t right_rows) {
   w.add<uint32_t>(8);
   WsSize sorted = w;
   if (counts_first(left_rows, right_rows)) count_ws_layout(left_rows, right_rows, join_sort_bytes(right_rows, false), w);
-  if (right_rows > kHashMaxRows) sorted_ws_layout(right_rows, join_sort_bytes(right_rows, true), sorted);
+  if (right_rows > kSortedMinRows) sorted_ws_layout(right_rows, join_sort_bytes(right_rows, true), sorted);
   return w.total() > sorted.total() ? w.total() : sorted.total();
 }
 
@@ -1392,8 +1441,8 @@ static int join_agg_params(const yq_batch* fact, const yq_program* fact_predicat
 
 // Probe launch over a built dimension table (nbuckets buckets, `kept` rows).
 static int join_agg_launch(JAParams& F, const yq_batch* fact, int32_t fact_key, uint32_t nbuckets, uint32_t kept,
-                           uint32_t* d_bstart, unsigned long long* d_hkeys, Acc* partials, uint32_t* d_misc,
-                           void* state, cudaStream_t s) {
+                           uint32_t* d_bstart, unsigned long long* d_hkeys, const uint32_t* d_counts, Acc* partials,
+                           uint32_t* d_misc, void* state, cudaStream_t s) {
   const yq_column& fk = fact->columns[fact_key];
   const int grid_cap = sm_count() * 8;
   const uint32_t counts[1] = {kept};
@@ -1402,6 +1451,7 @@ static int join_agg_launch(JAParams& F, const yq_batch* fact, int32_t fact_key, 
   F.hrows_n = counts[0];
   F.bstart = d_bstart;
   F.hkeys = d_hkeys;
+  F.krange = reinterpret_cast<const long long*>(d_counts + 2);
   const size_t table = table_smem(nbuckets, counts[0], false);
   // The ring leaves room for the table; with too few stages left the kernel
   // reads the fact columns from global memory.
@@ -1412,6 +1462,7 @@ static int join_agg_launch(JAParams& F, const yq_batch* fact, int32_t fact_key, 
   }
   const bool staged = F.SP.nstages > 0;
   F.table_off = (uint32_t)align_up(stage_smem_bytes(F.SP), 16);
+  F.table_words = (uint32_t)(table / 4);
   const size_t smem = F.table_off + table;
   const void* kern = staged ? (const void*)k_join_aggregate<true> : (const void*)k_join_aggregate<false>;
   YQ_TRY(kernel_allow_smem(kern, smem));
@@ -1475,7 +1526,8 @@ int yq_join_aggregate(const yq_batch* fact, const yq_program* fact_predicate, in
   uint32_t counts[2] = {0, 0};
   YQ_TRY(d2h_sync(counts, d_misc + 2, sizeof(counts), s));
   if (counts[1] != 0) return YQ_ERR_UNSUPPORTED;  // dimension keys repeat: use yq_join_pairs + an aggregate
-  return join_agg_launch(F, fact, fact_key, nbuckets, counts[0], d_bstart, d_hkeys, partials, d_misc, state, s);
+  return join_agg_launch(F, fact, fact_key, nbuckets, counts[0], d_bstart, d_hkeys, d_misc + 2, partials, d_misc, state,
+                         s);
 }
 
 // ------------------------------------------------ prepared dimension table
@@ -1544,7 +1596,7 @@ int yq_join_aggregate_prepared(const yq_batch* fact, const yq_program* fact_pred
   const size_t tbytes = yq_join_dim_table_size(dim_rows);
   Workspace tw;  // the caller's table, carved as yq_join_dim_table_build laid it out
   YQ_TRY(tw.acquire(const_cast<void*>(table), tbytes, tbytes, s));
-  tw.take<uint32_t>(8);
+  uint32_t* d_counts = tw.take<uint32_t>(8) + 2;
   uint32_t* d_bstart = tw.take<uint32_t>(nbuckets + 1);
   unsigned long long* d_hkeys = tw.take<unsigned long long>(dim_rows ? dim_rows : 1);
   Workspace ws;
@@ -1552,7 +1604,7 @@ int yq_join_aggregate_prepared(const yq_batch* fact, const yq_program* fact_pred
   uint32_t* d_misc = ws.take<uint32_t>(8);
   Acc* partials = ws.take<Acc>((size_t)sm_count() * 8 * YQ_MAX_AGGREGATES);
   YQ_TRY_CUDA(cudaMemsetAsync(d_misc, 0, 8 * sizeof(uint32_t), s));
-  return join_agg_launch(F, fact, fact_key, nbuckets, kept, d_bstart, d_hkeys, partials, d_misc, state, s);
+  return join_agg_launch(F, fact, fact_key, nbuckets, kept, d_bstart, d_hkeys, d_counts, partials, d_misc, state, s);
 }
 
 }  // extern "C"

@@ -470,6 +470,8 @@ struct JAParams {
   JCol fkey;
   uint32_t nbuckets, hrows_n;
   uint32_t table_off;  // byte offset of the dimension table in dynamic shared memory
+  uint32_t table_words;  // its size
+  const long long* krange;  // least and greatest dimension key
   const uint32_t* bstart;
   const unsigned long long* hkeys;
 };
@@ -490,8 +492,23 @@ __device__ __forceinline__ void join_aggregate_body(const JAParams& F, uint32_t 
   uint32_t* s_bstart = reinterpret_cast<uint32_t*>(yq_dyn_smem + F.table_off);
   unsigned long long* s_keys =
       reinterpret_cast<unsigned long long*>(yq_dyn_smem + F.table_off + 4 * ((F.nbuckets + 2) & ~1u));
-  for (uint32_t i = threadIdx.x; i <= F.nbuckets; i += kRowBlock) s_bstart[i] = __ldg(F.bstart + i);
-  for (uint32_t i = threadIdx.x; i < F.hrows_n; i += kRowBlock) s_keys[i] = __ldg(F.hkeys + i);
+  // The probe only asks whether a key is there. When the kept keys' range fits
+  // the table's shared memory a bit a key, it is a bitmap (one load and a shift
+  // a row; dimension keys are mostly dense numbers), otherwise the hash table.
+  const uint64_t kmin = (uint64_t)__ldg(F.krange), kspan = (uint64_t)__ldg(F.krange + 1) - kmin;
+  const bool bitmap = F.hrows_n > 0 && kspan < (uint64_t)F.table_words * 32u;
+  if (bitmap) {
+    const uint32_t words = (uint32_t)(kspan >> 5) + 1u;
+    for (uint32_t i = threadIdx.x; i < words; i += kRowBlock) s_bstart[i] = 0u;
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < F.hrows_n; i += kRowBlock) {
+      const uint64_t d = __ldg(F.hkeys + i) - kmin;
+      if (d <= kspan) atomicOr(s_bstart + (d >> 5), 1u << (d & 31u));
+    }
+  } else {
+    for (uint32_t i = threadIdx.x; i <= F.nbuckets; i += kRowBlock) s_bstart[i] = __ldg(F.bstart + i);
+    for (uint32_t i = threadIdx.x; i < F.hrows_n; i += kRowBlock) s_keys[i] = __ldg(F.hkeys + i);
+  }
   __syncthreads();
 
   uint32_t* err = agg_state_err(state);
@@ -511,6 +528,8 @@ __device__ __forceinline__ void join_aggregate_body(const JAParams& F, uint32_t 
       }
   }
   const DevCol& kc = F.P.cols[F.fkey_col];
+  static_assert(ITEMS == 4, "a thread's 4-byte keys are one 16-byte word");
+  const bool bitmap32 = bitmap && kc.type == YQ_INT32 && kc.width == 4;
   int slot = 0;
   uint32_t parity = 0;
   for (uint32_t tile = blockIdx.x; tile < ntiles; tile += G) {
@@ -535,6 +554,21 @@ __device__ __forceinline__ void join_aggregate_body(const JAParams& F, uint32_t 
     if (F.pred_end > 0) R::template run<STAGED>(F.P, 0, 0, F.pred_end, X, St, E);
     // probe: keep rows whose key is present among the (unique) dimension keys
     const uint32_t knull = null_bits<STAGED>(kc, X);
+    if (STAGED && bitmap32) {
+      // the thread's four 4-byte keys in one load, no branch a row: differences
+      // modulo 2^32 are exact here, the keys' range being below it
+      const uint4 kv = *reinterpret_cast<const uint4*>(yq_dyn_smem + X.stage + kc.soff + X.lr * 4u);
+      const uint32_t kk[4] = {kv.x, kv.y, kv.z, kv.w};
+      const uint32_t kmin32 = (uint32_t)kmin, span32 = (uint32_t)kspan;
+      uint32_t hits = 0u;
+#pragma unroll
+      for (int k = 0; k < ITEMS; ++k) {
+        const uint32_t d = kk[k] - kmin32;
+        const uint32_t w = s_bstart[min(d, span32) >> 5];
+        if (d <= span32) hits |= (w >> (d & 31u) & 1u) << k;
+      }
+      E.sel &= hits & ~knull;
+    } else {
 #pragma unroll
     for (int k = 0; k < ITEMS; ++k) {
       if (!(E.sel >> k & 1u)) continue;
@@ -550,10 +584,16 @@ __device__ __forceinline__ void join_aggregate_body(const JAParams& F, uint32_t 
         } else {
           key = hash_key(F.fkey, X.tile0 + X.lr + k);
         }
-        const uint32_t b = hash_bucket(key, F.nbuckets);
-        for (uint32_t x = s_bstart[b]; x < s_bstart[b + 1] && !hit; ++x) hit = (s_keys[x] == key);
+        if (bitmap) {
+          const uint64_t d = key - kmin;
+          hit = d <= kspan && (s_bstart[d >> 5] >> (d & 31u) & 1u);
+        } else {
+          const uint32_t b = hash_bucket(key, F.nbuckets);
+          for (uint32_t x = s_bstart[b]; x < s_bstart[b + 1] && !hit; ++x) hit = (s_keys[x] == key);
+        }
       }
       if (!hit) E.sel &= ~(1u << k);
+    }
     }
     R::template run<STAGED>(F.P, 1, F.pred_end, F.pc_end, X, St, E);
     nsel += __popc(E.sel);
