@@ -114,6 +114,7 @@ struct GAgg {
   const uint8_t* nulls;
   int32_t type;          // input type
   int32_t kind;          // yq_agg_kind
+  int32_t width;         // of a cell
 };
 
 struct GroupParams {
@@ -505,95 +506,124 @@ struct FewTable {
   unsigned long long group_key[kFewGroups];
 };
 
-// 4-byte keys zero-extended (never kNoKey), 8-byte keys as they are.
-__device__ __forceinline__ unsigned long long few_key(const yq_column& k, uint32_t r) {
-  return k.width == 4 ? (unsigned long long)__ldg(static_cast<const uint32_t*>(k.data) + r)
-                      : __ldg(static_cast<const unsigned long long*>(k.data) + r);
-}
-__device__ __forceinline__ uint32_t few_hash(unsigned long long k) {
-  return (uint32_t)((k * 0x9e3779b97f4a7c15ull) >> 55);  // the top 9 bits
+__device__ __forceinline__ uint32_t few_hash(unsigned long long k) {  // the top 9 bits of a product
+  return (((uint32_t)k ^ ((uint32_t)(k >> 32) * 0x85ebca6bu)) * 0x9e3779b1u) >> 23;
 }
 static_assert(kFewSlots == 512, "few_hash gives nine bits");
 
-// Puts `key` into the table; false when it holds too many keys.
-__device__ __forceinline__ bool few_insert(unsigned long long* keys, uint32_t* count, unsigned long long key) {
+// Puts `key` into the table (empty slots hold `empty`, which is not a key to
+// put in); false when it holds too many keys.
+template <typename K>
+__device__ __forceinline__ bool few_insert(K* keys, uint32_t* count, K key, K empty) {
   uint32_t h = few_hash(key);
   for (uint32_t n = 0; n < kFewSlots; ++n, h = (h + 1) & (kFewSlots - 1)) {
-    unsigned long long cur = *reinterpret_cast<volatile unsigned long long*>(keys + h);
+    K cur = *reinterpret_cast<volatile K*>(keys + h);
     if (cur == key) return true;
-    if (cur != kNoKey) continue;
-    cur = atomicCAS(keys + h, kNoKey, key);
-    if (cur == kNoKey) return atomicAdd(count, 1u) < kFewGroups;
+    if (cur != empty) continue;
+    cur = atomicCAS(keys + h, empty, key);
+    if (cur == empty) return atomicAdd(count, 1u) < kFewGroups;
     if (cur == key) return true;
   }
   return false;
 }
 
-__global__ void __launch_bounds__(kFewFindThreads) k_few_find(const yq_column key, uint32_t rows, FewTable* T) {
-  __shared__ unsigned long long s_keys[kFewSlots];
-  __shared__ uint32_t s_count, s_last, s_over;
-  for (uint32_t i = threadIdx.x; i < kFewSlots; i += kFewFindThreads) s_keys[i] = kNoKey;
-  if (threadIdx.x == 0) s_count = s_last = s_over = 0u;
+// K: the key's bits. Row 0's key is known to be there, so a block's table is
+// filled with it: empty slots need no value outside the key's own, and a probe
+// is a product, a load and a compare.
+template <typename K>
+__global__ void __launch_bounds__(kFewFindThreads) k_few_find(const K* __restrict__ keys,
+                                                              const uint8_t* __restrict__ nulls, uint32_t rows,
+                                                              FewTable* T) {
+  __shared__ K s_keys[kFewSlots];
+  __shared__ uint32_t s_count, s_over;
+  const K first = __ldg(keys);
+  for (uint32_t i = threadIdx.x; i < kFewSlots; i += kFewFindThreads) s_keys[i] = first;
+  if (threadIdx.x == 0) {
+    s_count = 1u;
+    s_over = 0u;
+  }
   __syncthreads();
   constexpr uint32_t STEP = kFewFindThreads * kFewItems;
   bool ok = true;
-  for (unsigned long long base = (unsigned long long)blockIdx.x * STEP; base < rows;
-       base += (unsigned long long)gridDim.x * STEP) {
-    // another thread or block has found too many keys: the table is not used
-    if (*reinterpret_cast<volatile uint32_t*>(&s_over) || ld_relaxed_u32(&T->overflow)) break;
-    unsigned long long k[kFewItems];
-    bool in[kFewItems];
+  for (uint32_t base = blockIdx.x * STEP; base < rows; base += gridDim.x * STEP) {
+    // one thread a block reads the other blocks' flag, along with its keys
+    const uint32_t over = threadIdx.x == 0 ? ld_relaxed_u32(&T->overflow) : 0u;
+    const uint32_t r0 = base + threadIdx.x;
+    K k[kFewItems];
+    if (base + STEP <= rows) {
+      const K* p = keys + r0;
 #pragma unroll
-    for (int q = 0; q < kFewItems; ++q) {
-      const unsigned long long r = base + q * kFewFindThreads + threadIdx.x;
-      in[q] = r < rows;
-      k[q] = in[q] ? few_key(key, (uint32_t)r) : 0ull;
-      if (in[q] && key.nulls && key.nulls[r]) ok = false;  // a NULL group's key cell is its first row's: the sort finds it
-    }
+      for (int q = 0; q < kFewItems; ++q) k[q] = __ldg(p + q * kFewFindThreads);
+    } else {
 #pragma unroll
-    for (int q = 0; q < kFewItems; ++q) {
-      if (!in[q]) continue;
-      if (k[q] == kNoKey) s_last = 1u;
-      else if (ok && !few_insert(s_keys, &s_count, k[q])) ok = false;
+      for (int q = 0; q < kFewItems; ++q) k[q] = r0 + q * kFewFindThreads < rows ? __ldg(keys + r0 + q * kFewFindThreads) : first;
     }
-    if (!ok) s_over = 1u;
+    if (nulls) {  // a NULL group's key cell is its first row's: the sort finds it
+#pragma unroll
+      for (int q = 0; q < kFewItems; ++q)
+        if (r0 + q * kFewFindThreads < rows && __ldg(nulls + r0 + q * kFewFindThreads)) ok = false;
+    }
+    // all first probes before any insertion: with few keys nearly every one hits
+    uint32_t miss = 0u;
+#pragma unroll
+    for (int q = 0; q < kFewItems; ++q)
+      miss |= (k[q] != first && *reinterpret_cast<volatile K*>(s_keys + few_hash(k[q])) != k[q]) ? 1u << q : 0u;
+    for (; miss && ok; miss &= miss - 1) {
+      const int m = __ffs(miss) - 1;
+      K key = k[0];
+#pragma unroll
+      for (int q = 1; q < kFewItems; ++q)
+        if (q == m) key = k[q];
+      ok = few_insert<K>(s_keys, &s_count, key, first);
+    }
+    if (!ok || over) s_over = 1u;
+    // this block or another one has found too many keys: the table is not used
+    if (__any_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t*>(&s_over) != 0u)) break;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    if (s_last) atomicOr(&T->has_last, 1u);
-    if (s_over) atomicOr(&T->overflow, 1u);
+  if (s_over) {
+    if (threadIdx.x == 0) atomicOr(&T->overflow, 1u);
+    return;
   }
-  if (s_over) return;
-  for (uint32_t i = threadIdx.x; i < kFewSlots; i += kFewFindThreads)
-    if (s_keys[i] != kNoKey && !few_insert(T->keys, &T->count, s_keys[i])) atomicOr(&T->overflow, 1u);
+  for (uint32_t i = threadIdx.x; i <= kFewSlots; i += kFewFindThreads) {
+    const K key = i < kFewSlots ? s_keys[i] : first;
+    if (i < kFewSlots && key == first) continue;
+    if ((unsigned long long)key == kNoKey) atomicOr(&T->has_last, 1u);
+    else if (!few_insert<unsigned long long>(T->keys, &T->count, key, kNoKey)) atomicOr(&T->overflow, 1u);
+  }
 }
 
-// Group index of every key: ascending signed order.
+// Group index of every key: ascending signed order. The keys are compacted
+// first, so that each looks at the others and not at every slot.
 __global__ void __launch_bounds__(kFewSlots) k_few_order(FewTable* T, int width) {
-  __shared__ unsigned long long s_keys[kFewSlots];
+  __shared__ long long s_val[kFewGroups];
+  __shared__ uint32_t s_n;
   const uint32_t i = threadIdx.x;
   const unsigned long long mine = T->keys[i];
-  s_keys[i] = mine;
-  __syncthreads();
   const uint32_t n = T->count + (T->has_last ? 1u : 0u);
   if (T->overflow || n > kFewGroups) {
     if (i == 0) T->overflow = 1u;
     return;
   }
-  auto value = [width](unsigned long long k) { return width == 4 ? (long long)(int32_t)(uint32_t)k : (long long)k; };
-  const bool has_last = T->has_last != 0u;  // the key ~0: signed -1
+  if (i == 0) s_n = 0u;
+  __syncthreads();
+  const long long value = width == 4 ? (long long)(int32_t)(uint32_t)mine : (long long)mine;
+  if (mine != kNoKey) s_val[atomicAdd(&s_n, 1u)] = value;
+  if (i == 0 && T->has_last) s_val[atomicAdd(&s_n, 1u)] = -1ll;  // the 8-byte key ~0
+  __syncthreads();
+  auto rank_of = [&](long long v) {
+    uint32_t r = 0;
+    for (uint32_t j = 0; j < n; ++j) r += s_val[j] < v ? 1u : 0u;
+    return r;
+  };
   if (mine != kNoKey) {
-    uint32_t rank = has_last && -1ll < value(mine) ? 1u : 0u;
-    for (uint32_t j = 0; j < kFewSlots; ++j)
-      if (s_keys[j] != kNoKey && value(s_keys[j]) < value(mine)) ++rank;
+    const uint32_t rank = rank_of(value);
     T->gid[i] = rank;
     T->group_key[rank] = mine;
   }
   if (i == 0) {
-    if (has_last) {
-      uint32_t rank = 0;
-      for (uint32_t j = 0; j < kFewSlots; ++j)
-        if (s_keys[j] != kNoKey && value(s_keys[j]) < -1ll) ++rank;
+    if (T->has_last) {
+      const uint32_t rank = rank_of(-1ll);
       T->last_gid = rank;
       T->group_key[rank] = kNoKey;
     }
@@ -608,10 +638,22 @@ struct FewAcc {
   int32_t val_off;  // value array (-1: a count)
   int32_t val_size;
 };
+// An input column and the aggregates over it (agg[first, first + count) of
+// FewParams::order): its cells are read once for all of them.
+struct FewCol {
+  const void* data;
+  const uint8_t* nulls;
+  int32_t type, width;  // width 0: only counted, no cell is read
+  int32_t first, count;
+  int32_t cnt_off;  // non-NULL counts (with nulls)
+};
 struct FewParams {
   GroupParams P;
   yq_column key;
   FewAcc acc[YQ_MAX_AGGREGATES];
+  FewCol col[YQ_MAX_AGGREGATES];
+  int32_t ncol;
+  int8_t order[YQ_MAX_AGGREGATES];
   int32_t bytes;      // of all arrays, for one group and thread
   uint32_t ngroups;
   uint32_t rows_per_block;
@@ -632,37 +674,61 @@ __device__ __forceinline__ long long widen_ordered32(int32_t k) {
   return ordered((double)__uint_as_float(u));
 }
 
-template <typename T>
-__device__ __forceinline__ void few_load(const GAgg& a, const uint32_t (&row)[kFewItems], uint32_t use,
-                                         T (&v)[kFewItems]) {
+// Raw cells of a thread's rows of one input column (4-byte cells zero-extended).
+// Rows r0, r0 + kFewThreads, ...; the ones at or past `rows` read the last row.
+template <typename T, typename V>
+__device__ __forceinline__ void few_cells(const void* data, uint32_t r0, uint32_t rows, V (&v)[kFewItems]) {
+  if (r0 + (kFewItems - 1) * kFewThreads < rows) {
+    const T* p = static_cast<const T*>(data) + r0;
 #pragma unroll
-  for (int q = 0; q < kFewItems; ++q) v[q] = (use >> q & 1u) ? __ldg(static_cast<const T*>(a.data) + row[q]) : T(0);
+    for (int q = 0; q < kFewItems; ++q) v[q] = __ldg(p + q * kFewThreads);
+  } else {
+#pragma unroll
+    for (int q = 0; q < kFewItems; ++q) v[q] = __ldg(static_cast<const T*>(data) + min(r0 + q * kFewThreads, rows - 1u));
+  }
+}
+__device__ __forceinline__ void few_load(const FewCol& c, uint32_t r0, uint32_t rows,
+                                         unsigned long long (&v)[kFewItems]) {
+  if (c.width == 4) few_cells<uint32_t>(c.data, r0, rows, v);
+  else if (c.width == 8) few_cells<unsigned long long>(c.data, r0, rows, v);
 }
 
-// One aggregate over a thread's rows: F folds a value into the accumulator.
-template <typename T, typename A, typename F>
-__device__ __forceinline__ void few_fold(const GAgg& a, A* acc, const uint32_t (&row)[kFewItems],
-                                         const uint32_t (&g)[kFewItems], uint32_t use, F f) {
-  T v[kFewItems];
-  few_load<T>(a, row, use, v);
+// One aggregate over a thread's rows: f folds a cell into the accumulator.
+// `e`: each row's element of an accumulator array; `all`: every row of every
+// thread of the warp counts (no test a row).
+template <typename A, typename F>
+__device__ __forceinline__ void few_fold(char* val, const unsigned long long (&v)[kFewItems],
+                                         const uint32_t (&e)[kFewItems], uint32_t use, bool all, F f) {
+  A* const acc = reinterpret_cast<A*>(val);
+  if (all) {
 #pragma unroll
-  for (int q = 0; q < kFewItems; ++q)
-    if (use >> q & 1u) {
-      A* p = acc + g[q] * kFewThreads + threadIdx.x;
-      *p = f(*p, v[q]);
-    }
+    for (int q = 0; q < kFewItems; ++q) acc[e[q]] = f(acc[e[q]], v[q]);
+  } else {
+#pragma unroll
+    for (int q = 0; q < kFewItems; ++q)
+      if (use >> q & 1u) acc[e[q]] = f(acc[e[q]], v[q]);
+  }
 }
 
-__global__ void __launch_bounds__(kFewThreads) k_few_accumulate(const __grid_constant__ FewParams F) {
+// A key's slot and its group index side by side: one load a probe.
+template <typename K>
+struct FewSlot {
+  K key;
+  K gid;  // kNoGroup: empty
+};
+constexpr uint32_t kNoGroup = 0xffffffffu;
+
+template <typename K>
+__global__ void __launch_bounds__(kFewThreads, 5) k_few_accumulate(const __grid_constant__ FewParams F) {
   extern __shared__ __align__(16) char s_few[];
-  unsigned long long* s_keys = reinterpret_cast<unsigned long long*>(s_few);
-  uint32_t* s_gid = reinterpret_cast<uint32_t*>(s_keys + kFewSlots);
-  char* s_acc = reinterpret_cast<char*>(s_gid + kFewSlots);
+  FewSlot<K>* s_slot = reinterpret_cast<FewSlot<K>*>(s_few);
+  char* s_acc = s_few + kFewSlots * sizeof(FewSlot<K>);
   const uint32_t G = F.ngroups, tid = threadIdx.x;
   const size_t unit = (size_t)G * kFewThreads;  // elements of one array
   for (uint32_t i = tid; i < kFewSlots; i += kFewThreads) {
-    s_keys[i] = F.T->keys[i];
-    s_gid[i] = F.T->gid[i];
+    const unsigned long long key = F.T->keys[i];
+    s_slot[i].key = (K)key;
+    s_slot[i].gid = key == kNoKey ? (K)kNoGroup : (K)F.T->gid[i];
   }
   for (size_t i = tid * 4; i < unit * F.bytes; i += kFewThreads * 4) *reinterpret_cast<uint32_t*>(s_acc + i) = 0u;
   __syncthreads();
@@ -676,83 +742,110 @@ __global__ void __launch_bounds__(kFewThreads) k_few_accumulate(const __grid_con
     }
   }
   uint32_t* const rows_acc = reinterpret_cast<uint32_t*>(s_acc);
-  const unsigned long long r_begin = (unsigned long long)blockIdx.x * F.rows_per_block;
-  const unsigned long long r_end = min((unsigned long long)F.P.rows, r_begin + F.rows_per_block);
+  constexpr uint32_t STEP = kFewThreads * kFewItems;
+  const uint32_t rows = F.P.rows;
+  const uint32_t r_begin = blockIdx.x * F.rows_per_block;  // a whole number of steps
+  const uint32_t r_end = min(rows, r_begin + F.rows_per_block);
   const uint32_t last_gid = F.T->last_gid;
-  for (unsigned long long base = r_begin; base < r_end; base += kFewThreads * kFewItems) {
-    uint32_t row[kFewItems], g[kFewItems], in = 0u;
-    unsigned long long k[kFewItems];
+  // The keys of the next step and the next column's cells are always in flight
+  // while the current ones are folded.
+  K k[kFewItems];
+  few_cells<K>(F.key.data, r_begin + tid, rows, k);
+  for (uint32_t base = r_begin; base < r_end; base += STEP) {
+    const uint32_t r0 = base + tid;
+    uint32_t g[kFewItems], in = (1u << kFewItems) - 1u;
+    unsigned long long v[kFewItems];
+    if (base + STEP > r_end) {
+#pragma unroll
+      for (int q = 0; q < kFewItems; ++q)
+        if (r0 + q * kFewThreads >= r_end) in &= ~(1u << q);
+    }
+    if (F.ncol) few_load(F.col[0], r0, rows, v);
 #pragma unroll
     for (int q = 0; q < kFewItems; ++q) {
-      const unsigned long long r = base + q * kFewThreads + tid;
-      row[q] = r < r_end ? (uint32_t)r : 0u;
-      if (r < r_end) in |= 1u << q;
-      k[q] = few_key(F.key, row[q]);
+      uint32_t h = few_hash(k[q]);
+      FewSlot<K> at = s_slot[h];
+      if (sizeof(K) == 8 && (unsigned long long)k[q] == kNoKey) {
+        at.gid = (K)last_gid;
+      } else {
+        for (uint32_t n = 0; n < kFewSlots && at.key != k[q]; ++n) {  // a collision (rare)
+          h = (h + 1) & (kFewSlots - 1);
+          at = s_slot[h];
+        }
+      }
+      g[q] = (uint32_t)at.gid;
     }
 #pragma unroll
     for (int q = 0; q < kFewItems; ++q) {
-      if (k[q] == kNoKey) {
-        g[q] = last_gid;
-      } else {
-        uint32_t h = few_hash(k[q]);
-        for (uint32_t n = 0; n < kFewSlots && s_keys[h] != k[q]; ++n) h = (h + 1) & (kFewSlots - 1);
-        g[q] = s_gid[h];
-      }
       if (g[q] >= G) {  // cannot be: k_few_find saw every key
+        if (in >> q & 1u) atomicOr(F.P.err, kErrBounds);
         in &= ~(1u << q);
         g[q] = 0u;
-        atomicOr(F.P.err, kErrBounds);
       }
+      g[q] = g[q] * kFewThreads + tid;  // its element from here on
     }
+    if (base + STEP < r_end) few_cells<K>(F.key.data, r0 + STEP, rows, k);
 #pragma unroll
     for (int q = 0; q < kFewItems; ++q)
-      if (in >> q & 1u) ++rows_acc[g[q] * kFewThreads + tid];
-    for (int j = 0; j < F.P.nagg; ++j) {
-      const GAgg& a = F.P.a[j];
-      const FewAcc& A = F.acc[j];
+      if (in >> q & 1u) ++rows_acc[g[q]];
+    for (int c = 0; c < F.ncol; ++c) {
+      const FewCol& C = F.col[c];
+      unsigned long long next[kFewItems];
+      if (c + 1 < F.ncol) few_load(F.col[c + 1], r0, rows, next);
       uint32_t use = in;
-      if (a.kind == YQ_AGG_COUNT_STAR) continue;
-      if (a.nulls) {
-        uint32_t* cnt = reinterpret_cast<uint32_t*>(s_acc + unit * A.cnt_off);
+      if (C.nulls) {
+        uint32_t* cnt = reinterpret_cast<uint32_t*>(s_acc + unit * C.cnt_off);
+        uint8_t nul[kFewItems];
+#pragma unroll
+        for (int q = 0; q < kFewItems; ++q) nul[q] = __ldg(C.nulls + min(r0 + q * kFewThreads, rows - 1u));
 #pragma unroll
         for (int q = 0; q < kFewItems; ++q)
           if (use >> q & 1u) {
-            if (a.nulls[row[q]]) use &= ~(1u << q);
-            else ++cnt[g[q] * kFewThreads + tid];
+            if (nul[q]) use &= ~(1u << q);
+            else ++cnt[g[q]];
           }
       }
-      if (A.val_off < 0) continue;
-      char* const val = s_acc + unit * A.val_off;
-      if (a.kind == YQ_AGG_SUM || a.kind == YQ_AGG_AVG) {
-        if (a.type == YQ_FLOAT32)
-          few_fold<float>(a, reinterpret_cast<double*>(val), row, g, use, [](double x, float v) { return x + (double)v; });
-        else if (a.type == YQ_FLOAT64)
-          few_fold<double>(a, reinterpret_cast<double*>(val), row, g, use, [](double x, double v) { return x + v; });
-        else if (a.type == YQ_INT32)
-          few_fold<int32_t>(a, reinterpret_cast<long long*>(val), row, g, use,
-                            [](long long x, int32_t v) { return (long long)((unsigned long long)x + (unsigned long long)(long long)v); });
-        else
-          few_fold<long long>(a, reinterpret_cast<long long*>(val), row, g, use,
-                              [](long long x, long long v) { return (long long)((unsigned long long)x + (unsigned long long)v); });
-      } else {
-        const bool lo = a.kind == YQ_AGG_MIN;
-        if (a.type == YQ_FLOAT32)
-          few_fold<float>(a, reinterpret_cast<int32_t*>(val), row, g, use, [lo](int32_t x, float v) {
-            const int32_t o = ordered32(v);
-            return lo ? min(x, o) : max(x, o);
-          });
-        else if (a.type == YQ_INT32)
-          few_fold<int32_t>(a, reinterpret_cast<int32_t*>(val), row, g, use,
-                            [lo](int32_t x, int32_t v) { return lo ? min(x, v) : max(x, v); });
-        else if (a.type == YQ_FLOAT64)
-          few_fold<double>(a, reinterpret_cast<long long*>(val), row, g, use, [lo](long long x, double v) {
-            const long long o = ordered(v);
-            return lo ? min(x, o) : max(x, o);
-          });
-        else
-          few_fold<long long>(a, reinterpret_cast<long long*>(val), row, g, use,
-                              [lo](long long x, long long v) { return lo ? min(x, v) : max(x, v); });
+      const bool all = __all_sync(0xffffffffu, use == (1u << kFewItems) - 1u);
+      for (int x = C.first; x < C.first + C.count; ++x) {
+        const int j = F.order[x];
+        if (F.acc[j].val_off < 0) continue;  // a count
+        char* const val = s_acc + unit * F.acc[j].val_off;
+        const int kind = F.P.a[j].kind;
+        if (kind == YQ_AGG_SUM || kind == YQ_AGG_AVG) {
+          if (C.type == YQ_FLOAT32)
+            few_fold<double>(val, v, g, use, all, [](double s, unsigned long long b) { return s + (double)__uint_as_float((uint32_t)b); });
+          else if (C.type == YQ_FLOAT64)
+            few_fold<double>(val, v, g, use, all, [](double s, unsigned long long b) { return s + __longlong_as_double((long long)b); });
+          else if (C.type == YQ_INT32)
+            few_fold<unsigned long long>(val, v, g, use, all, [](unsigned long long s, unsigned long long b) {
+              return s + (unsigned long long)(long long)(int32_t)(uint32_t)b;
+            });
+          else
+            few_fold<unsigned long long>(val, v, g, use, all, [](unsigned long long s, unsigned long long b) { return s + b; });
+        } else {
+          const bool lo = kind == YQ_AGG_MIN;
+          if (C.type == YQ_FLOAT32)
+            few_fold<int32_t>(val, v, g, use, all, [lo](int32_t s, unsigned long long b) {
+              const int32_t o = ordered32(__uint_as_float((uint32_t)b));
+              return lo ? min(s, o) : max(s, o);
+            });
+          else if (C.type == YQ_INT32)
+            few_fold<int32_t>(val, v, g, use, all, [lo](int32_t s, unsigned long long b) {
+              return lo ? min(s, (int32_t)(uint32_t)b) : max(s, (int32_t)(uint32_t)b);
+            });
+          else if (C.type == YQ_FLOAT64)
+            few_fold<long long>(val, v, g, use, all, [lo](long long s, unsigned long long b) {
+              const long long o = ordered(__longlong_as_double((long long)b));
+              return lo ? min(s, o) : max(s, o);
+            });
+          else
+            few_fold<long long>(val, v, g, use, all, [lo](long long s, unsigned long long b) {
+              return lo ? min(s, (long long)b) : max(s, (long long)b);
+            });
+        }
       }
+#pragma unroll
+      for (int q = 0; q < kFewItems; ++q) v[q] = next[q];
     }
   }
   __syncthreads();
@@ -792,11 +885,14 @@ __global__ void __launch_bounds__(kFewThreads) k_few_accumulate(const __grid_con
   }
 }
 
-// One warp per (group, aggregate): the blocks' partials in block order.
-__global__ void __launch_bounds__(32) k_few_finish(const __grid_constant__ FewParams F, uint32_t nblocks) {
+// One block per (group, aggregate): the blocks' partials in a fixed order (a
+// thread's in block order, lanes pairwise, then the warps).
+constexpr int kFinishThreads = 128;
+__global__ void __launch_bounds__(kFinishThreads) k_few_finish(const __grid_constant__ FewParams F, uint32_t nblocks) {
+  __shared__ GPart s_part[kFinishThreads / 32];
   const uint32_t g = blockIdx.x;
-  const int j = blockIdx.y, lane = threadIdx.x;
-  if (j == 0 && lane == 0) {
+  const int j = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (j == 0 && threadIdx.x == 0) {
     const unsigned long long k = F.T->group_key[g];
     if (F.out_key.width == 4) static_cast<uint32_t*>(F.out_key.data)[g] = (uint32_t)k;
     else static_cast<unsigned long long*>(F.out_key.data)[g] = k;
@@ -806,14 +902,21 @@ __global__ void __launch_bounds__(32) k_few_finish(const __grid_constant__ FewPa
   const GAgg& a = F.P.a[j];
   const bool flt = is_float(a.type);
   GPart acc = part_identity(a.kind);
-  for (uint32_t b = lane; b < nblocks; b += 32)
+#pragma unroll 4
+  for (uint32_t b = threadIdx.x; b < nblocks; b += kFinishThreads)
     acc = part_combine(a.kind, flt, acc, F.part[((size_t)b * F.ngroups + g) * F.P.nagg + j]);
 #pragma unroll
   for (int d = 1; d < 32; d <<= 1) {
     const GPart o{__shfl_down_sync(0xffffffffu, acc.cnt, d), __shfl_down_sync(0xffffffffu, acc.v, d)};
     if ((lane & (2 * d - 1)) == 0) acc = part_combine(a.kind, flt, acc, o);
   }
-  if (lane == 0) part_write(a, F.P.out[j], g, acc);
+  if (lane == 0) s_part[warp] = acc;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    GPart tot = s_part[0];
+    for (int w = 1; w < kFinishThreads / 32; ++w) tot = part_combine(a.kind, flt, tot, s_part[w]);
+    part_write(a, F.P.out[j], g, tot);
+  }
 }
 
 int out_type(int32_t kind, int32_t in) {
@@ -849,8 +952,9 @@ size_t few_workspace_bytes(int32_t nagg) {
 // its launches and its read-back take about 25 us).
 constexpr uint32_t kFewMinRows = 100000;
 
+// (Above 2^30 rows the sort refuses the call, and 32-bit row arithmetic ends.)
 bool few_applies(const yq_column& key, uint32_t rows) {
-  return rows >= kFewMinRows && (key.type == YQ_INT32 || key.type == YQ_INT64 || key.type == YQ_DATETIME);
+  return rows >= kFewMinRows && rows < (1u << 30) && (key.type == YQ_INT32 || key.type == YQ_INT64 || key.type == YQ_DATETIME);
 }
 
 // The sort-free path. *done = false: the keys are too many (or one is NULL)
@@ -867,10 +971,16 @@ int group_by_few(const GroupParams& P, const yq_column& key, const yq_column& ou
   YQ_TRY_CUDA(cudaMemsetAsync(&T->count, 0, sizeof(FewTable) - sizeof(T->keys), s));
   const unsigned step = kFewFindThreads * kFewItems;
   unsigned grid = grid_for(P.rows, step);
-  if (grid > (unsigned)sm_count() * 8) grid = (unsigned)sm_count() * 8;
+  const void* find = key.width == 4 ? (const void*)k_few_find<uint32_t> : (const void*)k_few_find<unsigned long long>;
+  const unsigned resident = (unsigned)(sm_count() * kernel_blocks_per_sm(find, kFewFindThreads, 0));
+  if (grid > resident) grid = resident;
   {
     ProfScope ps("group_few_find", s, (double)P.rows * key.width);
-    k_few_find<<<grid, kFewFindThreads, 0, s>>>(key, P.rows, T);
+    if (key.width == 4)
+      k_few_find<uint32_t><<<grid, kFewFindThreads, 0, s>>>(static_cast<const uint32_t*>(key.data), key.nulls, P.rows, T);
+    else
+      k_few_find<unsigned long long><<<grid, kFewFindThreads, 0, s>>>(static_cast<const unsigned long long*>(key.data),
+                                                                      key.nulls, P.rows, T);
     YQ_CHECK_LAUNCH();
   }
   k_few_order<<<1, kFewSlots, 0, s>>>(T, key.width);
@@ -892,14 +1002,30 @@ int group_by_few(const GroupParams& P, const yq_column& key, const yq_column& ou
   auto value_size = [&](int j) {
     const GAgg& a = P.a[j];
     if (a.kind == YQ_AGG_COUNT || a.kind == YQ_AGG_COUNT_STAR) return 0;
-    return a.kind == YQ_AGG_SUM || a.kind == YQ_AGG_AVG || type_width(a.type) == 8 ? 8 : 4;
+    return a.kind == YQ_AGG_SUM || a.kind == YQ_AGG_AVG || a.width == 8 ? 8 : 4;
   };
   off = 4;  // the row counts; padded to 8 with the 4-byte arrays placed first
+  F.ncol = 0;
+  int placed = 0;
+  for (int j = 0; j < P.nagg; ++j) F.acc[j] = FewAcc{0, -1, 0};
   for (int j = 0; j < P.nagg; ++j) {
-    F.acc[j] = FewAcc{0, -1, 0};
-    if (P.a[j].kind != YQ_AGG_COUNT_STAR && P.a[j].nulls) {
-      F.acc[j].cnt_off = off;
+    if (P.a[j].kind == YQ_AGG_COUNT_STAR || (P.a[j].kind == YQ_AGG_COUNT && !P.a[j].nulls)) continue;  // the row count
+    bool seen = false;
+    for (int i = 0; i < placed; ++i) seen |= F.order[i] == j;
+    if (seen) continue;
+    FewCol& C = F.col[F.ncol++];
+    C = FewCol{P.a[j].data, P.a[j].nulls, P.a[j].type, 0, placed, 0, 0};
+    if (C.nulls) {
+      C.cnt_off = off;
       off += 4;
+    }
+    for (int i = j; i < P.nagg; ++i) {
+      const GAgg& a = P.a[i];
+      if (a.kind == YQ_AGG_COUNT_STAR || a.data != C.data || a.nulls != C.nulls || a.type != C.type) continue;
+      F.order[placed++] = (int8_t)i;
+      ++C.count;
+      if (a.kind != YQ_AGG_COUNT) C.width = a.width;
+      F.acc[i].cnt_off = C.cnt_off;
     }
   }
   for (const int size : {4, 8}) {
@@ -911,15 +1037,17 @@ int group_by_few(const GroupParams& P, const yq_column& key, const yq_column& ou
     }
   }
   F.bytes = off;
-  const size_t smem = kFewSlots * 12 + (size_t)G * kFewThreads * off;
+  const size_t smem = (size_t)kFewSlots * 2 * key.width + (size_t)G * kFewThreads * off;
   if (smem > 220 * 1024) return YQ_OK;  // too many accumulators for one block
   if (G > capacity) {
     *groups = G;
     *done = true;
     return YQ_ERR_CAPACITY;
   }
-  YQ_TRY(kernel_allow_smem((const void*)k_few_accumulate, smem));
-  int per_sm = kernel_blocks_per_sm((const void*)k_few_accumulate, kFewThreads, smem);
+  void (*const accumulate)(FewParams) =
+      key.width == 4 ? k_few_accumulate<uint32_t> : k_few_accumulate<unsigned long long>;
+  YQ_TRY(kernel_allow_smem((const void*)accumulate, smem));
+  int per_sm = kernel_blocks_per_sm((const void*)accumulate, kFewThreads, smem);
   if (per_sm > kFewBlocksPerSm) per_sm = kFewBlocksPerSm;
   unsigned blocks = grid_for(P.rows, kFewThreads * kFewItems);
   if (blocks > (unsigned)(sm_count() * per_sm)) blocks = (unsigned)(sm_count() * per_sm);
@@ -931,10 +1059,10 @@ int group_by_few(const GroupParams& P, const yq_column& key, const yq_column& ou
     if (P.a[j].data) in_bytes += (double)P.rows * (type_width(P.a[j].type) + (P.a[j].nulls ? 1 : 0));
   {
     ProfScope ps("group_few_accumulate", s, in_bytes);
-    k_few_accumulate<<<blocks, kFewThreads, smem, s>>>(F);
+    accumulate<<<blocks, kFewThreads, smem, s>>>(F);
     YQ_CHECK_LAUNCH();
   }
-  k_few_finish<<<dim3(G, (unsigned)(P.nagg > 0 ? P.nagg : 1)), 32, 0, s>>>(F, blocks);
+  k_few_finish<<<dim3(G, (unsigned)(P.nagg > 0 ? P.nagg : 1)), kFinishThreads, 0, s>>>(F, blocks);
   YQ_CHECK_LAUNCH();
   uint32_t err = 0;
   YQ_TRY(d2h_sync(&err, d_err, sizeof(err), s));
@@ -1007,7 +1135,7 @@ int yq_group_by(const yq_batch* batch, int32_t key_col, const yq_group_agg* aggs
     const yq_column& o = out[1 + j];
     if (o.type != ot || o.width != type_width(ot) || (rows && !o.data)) return YQ_ERR_INVALID_ARG;
     if (!o.nulls && g.kind != YQ_AGG_COUNT && g.kind != YQ_AGG_COUNT_STAR && rows) return YQ_ERR_INVALID_ARG;
-    P.a[j] = GAgg{in.data, in.nulls, it, g.kind};
+    P.a[j] = GAgg{in.data, in.nulls, it, g.kind, in.width};
     P.out[j] = o;
   }
   if (rows == 0) return YQ_OK;
