@@ -827,15 +827,17 @@ YQ_CSV_HD bool fast_float32(FieldCursor& c, float* out) {
   uint32_t sign = 0;
   if (j < c.len && (c.rec[j] == '-' || c.rec[j] == '+')) { sign = c.rec[j] == '-' ? 0x80000000u : 0u; ++j; }
   uint64_t w = 0;
+  uint32_t w9 = 0;  // the first nine significant digits: most fields have no more
   int nd = 0, frac = 0, digits = 0;
   bool dot = false;
   for (; j < c.len; ++j) {
     const uint32_t ch = c.rec[j];
     if (ch - '0' < 10u) {
       ++digits;
-      if (w == 0 && ch == '0') { if (dot) ++frac; continue; }
+      if (nd == 0 && ch == '0') { if (dot) ++frac; continue; }
       if (nd == 19) return false;
-      w = w * 10 + (ch - '0');
+      if (nd < 9) w9 = w9 * 10 + (ch - '0');
+      else w = (nd == 9 ? (uint64_t)w9 : w) * 10 + (ch - '0');
       ++nd;
       if (dot) ++frac;
     } else if (ch == '.' && !dot) {
@@ -847,6 +849,7 @@ YQ_CSV_HD bool fast_float32(FieldCursor& c, float* out) {
   if (digits == 0) return false;
   if (j < c.len && (c.rec[j] == 'e' || c.rec[j] == 'E')) return false;
   const uint32_t j_end = j;
+  if (nd <= 9) w = w9;
   if (w == 0) {
     if (!FieldCursor_end(c, j_end)) return false;
     *out = bits_float(sign);
@@ -884,7 +887,16 @@ YQ_CSV_HD bool fast_datetime(FieldCursor& c, int64_t* out) {
   const int mi = m0 * 10 + (p[15] - '0'), se = s0 * 10 + (p[18] - '0');
   if (M < 1 || M > 12 || D < 1 || D > 31 || h > 23 || mi > 59 || se > 61) return false;
   if (!FieldCursor_end(c, c.i + 19)) return false;
-  *out = days_from_civil(Y, M, D) * 86400 + h * 3600 + mi * 60 + se;
+  int64_t days;
+  if (Y >= 1) {  // days_from_civil in 32 bits: the shifted year is not negative
+    const uint32_t y = (uint32_t)Y - (M <= 2), era = y / 400u, yoe = y - era * 400u;
+    const uint32_t doy = (153u * (uint32_t)(M + (M > 2 ? -3 : 9)) + 2u) / 5u + (uint32_t)D - 1u;
+    const uint32_t doe = yoe * 365u + yoe / 4u - yoe / 100u + doy;
+    days = (int32_t)(era * 146097u + doe) - 719468;
+  } else {
+    days = days_from_civil(Y, M, D);
+  }
+  *out = days * 86400 + (h * 3600 + mi * 60 + se);
   return true;
 }
 
@@ -895,6 +907,15 @@ YQ_CSV_HD bool fast_text(FieldCursor& c, uint32_t width, Store& store) {
   if (c.done || (c.i < c.len && c.rec[c.i] == '"')) return false;
   uint32_t j = c.i, o = 0, word = 0;
   bool stop = false;
+  // whole words of ordinary bytes, while the slot keeps room for the NUL
+  while (j + 4 <= c.len && o + 4 < width) {
+    const uint32_t w = (uint32_t)c.rec[j] | (uint32_t)c.rec[j + 1] << 8 | (uint32_t)c.rec[j + 2] << 16 |
+                       (uint32_t)c.rec[j + 3] << 24;
+    if (eq4(w, 0x2c2c2c2cu) | eq4(w, 0x0a0a0a0au) | eq4(w, 0x0d0d0d0du) | eq4(w, 0u)) break;
+    store(o / 4, w);
+    o += 4;
+    j += 4;
+  }
   for (; j < c.len; ++j) {
     const uint32_t ch = c.rec[j];
     if (ch == ',' || ch == '\n' || ch == '\r') break;
@@ -1037,8 +1058,26 @@ YQ_CSV_HD void copy_text(View v, bool escapes, uint32_t width, Store& store) {
 // put(c) (append a byte), put_at(k, c) (the byte k places after the current
 // end, before a skip(n) that moves the end past it) and skip(n).
 
+// Nearly every number written fits 32 bits, whose division by ten is one wide
+// multiply; a 64-bit one is an order more instructions, twice a digit.
+template <class Out>
+YQ_CSV_HD void put_u32(Out& o, uint32_t v) {
+  const uint32_t n = 1 + (v >= 10u) + (v >= 100u) + (v >= 1000u) + (v >= 10000u) + (v >= 100000u) + (v >= 1000000u) +
+                     (v >= 10000000u) + (v >= 100000000u) + (v >= 1000000000u);
+  for (uint32_t k = n; k-- > 0;) {
+    const uint32_t q = v / 10u;
+    o.put_at(k, '0' + (v - q * 10u));
+    v = q;
+  }
+  o.skip(n);
+}
+
 template <class Out>
 YQ_CSV_HD void put_u64(Out& o, uint64_t v) {
+  if (v >> 32 == 0) {
+    put_u32(o, (uint32_t)v);
+    return;
+  }
   uint32_t n = 1;
   for (uint64_t t = v; t >= 10; t /= 10) ++n;
   for (uint32_t k = n; k-- > 0; v /= 10) o.put_at(k, (uint32_t)('0' + v % 10));
@@ -1116,8 +1155,15 @@ YQ_CSV_HD void put_fixed4(Out& o, float x) {
     const uint64_t r = t & ((1ull << k) - 1), half = 1ull << (k - 1);
     if (r > half || (r == half && (q & 1))) ++q;
   }
-  put_u64(o, q / 10000);
-  uint32_t f = (uint32_t)(q % 10000);
+  uint32_t f;
+  if (q >> 32 == 0) {
+    const uint32_t i = (uint32_t)q / 10000u;
+    f = (uint32_t)q - i * 10000u;
+    put_u32(o, i);
+  } else {
+    put_u64(o, q / 10000);
+    f = (uint32_t)(q % 10000);
+  }
   o.put('.');
   o.put('0' + f / 1000);
   o.put('0' + f / 100 % 10);
@@ -1142,22 +1188,34 @@ YQ_CSV_HD void civil_from_days(int64_t z, int64_t* y, uint32_t* m, uint32_t* d) 
 // gmtime_r + strftime("%Y-%m-%d %H:%M:%S"): the year unpadded, with its sign.
 template <class Out>
 YQ_CSV_HD void put_datetime(Out& o, int64_t secs) {
-  int64_t days = secs / 86400, rem = secs % 86400;
-  if (rem < 0) { rem += 86400; --days; }
-  int64_t y;
-  uint32_t mo, d;
-  civil_from_days(days, &y, &mo, &d);
-  put_i64(o, y);
+  uint32_t mo, d, rem;
+  if ((uint64_t)secs >> 32 == 0) {  // 1970 to 2106: civil_from_days in 32 bits
+    const uint32_t days = (uint32_t)secs / 86400u, z = days + 719468u;
+    rem = (uint32_t)secs - days * 86400u;
+    const uint32_t era = z / 146097u, doe = z - era * 146097u;
+    const uint32_t yoe = (doe - doe / 1460u + doe / 36524u - doe / 146096u) / 365u;
+    const uint32_t doy = doe - (365u * yoe + yoe / 4u - yoe / 100u);
+    const uint32_t mp = (5u * doy + 2u) / 153u;
+    d = doy - (153u * mp + 2u) / 5u + 1u;
+    mo = mp < 10u ? mp + 3u : mp - 9u;
+    put_u32(o, yoe + era * 400u + (mo <= 2u));
+  } else {
+    int64_t days = secs / 86400, r = secs % 86400, y;
+    if (r < 0) { r += 86400; --days; }
+    rem = (uint32_t)r;
+    civil_from_days(days, &y, &mo, &d);
+    put_i64(o, y);
+  }
   o.put('-');
   put_2(o, mo);
   o.put('-');
   put_2(o, d);
   o.put(' ');
-  put_2(o, (uint32_t)(rem / 3600));
+  put_2(o, rem / 3600u);
   o.put(':');
-  put_2(o, (uint32_t)(rem / 60 % 60));
+  put_2(o, rem / 60u % 60u);
   o.put(':');
-  put_2(o, (uint32_t)(rem % 60));
+  put_2(o, rem % 60u);
 }
 
 // One cell. type: YQ_INT32 0, YQ_FLOAT32 1, YQ_DATETIME 2, YQ_TEXT 3, YQ_INT64 4.
