@@ -57,8 +57,10 @@ __device__ __forceinline__ uint32_t digit_of(const uint32_t (&k)[KW], int shift)
 // Fixed-width numeric columns without nulls, the common case, load every value
 // before any is transformed, so a thread keeps N reads in flight; a type switch
 // around each load would wait for one before it issues the next.
+// *lossy (when the caller asks for it): set when a value would not survive its key.
 template <int KW, int N>
-__device__ __forceinline__ void load_keys(const KeySrc& s, const uint32_t (&rows)[N], uint32_t ok, uint32_t (&k)[N][KW]) {
+__device__ __forceinline__ void load_keys(const KeySrc& s, const uint32_t (&rows)[N], uint32_t ok, uint32_t (&k)[N][KW],
+                                          bool* lossy = nullptr) {
   if (KW == 1 && !s.null_word && (s.type == YQ_INT32 || s.type == YQ_FLOAT32)) {
     uint32_t v[N];
 #pragma unroll
@@ -69,8 +71,13 @@ __device__ __forceinline__ void load_keys(const KeySrc& s, const uint32_t (&rows
       for (int i = 0; i < N; ++i) k[i][0] = v[i] ^ 0x80000000u ^ inv;
     } else {
 #pragma unroll
-      for (int i = 0; i < N; ++i) k[i][0] = float_key(v[i]) ^ inv;
+      for (int i = 0; i < N; ++i) {
+        const uint32_t f = float_key(v[i]);
+        if (lossy) *lossy |= ((f & 0x80000000u) ? (f & 0x7fffffffu) : ~f) != v[i];
+        k[i][0] = f ^ inv;
+      }
     }
+    return;
   } else if (KW == 2 && !s.null_word && (s.type == YQ_INT64 || s.type == YQ_DATETIME)) {
     uint2 v[N];
 #pragma unroll
@@ -82,7 +89,9 @@ __device__ __forceinline__ void load_keys(const KeySrc& s, const uint32_t (&rows
       k[i][0] = v[i].x ^ inv;
       k[i][KW > 1 ? 1 : 0] = v[i].y ^ 0x80000000u ^ inv;
     }
-  } else if (KW == 2 && s.nsel) {
+    return;
+  }
+  if (KW == 2 && s.nsel) {
 #pragma unroll
     for (int i = 0; i < N; ++i) {
       uint32_t f[4] = {0u, 0u, 0u, 0u};
@@ -104,6 +113,12 @@ __device__ __forceinline__ void load_keys(const KeySrc& s, const uint32_t (&rows
         for (int j = 0; j < KW; ++j) k[i][j] = 0u;
       }
     }
+  }
+  if (lossy) {
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+      *lossy |= (ok >> i & 1u) && !(s.nulls && s.nulls[rows[i]]) &&
+                key_value_lossy(s.type, s.data + (size_t)rows[i] * s.width);
   }
 }
 
@@ -155,6 +170,7 @@ __global__ void __launch_bounds__(kSortBlock) k_sort_histogram(const KeySrc src,
   const uint32_t t0 = blockIdx.x * per;
   const uint32_t t1 = min(ntiles, t0 + per);
   int cur = -1;
+  bool lossy = false;
   for (uint32_t t = t0; t < t1; ++t) {
     const int sg = find_segment(seg, t);
     if (sg != cur) {
@@ -176,15 +192,12 @@ __global__ void __launch_bounds__(kSortBlock) k_sort_histogram(const KeySrc src,
         if (e < r1) ok |= 1u << i;
         row[i] = e < r1 ? (src.in_perm ? __ldg(src.in_perm + e) : e) : 0u;
       }
-      load_keys<KW, N>(src, row, ok, k);
+      // the key column is read here anyway: flag values the key words cannot restore
+      if (src.lossy) load_keys<KW, N>(src, row, ok, k, &lossy);
+      else load_keys<KW, N>(src, row, ok, k);
 #pragma unroll
       for (int i = 0; i < N; ++i) {
         const bool valid = ok >> i & 1u;
-        if (src.lossy) {  // the key column is read here anyway: flag values the key words cannot restore
-          const bool l = valid && !(src.nulls && src.nulls[row[i]]) &&
-                         key_value_lossy(src.type, src.data + (size_t)row[i] * src.width);
-          if (__any_sync(0xffffffffu, l) && lane == 0) atomicOr(src.lossy, 1u);
-        }
         const uint32_t vb = __ballot_sync(0xffffffffu, valid);
         const int first = __ffs(vb) - 1;
         // One vote per key: when every valid lane of the warp holds the same key
@@ -209,6 +222,7 @@ __global__ void __launch_bounds__(kSortBlock) k_sort_histogram(const KeySrc src,
       }
     }
   }
+  if (src.lossy && __any_sync(0xffffffffu, lossy) && lane == 0) atomicOr(src.lossy, 1u);
   __syncthreads();
   if (cur >= 0) flush(cur);
 }
@@ -769,7 +783,7 @@ static bool pick_kernels(int kw, int d, int items, int block, SortKernels& k) {
   if (block != 0 && block != kSortBlock) return false;
   switch (kw * 10000 + d * 100 + items) {
     case 10816: k = make_kernels<1, 8, 16>(); return true;
-    case 10812: case 10800: k = make_kernels<1, 8, 12>(); return true;  // 12 items: four blocks per SM
+    case 10812: case 10800: k = make_kernels<1, 8, 12>(); return true;
     case 10808: k = make_kernels<1, 8, 8>(); return true;
     case 10616: case 10600: k = make_kernels<1, 6, 16>(); return true;
     case 10416: case 10400: k = make_kernels<1, 4, 16>(); return true;
@@ -805,11 +819,30 @@ static int rows_bucket(uint32_t rows, int nseg) {
   return b;
 }
 
+// The variant of an untuned sort: 8-bit digits, and for one-word keys a tile by
+// the rows at hand. Tiles of 4,096 rows are the fewest look-backs (64M rows:
+// 1.98 ms against 2.05 with 3,072, whose histogram steps are also ragged); a
+// sort of fewer tiles than the device holds finishes sooner with its 4,096 rows
+// on 512 threads (4M: 0.21 against 0.23 ms; 1M: 0.12 against 0.13); segments of
+// a tile or two want the smallest tile (90 segments of 13K rows on average:
+// 0.147 against 0.155 ms).
+constexpr uint32_t kManyRows = 1u << 23, kShortSegment = 1u << 16;
+static TunedSort default_choice(int kw, uint32_t rows, int nseg) {
+  if (kw != 1) return TunedSort{};
+  if (rows / (uint32_t)(nseg > 0 ? nseg : 1) < kShortSegment) return TunedSort{8, 8, 256};
+  return rows >= kManyRows ? TunedSort{8, 16, 256} : TunedSort{8, 8, 512};
+}
+
 static TunedSort tuned_choice(int kw, uint32_t rows, int nseg) {
   std::lock_guard<std::mutex> lk(g_tune_mu);
   auto it = g_tuned.find({kw, rows_bucket(rows, nseg)});
-  if (it == g_tuned.end()) return TunedSort{};
-  return it->second;
+  return it == g_tuned.end() ? default_choice(kw, rows, nseg) : it->second;
+}
+
+// Kernels for a key narrowed to `kw` words by the histogram.
+static bool pick_narrowed(int kw, int d, uint32_t rows, int nseg, SortKernels& k) {
+  const TunedSort t = default_choice(kw, rows, nseg);
+  return (t.d == d && pick_kernels(kw, d, t.items, t.block, k)) || pick_kernels(kw, d, 0, k);
 }
 
 struct SegPlan {
@@ -857,8 +890,10 @@ static int plan_key(const yq_column& c, int vwords_override, int want_d, int wan
   if (kp.D == 0) {
     const TunedSort t = tuned_choice(kp.sh.kw, seg_offsets[nseg] - seg_offsets[0], nseg);
     kp.D = t.d;
-    if (items == 0) items = t.items;
-    if (block == 0) block = t.block;
+    if (items == 0 && block == 0) {  // the caller's own items or block: that digit width's variant with them
+      items = t.items;
+      block = t.block;
+    }
   }
   if (!pick_kernels(kp.sh.kw, kp.D, items, block, kp.K)) {
     kp.D = 8;
@@ -1102,7 +1137,7 @@ int sort_segments_impl(const KeyJob* jobs, int njobs, uint32_t rows, const uint3
           ++shared;
         }
         const int kw_eff = round_kw(kp.sh.kw - shared);
-        if (kw_eff > 0 && kw_eff < kp.sh.kw && pick_kernels(kw_eff, kp.D, 0, kq.K)) {
+        if (kw_eff > 0 && kw_eff < kp.sh.kw && pick_narrowed(kw_eff, kp.D, rows, nseg, kq.K)) {
           kq.sh.kw = kw_eff;
           kq.P = kw_eff * ppw;
           kq.tile_rows = kq.K.tile_rows();
