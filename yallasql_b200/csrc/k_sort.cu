@@ -91,6 +91,28 @@ __device__ __forceinline__ void load_keys(const KeySrc& s, const uint32_t (&rows
     }
     return;
   }
+  const bool nullable8 = s.nulls && s.null_word && (s.type == YQ_INT64 || s.type == YQ_DATETIME);
+  if ((KW == 4 || (KW == 2 && s.nsel)) && nullable8) {  // their values and null bytes the same way
+    uint2 v[N];
+    uint8_t nul[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      v[i] = (ok >> i & 1u) ? __ldg(reinterpret_cast<const uint2*>(s.data) + rows[i]) : make_uint2(0u, 0u);
+      nul[i] = (ok >> i & 1u) ? __ldg(s.nulls + rows[i]) : 0;
+    }
+    const uint32_t inv = s.desc ? 0xffffffffu : 0u;
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const uint32_t f[3] = {(nul[i] ? 0u : v[i].x) ^ inv, ((nul[i] ? 0u : v[i].y) ^ 0x80000000u) ^ inv,
+                             (uint32_t)((nul[i] != 0) != (s.nulls_first != 0))};
+#pragma unroll
+      for (int j = 0; j < KW; ++j) {
+        k[i][j] = KW == 4 && j < 3 ? f[j < 3 ? j : 0] : 0u;
+        if (KW == 2 && j < s.nsel) k[i][j] = s.sel[j] == 0 ? f[0] : (s.sel[j] == 1 ? f[1] : f[2]);
+      }
+    }
+    return;
+  }
   if (KW == 2 && s.nsel) {
 #pragma unroll
     for (int i = 0; i < N; ++i) {
@@ -507,15 +529,6 @@ __global__ void __launch_bounds__(BLOCK, sweep_min_blocks(KW, D, ITEMS, BLOCK)) 
 // sum[4p+1] / sum[4p+2] = the least / greatest such digit, sum[4p+3] = 1 when a
 // non-empty segment exists. Block (p, b): its warps take segments
 // b*64 + warp, + 8, ...; a warp's lanes look at 8 bins each.
-__global__ void k_pass_summary_init(int32_t* sum, int P) {
-  for (int p = threadIdx.x; p < P; p += blockDim.x) {
-    sum[4 * p] = 1;
-    sum[4 * p + 1] = 0x7fffffff;
-    sum[4 * p + 2] = -1;
-    sum[4 * p + 3] = 0;
-  }
-}
-
 __global__ void k_pass_summary(const uint32_t* __restrict__ hist, const uint32_t* __restrict__ seg_start, int nseg,
                                int P, int R, int32_t* sum) {
   const int p = blockIdx.x;
@@ -984,12 +997,12 @@ int sort_segments_impl(const KeyJob* jobs, int njobs, uint32_t rows, const uint3
     if (kp.ntiles > max_tiles) max_tiles = kp.ntiles;
   }
 
+  constexpr size_t kCounters = 64, kSummary = 4 * 64;
   WsSize w;
-  w.add<uint32_t>(nseg + 1);
-  w.add<uint32_t>(nseg + 1);
-  w.add<uint32_t>(max_hist);
+  w.add<uint32_t>(2 * ((size_t)nseg + 1) + kSummary);  // segment and tile offsets, pass summary
+  w.add<uint32_t>(kCounters + max_hist);
   w.add<uint32_t>(max_status);
-  w.add<uint32_t>(80 + 4 * 64);
+  w.add<uint32_t>(4);
   w.add<uint32_t>((size_t)rows * max_kw);
   w.add<uint32_t>((size_t)rows * max_kw);
   w.add<uint32_t>(rows);
@@ -1005,28 +1018,29 @@ int sort_segments_impl(const KeyJob* jobs, int njobs, uint32_t rows, const uint3
 
   Workspace ws;
   YQ_TRY(ws.acquire(workspace, workspace_bytes, w.total(), s));
-  uint32_t* d_seg = ws.take<uint32_t>(nseg + 1);
-  uint32_t* d_tiles = ws.take<uint32_t>(nseg + 1);
-  uint32_t* d_hist = ws.take<uint32_t>(max_hist);
+  // What the host sends goes in one upload, what starts at zero in one memset.
+  uint32_t* d_seg = ws.take<uint32_t>(2 * ((size_t)nseg + 1) + kSummary);
+  uint32_t* d_tiles = d_seg + nseg + 1;
+  int32_t* d_sum = reinterpret_cast<int32_t*>(d_tiles + nseg + 1);  // [4 * P] pass summary
+  uint32_t* d_counters = ws.take<uint32_t>(kCounters + max_hist);   // a tile counter a pass, then the histograms
+  uint32_t* d_hist = d_counters + kCounters;
   uint32_t* d_status = ws.take<uint32_t>(max_status);
-  uint32_t* d_misc = ws.take<uint32_t>(80 + 4 * 64);  // [0..63] tile counters, [64] error, [65] text words,
-                                                       // [66..] pass summary
+  uint32_t* d_err = ws.take<uint32_t>(4);  // [0] error, [1] text words
   uint32_t* d_keys[2] = {ws.take<uint32_t>((size_t)rows * max_kw), ws.take<uint32_t>((size_t)rows * max_kw)};
   uint32_t* d_vals[2] = {ws.take<uint32_t>(rows), ws.take<uint32_t>(rows)};
   uint32_t* d_perm_tmp = ws.take<uint32_t>(rows);
   uint32_t* d_tile_seg = ws.take<uint32_t>(max_tiles + 1);
-  // tile offsets of a plan on the device, with the segment of every tile
-  auto upload_tiles = [&](const SegPlan& p) -> int {
-    YQ_TRY(h2d_async(d_tiles, p.tiles.data(), (nseg + 1) * sizeof(uint32_t), s));
+  // the segment of every tile (one segment: every tile's)
+  auto fill_tile_seg = [&](const SegPlan& p) -> int {
     if (p.ntiles > max_tiles) return YQ_ERR_UNSUPPORTED;
+    if (nseg == 1) return YQ_OK;
     const int g = nseg < 4096 ? nseg : 4096;
     k_fill_tile_seg<<<g, 256, 0, s>>>(d_tiles, nseg, d_tile_seg);
     YQ_CHECK_LAUNCH();
     return YQ_OK;
   };
-  uint32_t* d_err = d_misc + 64;
-  uint32_t* d_textw = d_misc + 65;
-  YQ_TRY_CUDA(cudaMemsetAsync(d_misc, 0, 80 * sizeof(uint32_t), s));
+  uint32_t* d_textw = d_err + 1;
+  YQ_TRY_CUDA(cudaMemsetAsync(d_err, 0, 4 * sizeof(uint32_t), s));
 
   const uint32_t* perm_in = nullptr;  // order from the less significant keys (null = identity)
   for (int jj = njobs - 1; jj >= 0; --jj) {
@@ -1070,11 +1084,15 @@ int sort_segments_impl(const KeyJob* jobs, int njobs, uint32_t rows, const uint3
     YQ_TRY(plan_key(cc, cvw, want_d, want_items, want_block, seg_offsets_host, nseg, kp, false, cnull));
     SegPlan sp;
     plan_segments(seg_offsets_host, nseg, kp.tile_rows, sp);
-    YQ_TRY(h2d_async(d_seg, sp.seg.data(), (nseg + 1) * sizeof(uint32_t), s));
-    YQ_TRY(upload_tiles(sp));
-    YQ_TRY_CUDA(cudaMemsetAsync(d_hist, 0, (size_t)nseg * kp.P * kp.R * sizeof(uint32_t), s));
-    YQ_TRY_CUDA(cudaMemsetAsync(d_status, 0, (size_t)kp.P * sp.ntiles * kp.R * sizeof(uint32_t), s));
-    YQ_TRY_CUDA(cudaMemsetAsync(d_misc, 0, 64 * sizeof(uint32_t), s));
+    if (kp.P > 64) return YQ_ERR_UNSUPPORTED;
+    std::vector<uint32_t> head(sp.seg);
+    head.insert(head.end(), sp.tiles.begin(), sp.tiles.end());
+    if (!keep_trivial)
+      for (int p = 0; p < kp.P; ++p)  // identities of k_pass_summary's four words
+        head.insert(head.end(), {1u, 0x7fffffffu, 0xffffffffu, 0u});
+    YQ_TRY(h2d_async(d_seg, head.data(), head.size() * sizeof(uint32_t), s));
+    YQ_TRY(fill_tile_seg(sp));
+    YQ_TRY_CUDA(cudaMemsetAsync(d_counters, 0, (kCounters + (size_t)nseg * kp.P * kp.R) * sizeof(uint32_t), s));
 
     KeySrc src;
     src.nsel = 0;
@@ -1091,7 +1109,7 @@ int sort_segments_impl(const KeyJob* jobs, int njobs, uint32_t rows, const uint3
     SegInfo seg;
     seg.seg_start = d_seg;
     seg.tile_start = d_tiles;
-    seg.tile_seg = d_tile_seg;
+    seg.tile_seg = nseg == 1 ? nullptr : d_tile_seg;
     seg.nseg = nseg;
     {
       // algorithmic bytes: each key read once (+ the incoming permutation)
@@ -1108,10 +1126,6 @@ int sort_segments_impl(const KeyJob* jobs, int njobs, uint32_t rows, const uint3
       // A pass whose digit is the same for every key of every segment leaves
       // the order unchanged and is skipped. common[p] = that digit when it is
       // also the same across segments, else -1.
-      if (kp.P > 64) return YQ_ERR_UNSUPPORTED;
-      int32_t* d_sum = reinterpret_cast<int32_t*>(d_misc + 66);  // [4 * P] summary words (P <= 64 here)
-      k_pass_summary_init<<<1, 64, 0, s>>>(d_sum, kp.P);
-      YQ_CHECK_LAUNCH();
       k_pass_summary<<<dim3((unsigned)kp.P, (unsigned)ceil_div(nseg, 64)), 256, 0, s>>>(d_hist, d_seg, nseg, kp.P,
                                                                                           kp.R, d_sum);
       YQ_CHECK_LAUNCH();
@@ -1182,10 +1196,10 @@ int sort_segments_impl(const KeyJob* jobs, int njobs, uint32_t rows, const uint3
     }
     if (kq.sh.kw != kp.sh.kw) {  // tiles of the narrower kernels
       plan_segments(seg_offsets_host, nseg, kq.tile_rows, sp);
-      YQ_TRY(upload_tiles(sp));
-      YQ_TRY_CUDA(cudaMemsetAsync(d_status, 0, passes.size() * sp.ntiles * kq.R * sizeof(uint32_t), s));
+      YQ_TRY(h2d_async(d_tiles, sp.tiles.data(), (nseg + 1) * sizeof(uint32_t), s));
+      YQ_TRY(fill_tile_seg(sp));
     }
-    if (passes.size() > 64) return YQ_ERR_UNSUPPORTED;
+    YQ_TRY_CUDA(cudaMemsetAsync(d_status, 0, passes.size() * sp.ntiles * kq.R * sizeof(uint32_t), s));
     uint32_t* dst_perm = (perm_in == out_perm) ? d_perm_tmp : out_perm;
     for (size_t i = 0; i < passes.size(); ++i) {
       const bool first = (i == 0), last = (i + 1 == passes.size());
@@ -1198,7 +1212,7 @@ int sort_segments_impl(const KeyJob* jobs, int njobs, uint32_t rows, const uint3
       Sp.seg = seg;
       Sp.hist = d_hist;
       Sp.status = d_status + (size_t)i * sp.ntiles * kq.R;
-      Sp.tile_counter = d_misc + i;
+      Sp.tile_counter = d_counters + i;
       Sp.err = d_err;
       Sp.pass = passes[i];
       int word = passes[i] * kq.D / 32, bit = passes[i] * kq.D % 32;
