@@ -567,19 +567,19 @@ int yq_filter_project(const yq_batch* batch, const yq_program* predicate, const 
   const uint32_t ntiles = ceil_div<uint32_t>(rows, kStepRows);
   Workspace ws;
   YQ_TRY(ws.acquire(workspace, workspace_bytes, yq_filter_project_workspace_size(rows), s));
-  unsigned long long* status = ws.take<unsigned long long>((size_t)ntiles + 1);
-  uint32_t* misc = ws.take<uint32_t>(4);  // [0] chunk counter, [1] error, [2] count
-  YQ_TRY_CUDA(cudaMemsetAsync(status, 0, ((size_t)ntiles + 1) * sizeof(unsigned long long), s));
-  YQ_TRY_CUDA(cudaMemsetAsync(misc, 0, 4 * sizeof(uint32_t), s));
-  uint32_t* cnt_dev = count_device ? count_device : misc + 2;
-  YQ_TRY(launch_filter_project(F, rows, misc, status, cnt_dev, s));
+  // [chunk counter, error, count, -], then the status words: one memset, one read-back
+  uint32_t* misc = reinterpret_cast<uint32_t*>(ws.take<unsigned long long>((size_t)ntiles + 3));
+  unsigned long long* status = reinterpret_cast<unsigned long long*>(misc + 4);
+  YQ_TRY_CUDA(cudaMemsetAsync(misc, 0, ((size_t)ntiles + 3) * sizeof(unsigned long long), s));
+  YQ_TRY(launch_filter_project(F, rows, misc, status, misc + 2, s));
+  if (count_device)
+    YQ_TRY_CUDA(cudaMemcpyAsync(count_device, misc + 2, sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
   if (count_host) {
-    uint32_t h[2];
-    YQ_TRY(d2h_sync(&h[0], cnt_dev, sizeof(uint32_t), s));
-    YQ_TRY(d2h_sync(&h[1], misc + 1, sizeof(uint32_t), s));
-    *count_host = h[0];
+    uint32_t h[4];
+    YQ_TRY(d2h_sync(h, misc, sizeof(h), s));
+    *count_host = h[2];
     if (h[1] & kErrTimeout) return YQ_ERR_TIMEOUT;
-    if (h[0] > capacity) return YQ_ERR_CAPACITY;
+    if (h[2] > capacity) return YQ_ERR_CAPACITY;
   }
   return YQ_OK;
 }
