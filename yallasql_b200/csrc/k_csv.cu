@@ -156,20 +156,24 @@ __device__ Summ thread_summary(const uint8_t* data, uint64_t nbytes, uint64_t lo
 
 // A tile of whole 64-byte chunks without a quote (most tiles of most files)
 // needs no tokenizer maps: outside quotes a record starts where a newline is
-// followed by something else, so a thread's record starts are a count that
-// depends on the byte before its chunk alone, and the block adds integers where
-// the general path composes five-state summaries (0.5K instructions a warp: the
-// two index kernels took 80 + 120 us on 104 MB of text, now 27 + 39 us).
-// Returns this thread's starts (thread 0's as if the tile began inside a
-// record); every thread of the block calls it.
-__device__ __forceinline__ uint32_t quote_free_starts(const Chunk64& k, uint32_t* s_last) {
+// followed by something else, so a chunk's record starts are a bitmask that
+// depends on the byte before it alone, and the block adds integers where the
+// general path composes five-state summaries (0.5K instructions a warp). The
+// masks are kept (an eighth of the text) for the emit kernel, which then reads
+// them instead of scanning the text again: 80 + 120 us for 104 MB of text by
+// summaries, 45 + 59 by integers, 45 + 33 with the masks kept.
+// Returns this thread's mask (thread 0's bit 0: a start if the tile begins
+// after a newline); every thread of the block calls it.
+__device__ __forceinline__ uint64_t quote_free_mask(const Chunk64& k, uint32_t* s_last) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t prev = __shfl_up_sync(0xffffffffu, k.cl, 1);
   if (lane == 31) s_last[warp] = k.cl;
   __syncthreads();
-  if (lane == 0) prev = warp ? s_last[warp - 1] : (uint32_t)C_OTHER;
-  return (uint32_t)popc64(~k.nl & (k.nl << 1)) + (prev == C_NL && k.c0 != C_NL ? 1u : 0u);
+  if (lane == 0) prev = warp ? s_last[warp - 1] : (uint32_t)C_NL;
+  return (~k.nl & (k.nl << 1)) | (prev == C_NL && k.c0 != C_NL ? 1ull : 0ull);
 }
+// Above a tile's state map (15 bits): no quote in it, its first byte is ordinary.
+constexpr uint32_t kTilePlain = 1u << 31, kTileFirstOther = 1u << 30;
 
 // Loads and scans this thread's chunk when the whole tile is aligned text (the
 // same answer for every thread of the block); *plain: the tile has no quote.
@@ -185,7 +189,8 @@ __device__ __forceinline__ bool whole_tile(const uint8_t* data, uint64_t nbytes,
 
 __global__ void __launch_bounds__(kTileThreads) k_csv_tiles(const uint8_t* __restrict__ data, uint64_t nbytes,
                                                             int aligned, uint32_t* __restrict__ tile_map,
-                                                            uint32_t* __restrict__ tile_cnt) {
+                                                            uint32_t* __restrict__ tile_cnt,
+                                                            uint64_t* __restrict__ masks) {
   __shared__ uint64_t s_step[NMAPS * 4];
   __shared__ uint32_t s_mapw[NMAPS];
   __shared__ Summ s_warp[kTileThreads / 32];
@@ -198,7 +203,10 @@ __global__ void __launch_bounds__(kTileThreads) k_csv_tiles(const uint8_t* __res
   bool plain;
   whole_tile(data, nbytes, tile, aligned, w, k, &plain);
   if (plain) {
-    const uint32_t sum = __reduce_add_sync(0xffffffffu, quote_free_starts(k, s_last));
+    const uint64_t m = quote_free_mask(k, s_last);
+    masks[tile * kTileThreads + threadIdx.x] = m;
+    // thread 0's bit 0 depends on what came before the tile: counted below
+    const uint32_t sum = __reduce_add_sync(0xffffffffu, (uint32_t)popc64(threadIdx.x == 0 ? m & ~1ull : m));
     if ((threadIdx.x & 31) == 0) s_sum[threadIdx.x >> 5] = sum;
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -209,7 +217,7 @@ __global__ void __launch_bounds__(kTileThreads) k_csv_tiles(const uint8_t* __res
       whole.nl = 0;
       whole.cl = s_last[kTileThreads / 32 - 1];
       const Summ t = summary_quote_free(whole);
-      tile_map[tile] = t.map;
+      tile_map[tile] = t.map | kTilePlain | (k.c0 == C_OTHER ? kTileFirstOther : 0u);
       const bool in_quotes[NSTATES] = {false, false, true, k.c0 == C_OTHER, false};
 #pragma unroll
       for (int s = 0; s < NSTATES; ++s) tile_cnt[tile * NSTATES + s] = in_quotes[s] ? 0u : t.c[s] + n;
@@ -259,40 +267,30 @@ __global__ void __launch_bounds__(kScanThreads) k_csv_tile_scan(const uint32_t* 
 }
 
 __global__ void __launch_bounds__(kTileThreads) k_csv_emit(const uint8_t* __restrict__ data, uint64_t nbytes,
-                                                           int aligned,
+                                                           int aligned, const uint32_t* __restrict__ tile_map,
+                                                           const uint64_t* __restrict__ masks,
                                                            const unsigned long long* __restrict__ tile_start,
                                                            uint32_t* __restrict__ starts) {
   __shared__ uint64_t s_step[NMAPS * 4];
   __shared__ uint32_t s_mapw[NMAPS];
   __shared__ Summ s_warp[kTileThreads / 32];
-  __shared__ uint32_t s_last[kTileThreads / 32], s_sum[kTileThreads / 32 + 1];
   const uint64_t tile = blockIdx.x;
   const uint64_t lo = tile * kTileBytes + (uint64_t)threadIdx.x * kBytesPerThread;
-  uint32_t w[16];
-  Chunk64 k;
-  bool plain;
-  const bool whole = whole_tile(data, nbytes, tile, aligned, w, k, &plain);
-  if (plain) {
+  const uint32_t flags = __ldg(tile_map + tile);
+  if (flags & kTilePlain) {
+    __shared__ uint32_t s_sum[kTileThreads / 32 + 1];
+    uint64_t m = __ldg(masks + tile * kTileThreads + threadIdx.x);
     const unsigned long long ts = __ldg(tile_start + tile);
     const uint32_t tstate = (uint32_t)(ts >> 32);
-    uint32_t n = quote_free_starts(k, s_last);
-    uint64_t m = ~k.nl & (k.nl << 1);
-    if (threadIdx.x == 0) {
-      m = starts_quote_free(k, tstate);
-      n = (uint32_t)popc64(m);
-    } else if (n != (uint32_t)popc64(m)) {
-      m |= 1;  // the byte before this chunk is a newline
-    }
+    if (tstate == S_QUO || (tstate == S_QQ && (flags & kTileFirstOther))) return;  // entered inside quotes: no start
+    if (threadIdx.x == 0 && tstate != S_REC) m &= ~1ull;
     uint32_t total;
-    uint32_t idx = (uint32_t)ts + block_exclusive_sum<kTileThreads>(n, s_sum, total);
-    // a tile entered inside quotes holds no start (thread 0 saw the state and the first byte)
-    __shared__ uint32_t s_quoted;
-    if (threadIdx.x == 0) s_quoted = tstate == S_QUO || (tstate == S_QQ && k.c0 == C_OTHER);
-    __syncthreads();
-    if (s_quoted) return;
+    uint32_t idx = (uint32_t)ts + block_exclusive_sum<kTileThreads>((uint32_t)popc64(m), s_sum, total);
     for (; m; m &= m - 1) starts[idx++] = (uint32_t)(lo + __ffsll(m) - 1);
     return;
   }
+  uint32_t w[16];
+  Chunk64 k;
   load_tables(s_step, s_mapw);
   Summ mine = lo < nbytes ? thread_summary(data, nbytes, lo, aligned != 0, s_step, s_mapw) : identity_summ();
   Summ excl = block_exclusive<kTileThreads>(mine, s_warp, nullptr);
@@ -303,10 +301,8 @@ __global__ void __launch_bounds__(kTileThreads) k_csv_emit(const uint8_t* __rest
   uint32_t idx = (uint32_t)ts + excl.c[tstate];
   const uint64_t hi = lo + kBytesPerThread < nbytes ? lo + kBytesPerThread : nbytes;
   if (aligned && hi - lo == kBytesPerThread) {
-    if (!whole) {  // the last tile: its whole chunks are read here
-      load64(data + lo, w);
-      k = scan64(w);
-    }
+    load64(data + lo, w);  // a second read of the same 64 bytes: an L1 hit
+    k = scan64(w);
     if (!k.quotes) {
       for (uint64_t m = starts_quote_free(k, state); m; m &= m - 1) starts[idx++] = (uint32_t)(lo + __ffsll(m) - 1);
       return;
@@ -543,6 +539,7 @@ size_t yq_csv_index_workspace_size(uint64_t nbytes) {
   w.add<uint32_t>(nt * NSTATES);
   w.add<unsigned long long>(nt);
   w.add<unsigned long long>(2);
+  w.add<uint64_t>(nt * kTileThreads);
   return w.total();
 }
 
@@ -560,10 +557,11 @@ int yq_csv_index(const uint8_t* data, uint64_t nbytes, uint32_t* record_starts, 
   uint32_t* tile_cnt = ws.take<uint32_t>(((size_t)nt + 1) * NSTATES);
   unsigned long long* tile_start = ws.take<unsigned long long>((size_t)nt + 1);
   unsigned long long* total = ws.take<unsigned long long>(2);
+  uint64_t* masks = ws.take<uint64_t>(((size_t)nt + 1) * kTileThreads);
   const int aligned = (reinterpret_cast<uintptr_t>(data) & 15) == 0;
   {
     ProfScope ps("csv_tiles", s, (double)nbytes);
-    k_csv_tiles<<<nt, kTileThreads, 0, s>>>(data, nbytes, aligned, tile_map, tile_cnt);
+    k_csv_tiles<<<nt, kTileThreads, 0, s>>>(data, nbytes, aligned, tile_map, tile_cnt, masks);
     YQ_CHECK_LAUNCH();
   }
   {
@@ -578,7 +576,7 @@ int yq_csv_index(const uint8_t* data, uint64_t nbytes, uint32_t* record_starts, 
   if (!record_starts) return h ? YQ_ERR_INVALID_ARG : YQ_OK;
   {
     ProfScope ps("csv_emit", s, (double)nbytes + 4.0 * (double)h);
-    k_csv_emit<<<nt, kTileThreads, 0, s>>>(data, nbytes, aligned, tile_start, record_starts);
+    k_csv_emit<<<nt, kTileThreads, 0, s>>>(data, nbytes, aligned, tile_map, masks, tile_start, record_starts);
     YQ_CHECK_LAUNCH();
   }
   return YQ_OK;
