@@ -387,21 +387,22 @@ __global__ void __launch_bounds__(kJoinBlock) k_join_hash(const __grid_constant_
 // --------------------------------------- equality probing, long right sides
 // A right side too long for a shared-memory table is sorted once by its key
 // (the stable radix sort, so rows of one key are contiguous and ascending) and
-// a hash table in global memory maps each distinct key to its first sorted
-// position. A probe costs three dependent reads that L2 serves (slot, key,
-// next key) whatever the right side's length, and a key's repeats are a
-// contiguous run, so the outputs of a tile are written position by position
-// by all its threads (coalesced, and one left row with many matches does not
-// serialise a thread). The nested loop this replaces compares every pair:
-// 2M x 300K INT32 rows took 303 ms, this takes 0.3 ms.
+// a hash table in global memory maps each distinct key to its run. A slot holds
+// key, run and, for a key that does not repeat, the right row itself, so such a
+// probe is one 16-byte read (2M rows to 300K: 122 us with separate arrays of
+// slots, keys and rows, 104 so). A key's repeats
+// are a contiguous run, so the outputs of a tile are written position by
+// position by all its threads (coalesced, and one left row with many matches
+// does not serialise a thread). The nested loop this replaces compares every
+// pair: 2M x 300K INT32 rows took 303 ms.
 struct SortedJoin {
-  const uint32_t* perm;           // right rows in key order
-  unsigned long long* skey;       // key of every sorted position
-  uint32_t* slots;                // hash table: first sorted position of a key (kNoSlot: empty)
-  uint32_t* nvalid;               // sorted positions before the NaN and NULL keys (they never join)
-  uint32_t nslots;                // power of two, >= 2 R
+  const uint32_t* perm;  // right rows in key order
+  uint4* slots;          // {key, first sorted position (kNoSlot: empty), run}
+  uint32_t nslots;       // power of two, >= 1.5 R
+  uint32_t rows;         // R
 };
 constexpr uint32_t kNoSlot = 0xffffffffu;
+constexpr uint32_t kOneRow = 0x80000000u;  // run field: the key's only row (row ids are below 2^30)
 constexpr uint32_t kSortedMinRows = 1024;  // right rows from which a sorted table may be chosen, and from
 constexpr uint32_t kTableRows = 4096;      // which it always is
 
@@ -415,46 +416,79 @@ __device__ __forceinline__ bool key_joins(const JCol& c, uint32_t row) {
 __global__ void __launch_bounds__(256) k_join_sorted_build(const __grid_constant__ SortedJoin S, const JCol key,
                                                            uint32_t R, const uint32_t* sort_err, uint32_t* err) {
   if (blockIdx.x == 0 && threadIdx.x == 0 && *sort_err) atomicOr(err, *sort_err);
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < R; i += gridDim.x * blockDim.x) {
+  auto row_at = [&](uint32_t i) {
     const uint32_t row = __ldg(S.perm + i);
-    if (row >= R) {  // a failed sort left no permutation
-      atomicOr(err, kErrBounds);
-      continue;
-    }
-    const uint64_t k = hash_key(key, row);
-    S.skey[i] = k;
+    if (row >= R) atomicOr(err, kErrBounds);  // a failed sort left no permutation
+    return min(row, R - 1u);
+  };
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < R; i += gridDim.x * blockDim.x) {
+    const uint32_t row = row_at(i);
     if (!key_joins(key, row)) continue;
-    if (i + 1 == R || !key_joins(key, min(__ldg(S.perm + i + 1), R - 1u))) *S.nvalid = i + 1;
-    if (i > 0 && hash_key(key, min(__ldg(S.perm + i - 1), R - 1u)) == k) continue;
+    const uint64_t k = hash_key(key, row);
+    auto same = [&](uint32_t j) {
+      const uint32_t r = row_at(j);
+      return key_joins(key, r) && hash_key(key, r) == k;
+    };
+    if (i > 0 && same(i - 1)) continue;
+    uint32_t step = 1;  // run end: doubling steps, then a binary search inside the last one
+    while (step < R - i && same(i + step)) step <<= 1;
+    uint32_t lo = i + (step >> 1), hi = step < R - i ? i + step : R;  // key at lo matches; hi is past the run
+    while (lo + 1 < hi) {
+      const uint32_t mid = lo + ((hi - lo) >> 1);
+      if (same(mid)) lo = mid;
+      else hi = mid;
+    }
+    const uint32_t run = lo + 1u - i;
     uint32_t h = hash_bucket(k, S.nslots);  // keys are distinct here: the first empty slot is this key's
-    for (uint32_t n = 0; n < S.nslots; ++n, h = (h + 1u) & (S.nslots - 1u))
-      if (atomicCAS(S.slots + h, kNoSlot, i) == kNoSlot) break;
+    for (uint32_t n = 0; n < S.nslots; ++n, h = (h + 1u) & (S.nslots - 1u)) {
+      uint32_t* slot = reinterpret_cast<uint32_t*>(S.slots + h);
+      if (atomicCAS(slot + 2, kNoSlot, i) != kNoSlot) continue;
+      slot[0] = (uint32_t)k;
+      slot[1] = (uint32_t)(k >> 32);
+      slot[3] = run == 1u ? kOneRow | row : run;
+      break;
+    }
   }
 }
 
-// First sorted position and run length of the keys equal to left row l's.
-__device__ __forceinline__ uint32_t sorted_matches(const SortedJoin& S, uint32_t nvalid, const JCol& key, uint32_t l,
-                                                   uint32_t& first) {
-  first = 0;
-  if (!key_joins(key, l)) return 0u;
-  const uint64_t k = hash_key(key, l);
-  uint32_t h = hash_bucket(k, S.nslots);
-  uint32_t p = kNoSlot;
-  for (uint32_t n = 0; n < S.nslots; ++n, h = (h + 1u) & (S.nslots - 1u)) {
-    p = __ldg(S.slots + h);
-    if (p == kNoSlot || __ldg(S.skey + p) == k) break;
+// Matches of a thread's kJoinItems consecutive left rows: the number of rows of
+// each one's key, and where they are (a sorted position, or kOneRow and the
+// row). The first probe of every row goes out before any is looked at.
+__device__ __forceinline__ void sorted_matches(const SortedJoin& S, const JCol& key, uint32_t l0, uint32_t L,
+                                               uint32_t (&where)[kJoinItems], uint32_t (&run)[kJoinItems]) {
+  uint64_t k[kJoinItems];
+  uint32_t h[kJoinItems], joins = 0u;
+  uint4 at[kJoinItems];
+#pragma unroll
+  for (int i = 0; i < kJoinItems; ++i) {
+    const uint32_t l = l0 + i < L ? l0 + i : L - 1u;
+    if (l0 + i < L && key_joins(key, l)) joins |= 1u << i;
+    k[i] = hash_key(key, l);
   }
-  if (p == kNoSlot || p >= nvalid) return 0u;
-  first = p;
-  uint32_t step = 1;  // run end: doubling steps, then a binary search inside the last one
-  while (p + step < nvalid && __ldg(S.skey + p + step) == k) step <<= 1;
-  uint32_t lo = p + (step >> 1), hi = min(p + step, nvalid);  // key at lo matches; hi is past the run
-  while (lo + 1 < hi) {
-    const uint32_t mid = lo + ((hi - lo) >> 1);
-    if (__ldg(S.skey + mid) == k) lo = mid;
-    else hi = mid;
+#pragma unroll
+  for (int i = 0; i < kJoinItems; ++i) {
+    h[i] = hash_bucket(k[i], S.nslots);
+    at[i] = __ldg(S.slots + h[i]);
   }
-  return lo + 1u - p;
+#pragma unroll
+  for (int i = 0; i < kJoinItems; ++i) {
+    where[i] = run[i] = 0u;
+    if (!(joins >> i & 1u)) continue;
+    auto mine = [&](const uint4& e) { return e.x == (uint32_t)k[i] && e.y == (uint32_t)(k[i] >> 32); };
+    for (uint32_t n = 1; n < S.nslots && at[i].z != kNoSlot && !mine(at[i]); ++n) {
+      h[i] = (h[i] + 1u) & (S.nslots - 1u);
+      at[i] = __ldg(S.slots + h[i]);
+    }
+    if (at[i].z == kNoSlot || !mine(at[i])) continue;
+    run[i] = (at[i].w & kOneRow) ? 1u : at[i].w;
+    where[i] = (at[i].w & kOneRow) ? at[i].w : at[i].z;
+  }
+}
+
+// Right row of match x of a key at `where` (a failed sort, which the error word
+// reports, must not send the reads out of range).
+__device__ __forceinline__ uint32_t match_row(const SortedJoin& S, uint32_t where, uint32_t x) {
+  return (where & kOneRow) ? where & ~kOneRow : min(__ldg(S.perm + where + x), S.rows - 1u);
 }
 
 __device__ __forceinline__ void write_col(const JOut& w, unsigned long long pos, uint32_t row) {
@@ -480,31 +514,26 @@ __global__ void __launch_bounds__(kJoinBlock) k_join_sorted(const __grid_constan
   __syncthreads();
   const uint32_t tile = s_tile;
   const uint32_t base = tile * kJoinTile;
-  const uint32_t nvalid = *S.nvalid;
   const JCond& ec = J.cond[J.eq];
   const int lane = threadIdx.x & 31;
   uint32_t first[kJoinItems], run[kJoinItems], cnt[kJoinItems], sum = 0;
+  sorted_matches(S, ec.l, base + threadIdx.x * kJoinItems, J.L, first, run);
 #pragma unroll
-  for (int k = 0; k < kJoinItems; ++k) {
-    const uint32_t l = base + threadIdx.x * kJoinItems + k;
-    first[k] = 0;
-    run[k] = l < J.L ? sorted_matches(S, nvalid, ec.l, l, first[k]) : 0u;
-    cnt[k] = run[k];
-  }
+  for (int k = 0; k < kJoinItems; ++k) cnt[k] = run[k];
   if constexpr (!EQ_ONLY) {
 #pragma unroll 1
     for (int k = 0; k < kJoinItems; ++k) {
       const uint32_t l = base + threadIdx.x * kJoinItems + k;
       cnt[k] = 0;
       if (run[k] <= 32)
-        for (uint32_t x = 0; x < run[k]; ++x) cnt[k] += all_conds(J, l, __ldg(S.perm + first[k] + x), J.eq) ? 1u : 0u;
+        for (uint32_t x = 0; x < run[k]; ++x) cnt[k] += all_conds(J, l, match_row(S, first[k], x), J.eq) ? 1u : 0u;
       for (uint32_t todo = __ballot_sync(0xffffffffu, run[k] > 32); todo; todo &= todo - 1) {
         const int src = __ffs(todo) - 1;
         const uint32_t n = __shfl_sync(0xffffffffu, run[k], src), f = __shfl_sync(0xffffffffu, first[k], src);
         const uint32_t wl = __shfl_sync(0xffffffffu, l, src);
         uint32_t c = 0;
         for (uint32_t x = lane; x < ((n + 31u) & ~31u); x += 32) {
-          const bool m = x < n && all_conds(J, wl, __ldg(S.perm + f + x), J.eq);
+          const bool m = x < n && all_conds(J, wl, match_row(S, f, x), J.eq);
           c += __popc(__ballot_sync(0xffffffffu, m));
         }
         if (lane == src) cnt[k] = c;
@@ -560,7 +589,7 @@ __global__ void __launch_bounds__(kJoinBlock) k_join_sorted(const __grid_constan
           else hi = mid;
         }
         s_l[i] = base + lo;
-        s_r[i] = __ldg(S.perm + s_first[lo] + (c0 + i - s_off[lo]));
+        s_r[i] = match_row(S, s_first[lo], c0 + i - s_off[lo]);
       }
       __syncthreads();
       const unsigned long long p0 = prefix + c0;
@@ -585,7 +614,7 @@ __global__ void __launch_bounds__(kJoinBlock) k_join_sorted(const __grid_constan
     const uint32_t l = base + threadIdx.x * kJoinItems + k;
     if (run[k] <= 32) {
       for (uint32_t x = 0; x < run[k]; ++x) {
-        const uint32_t r = __ldg(S.perm + first[k] + x);
+        const uint32_t r = match_row(S, first[k], x);
         if (EQ_ONLY || all_conds(J, l, r, J.eq)) emit_pair(J, pos++, l, r);
       }
     }
@@ -595,7 +624,7 @@ __global__ void __launch_bounds__(kJoinBlock) k_join_sorted(const __grid_constan
       const uint32_t wl = __shfl_sync(0xffffffffu, l, src);
       unsigned long long wp = __shfl_sync(0xffffffffu, pos, src);
       for (uint32_t x = lane; x < ((n + 31u) & ~31u); x += 32) {
-        const uint32_t r = x < n ? __ldg(S.perm + f + x) : 0u;
+        const uint32_t r = x < n ? match_row(S, f, x) : 0u;
         const bool m = x < n && (EQ_ONLY || all_conds(J, wl, r, J.eq));
         const uint32_t bal = __ballot_sync(0xffffffffu, m);
         if (m) emit_pair(J, wp + __popc(bal & lanemask_lt()), wl, r);
@@ -1075,12 +1104,13 @@ static void count_ws_layout(uint32_t L, uint32_t R, size_t sort_bytes, WsSize& w
   w.add<uint32_t>(L ? L : 1);
 }
 
+// Slots of the sorted join's table: a load of 0.33 to 0.67.
+static uint32_t sorted_slots(uint32_t R) { return pow2_at_least(R + R / 2); }
+
 static void sorted_ws_layout(uint32_t R, size_t sort_bytes, WsSize& w) {
   w.add<char>(sort_bytes);
   w.add<uint32_t>(R);
-  w.add<unsigned long long>(R);
-  w.add<uint32_t>(4);
-  w.add<uint32_t>((size_t)pow2_at_least(R) * 2);
+  w.add<uint4>(sorted_slots(R));
 }
 
 template <typename T>
@@ -1264,18 +1294,20 @@ static int join_impl(const yq_batch* left, const yq_batch* right, const yq_join_
     uint32_t* perm = ws.take<uint32_t>(J.R);
     SortedJoin S;
     S.perm = perm;
-    S.skey = ws.take<unsigned long long>(J.R);
-    S.nvalid = ws.take<uint32_t>(4);
-    S.nslots = pow2_at_least(J.R) * 2u;
-    S.slots = ws.take<uint32_t>(S.nslots);
+    S.rows = J.R;
+    S.nslots = sorted_slots(J.R);
+    S.slots = ws.take<uint4>(S.nslots);
     const yq_column rc{const_cast<char*>(ec.r.data), ec.r.nulls, ec.r.type, ec.r.width};
     KeyJob j{rc, 0, 0};
     uint32_t offs[2] = {0, J.R};
     uint32_t* sort_err = nullptr;
-    YQ_TRY(sort_segments_impl(&j, 1, J.R, offs, 1, perm, nullptr, sort_ws, eq_sort_bytes, s, nullptr, nullptr, nullptr,
-                              true, &sort_err));
-    YQ_TRY_CUDA(cudaMemsetAsync(S.nvalid, 0, 4 * sizeof(uint32_t), s));
-    YQ_TRY_CUDA(cudaMemsetAsync(S.slots, 0xff, (size_t)S.nslots * sizeof(uint32_t), s));
+    // A 4-byte key keeps all four passes rather than wait for the host to learn
+    // which of them change nothing (13 us a pass against some 20 for the wait).
+    const yq_sort_config keep{0, 0, 0, 1};
+    const bool no_wait = ec.r.width == 4 && !ec.r.nulls;
+    YQ_TRY(sort_segments_impl(&j, 1, J.R, offs, 1, perm, no_wait ? &keep : nullptr, sort_ws, eq_sort_bytes, s, nullptr,
+                              nullptr, nullptr, true, &sort_err));
+    YQ_TRY_CUDA(cudaMemsetAsync(S.slots, 0xff, (size_t)S.nslots * sizeof(uint4), s));
     int grid = (int)ceil_div<uint32_t>(J.R, 256);
     if (grid > sm_count() * 8) grid = sm_count() * 8;
     {
