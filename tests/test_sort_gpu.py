@@ -178,9 +178,10 @@ def test_nullable_wide_keys(cuda, words, nulls_first, n):
 
 @pytest.mark.parametrize("n", [2_000_003, 3_000_001])
 def test_gather_of_large_tables(cuda, n):
-    """Tables around and above the packed-row threshold: every cell width the
-    records hold, null bytes on both or one side, a wide text column that moves
-    by itself, and a permutation that is not one (its bad rows are skipped)."""
+    """Tables around and above the packed-row threshold, by a permutation and by
+    the ORDER BY of its inverse (through packed rows): every cell width the
+    records hold, null bytes, a wide text column that moves by itself, and a
+    permutation that is not one (its bad rows are skipped)."""
     rng = np.random.default_rng(n)
     g = torch.Generator(device="cuda")
     g.manual_seed(n)
@@ -197,6 +198,13 @@ def test_gather_of_large_tables(cuda, n):
         assert torch.equal(o.data.view(torch.uint8), c.data[idx].view(torch.uint8))
         if c.nulls is not None:
             assert torch.equal(o.nulls, c.nulls[idx])
+    inverse = torch.empty_like(perm)
+    inverse[idx] = torch.arange(n, device="cuda", dtype=torch.int32)
+    ordered = ops.order_by(ops.DeviceBatch([ops.DeviceColumn(inverse, A.INT32)] + cols), 0, False, [0, n])
+    for o, w in zip(ordered.columns[1:], out.columns):
+        assert torch.equal(o.data.view(torch.uint8), w.data.view(torch.uint8))
+        if w.nulls is not None:
+            assert torch.equal(o.nulls, w.nulls)
     bad = perm.clone()
     bad[5], bad[n - 1] = n, -1
     for o in out.columns:

@@ -1254,7 +1254,7 @@ int sort_segments_impl(const KeyJob* jobs, int njobs, uint32_t rows, const uint3
 
 // Gather used by yq_gather and yq_order_by (see yq_sort.cuh).
 int gather_impl(const yq_column* in, int32_t ncols, const uint32_t* perm, uint32_t rows, const yq_column* out,
-                const uint32_t* const* only_if, cudaStream_t s, void* records, size_t record_bytes, bool may_alloc) {
+                const uint32_t* const* only_if, cudaStream_t s, void* records, size_t record_bytes) {
   if (ncols < 0 || ncols > YQ_MAX_BATCH_COLUMNS || (ncols > 0 && (!in || !out)) || (rows > 0 && !perm))
     return YQ_ERR_INVALID_ARG;
   if (rows == 0 || ncols == 0) return YQ_OK;
@@ -1263,17 +1263,9 @@ int gather_impl(const yq_column* in, int32_t ncols, const uint32_t* perm, uint32
     if (in[c].width != 1 && in[c].width % 4 != 0) return YQ_ERR_INVALID_ARG;
   }
   uint32_t moved = 0;
-  if (const size_t need = packed_gather_bytes(in, ncols, out, only_if, rows)) {
-    Workspace ws;
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    YQ_TRY_CUDA(cudaStreamIsCapturing(s, &cap));
-    if (records ? record_bytes < need
-                : !may_alloc || cap != cudaStreamCaptureStatusNone || need > pool_kept_bytes()) {
-      records = nullptr;
-    } else if (!records && ws.acquire(nullptr, 0, need, s) == YQ_OK) {  // no memory: column by column
-      records = ws.base;
-    }
-    if (records) YQ_TRY(packed_gather(in, ncols, out, only_if, perm, rows, records, s, &moved));
+  if (records) {
+    const size_t need = packed_gather_bytes(in, ncols, out, only_if, rows);
+    if (need && record_bytes >= need) YQ_TRY(packed_gather(in, ncols, out, only_if, perm, rows, records, s, &moved));
   }
   GatherParams G;
   memset(&G, 0, sizeof(G));
@@ -1431,7 +1423,7 @@ int yq_sort_autotune(const yq_column* key, uint32_t rows, const uint32_t* seg_of
 }
 
 int yq_gather(const yq_column* in, int32_t ncols, const uint32_t* perm, uint32_t rows, yq_column* out, void* stream) {
-  return gather_impl(in, ncols, perm, rows, out, nullptr, as_stream(stream), nullptr, 0, true);
+  return gather_impl(in, ncols, perm, rows, out, nullptr, as_stream(stream));
 }
 
 }  // extern "C"

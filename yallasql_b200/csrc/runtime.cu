@@ -188,18 +188,6 @@ cudaMemPool_t workspace_pool(int dev) {
 }
 }  // namespace
 
-size_t pool_kept_bytes() {
-  int dev = 0;
-  uint64_t keep = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
-  cudaMemPool_t pool = workspace_pool(dev);
-  if (!pool || cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
-    cudaGetLastError();
-    return 0;
-  }
-  return (size_t)keep;
-}
-
 int pool_alloc(void** p, size_t bytes, cudaStream_t s) {
   int dev = 0;
   YQ_TRY_CUDA(cudaGetDevice(&dev));

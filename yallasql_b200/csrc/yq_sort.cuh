@@ -33,17 +33,15 @@ int sort_segments_impl(const KeyJob* jobs, int njobs, uint32_t rows, const uint3
                        cudaStream_t s, size_t* size_only, uint32_t* keys_out = nullptr, int* kw_out = nullptr,
                        bool defer_err = false, uint32_t** err_out = nullptr, uint32_t* high_out = nullptr);
 
-// Bytes the workspace pool keeps between calls (runtime.cu): an allocation
-// beyond it is mapped anew each call, some 13 ms a GB.
-size_t pool_kept_bytes();
-
 // out[c][i] = in[c][perm[i]] for every column (yq_gather); with `only_if`,
 // column c moves only when only_if[c] is null or *only_if[c] != 0 on the device.
 // Large tables move through packed rows (k_pack.cu) when `records` holds
-// packed_gather_bytes() or, with `may_alloc`, the workspace pool does.
+// packed_gather_bytes(); yq_gather has no workspace and stays column by column
+// (several streams gathering at once would each map 32 bytes a row anew, 13 ms
+// a GB, beyond what the workspace pool keeps: the serving loop's shared ORDER BY
+// permutations lost half their rate so).
 int gather_impl(const yq_column* in, int32_t ncols, const uint32_t* perm, uint32_t rows, const yq_column* out,
-                const uint32_t* const* only_if, cudaStream_t s, void* records = nullptr, size_t record_bytes = 0,
-                bool may_alloc = false);
+                const uint32_t* const* only_if, cudaStream_t s, void* records = nullptr, size_t record_bytes = 0);
 
 // Packed-row gather (k_pack.cu): bytes of records it needs for these columns,
 // 0 where it does not apply or a column-by-column gather is the faster one;
