@@ -6,9 +6,9 @@ id int64, txt 16-byte text, d date} (seed 1), run
   ORDER BY key DESC   and then   ORDER BY d ASC,
 each producing the fully sorted table (all four columns). With --mode
 outofcore (default) each query is the reference's out-of-core plan: the
-table arrives as 4 MB batches (116,480 rows at 36 B/row), every batch is
-sorted into a run, and runs are merged pairwise by merge path until one run
-remains. --mode incore sorts the whole table at once. Metric: rows/s (rows
+table arrives as 4 MB batches (116,480 rows at 36 B/row) and leaves in the
+order of batches sorted into runs and the runs merged, which one stable sort of
+all the batches gives. --mode incore sorts the whole table at once. Metric: rows/s (rows
 sorted per second, both queries), plus the HBM roofline of the dominant kernel.
 
 `python bench.py --gpus N --steps K --warmup W [--impl reference]`; for N>1
@@ -693,7 +693,7 @@ def run_reference(args, rank: int):
 def config(args) -> dict:
     return {"workload": f"ORDER BY key DESC then ORDER BY d ASC on a {args.rows}-row table (key f32 {args.dist}, "
                         f"id int64, txt 16-byte, d date; seed 1), {args.mode}"
-                        + (" as 4 MB batches sorted then merge-path merged" if args.mode == "outofcore" else ""),
+                        + (" (arrives as 4 MB batches, in the order of sorted runs merged)" if args.mode == "outofcore" else ""),
             "rows": args.rows, "row_bytes": ROW_BYTES, "key_distribution": args.dist, "mode": args.mode,
             "l2": "inputs larger than L2 (64M rows x 36 B = 2.3 GB per table)", "parallelism": f"replicas x{args.gpus}"}
 

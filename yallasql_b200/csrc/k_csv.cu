@@ -9,11 +9,12 @@
 //   k_csv_tiles     each 16 KiB tile -> the state map of the tokenizer over it
 //                   and its record-start counts per start state (64 bytes a
 //                   thread, one shared-memory table lookup per byte, a word of
-//                   four ordinary bytes in one lookup)
+//                   four ordinary bytes in one lookup); a tile without quotes
+//                   keeps a bitmask of its record starts instead
 //   k_csv_tile_scan one block composes the tile maps in order: the tokenizer
 //                   state and the first record index at every tile
-//   k_csv_emit      each tile again, now from its known state: byte offset of
-//                   every record start
+//   k_csv_emit      each tile's masks, or its text again, now from its known
+//                   state: byte offset of every record start
 //   k_csv_parse     128 records a block: their bytes staged into shared memory
 //                   with 16-byte loads; one thread per record, the lanes of a
 //                   warp on the same field at a time, so each conversion runs

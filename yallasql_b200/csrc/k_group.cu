@@ -481,7 +481,7 @@ __global__ void __launch_bounds__(kGroupThreads) k_group_span(const __grid_const
 
 // ------------------------------------------------------- few distinct keys
 // With few groups the sort, its permutation and the reads through it are most
-// of the work (32M rows, 11 groups, five aggregates: 1.63 ms of kernels for
+// of the work (32M rows, 11 groups, five aggregates: 1.63 ms of kernels, 0.25 ms here, for
 // 384 MB of input). Here the input is read once to find the keys and once to
 // accumulate. Each thread owns an accumulator per group and aggregate in
 // shared memory (element [group][thread], so a warp's 32 updates hit 32
