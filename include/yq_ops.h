@@ -680,6 +680,9 @@ int yq_csv_parse(const uint8_t* data, uint64_t nbytes, const uint32_t* record_st
                  yq_csv_error* error, void* workspace, size_t workspace_bytes, void* stream);
 
 size_t yq_csv_format_workspace_size(uint32_t rows);
+/* Bytes that hold the text of any rows of this batch's size and types (its
+ * `rows` times the longest possible line); 0 for a batch yq_csv_format refuses. */
+uint64_t yq_csv_format_bound(const yq_batch* batch);
 /* CsvWriter::batchToCsv (include/engine/operators/csv_writer.hpp:24-76) on the
  * device, without the header line: each row's cells joined by ',' and ended
  * by '\n'; NULL -> ""; INT32/INT64 -> std::to_chars; FLOAT32 -> std::to_chars
@@ -688,8 +691,10 @@ size_t yq_csv_format_workspace_size(uint32_t rows);
  * bytes up to the slot's first NUL, not escaped. Writes the text to `out`
  * (device) and its length to *bytes; synchronises `stream` to read the
  * length, and returns YQ_ERR_CAPACITY (nothing written, *bytes = the length)
- * when it exceeds `capacity`. Line offsets are 32-bit: YQ_ERR_UNSUPPORTED when
- * rows x the widest possible line reaches 4 GiB. */
+ * when it exceeds `capacity`. With capacity >= yq_csv_format_bound(batch) the
+ * text is written without a wait for its length first. Line offsets are 32-bit:
+ * YQ_ERR_UNSUPPORTED when rows x the widest line (dates at 29 bytes) reaches
+ * 4 GiB, or the text does. */
 int yq_csv_format(const yq_batch* batch, uint8_t* out, uint64_t capacity, uint64_t* bytes, void* workspace,
                   size_t workspace_bytes, void* stream);
 

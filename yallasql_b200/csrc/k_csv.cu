@@ -456,6 +456,7 @@ struct FmtParams {
   uint32_t* len;        // bytes of each row's line
   const uint32_t* end;  // inclusive scan of len: where each line ends
   uint8_t* out;
+  uint64_t capacity;     // of `out`
   int32_t out_aligned4;  // `out` is 4-byte aligned: the copy-out may use word stores
 };
 
@@ -486,6 +487,7 @@ __global__ void __launch_bounds__(kFmtThreads) k_csv_format_write(const __grid_c
   const uint32_t r0 = blockIdx.x * kFmtThreads;
   const uint32_t rend = r0 + kFmtThreads < P.rows ? r0 + kFmtThreads : P.rows;
   const uint32_t base = r0 ? P.end[r0 - 1] : 0u, stop = P.end[rend - 1];
+  if (stop > P.capacity) return;  // (the host's checks keep it from happening; the call reports ERR_CAPACITY)
   const uint32_t abase = base & ~3u;  // s_out[i] holds output byte abase + i
   const bool staged = stop - abase <= kFmtSpan;
   const uint32_t r = r0 + threadIdx.x;
@@ -507,15 +509,15 @@ __global__ void __launch_bounds__(kFmtThreads) k_csv_format_write(const __grid_c
     *reinterpret_cast<uint32_t*>(P.out + i) = *reinterpret_cast<const uint32_t*>(s_out + (i - abase));
 }
 
-int fmt_max_cell(int32_t type, int32_t width) {
-  switch (type) {
-    case YQ_INT32: return 11;
-    case YQ_INT64: return 20;
-    case YQ_FLOAT32: return 46;   // sign, 39 integer digits, '.', 4 decimals
-    case YQ_DATETIME: return 29;  // quotes, signed 11-digit year, "-MM-DD HH:MM:SS"
-    case YQ_TEXT: return width + 2;
-    default: return -1;
+// Bytes of the longest line a batch can give, 0 for a column without a text form.
+uint64_t fmt_max_line(const yq_batch& b) {
+  uint64_t n = 0;
+  for (int c = 0; c < b.ncols; ++c) {
+    const int mc = max_cell(b.columns[c].type, b.columns[c].width);
+    if (mc < 0) return 0;
+    n += (uint64_t)mc + 1;
   }
+  return n;
 }
 
 uint32_t csv_tiles(uint64_t nbytes) { return (uint32_t)((nbytes + kTileBytes - 1) / kTileBytes); }
@@ -690,6 +692,11 @@ size_t yq_csv_format_workspace_size(uint32_t rows) {
   return w.total();
 }
 
+uint64_t yq_csv_format_bound(const yq_batch* batch) {
+  if (!batch || batch->ncols <= 0 || batch->ncols > YQ_CSV_MAX_FIELDS || !batch->columns) return 0;
+  return batch->rows * fmt_max_line(*batch);
+}
+
 int yq_csv_format(const yq_batch* batch, uint8_t* out, uint64_t capacity, uint64_t* bytes, void* workspace,
                   size_t workspace_bytes, void* stream) {
   if (!batch || !bytes || batch->ncols <= 0 || batch->ncols > YQ_CSV_MAX_FIELDS || !batch->columns)
@@ -697,20 +704,27 @@ int yq_csv_format(const yq_batch* batch, uint8_t* out, uint64_t capacity, uint64
   *bytes = 0;
   const uint32_t rows = batch->rows;
   FmtParams P;
-  uint64_t max_line = 0;
+  uint64_t dates = 0;
   for (int c = 0; c < batch->ncols; ++c) {
     const yq_column& col = batch->columns[c];
-    const int mc = fmt_max_cell(col.type, col.width);
-    if (mc < 0) return YQ_ERR_UNSUPPORTED;
+    if (max_cell(col.type, col.width) < 0) return YQ_ERR_UNSUPPORTED;
     if ((col.type == YQ_TEXT && (col.width < 1 || col.width > YQ_MAX_TEXT_WIDTH)) ||
         (col.type != YQ_TEXT && col.width != (col.type == YQ_INT32 || col.type == YQ_FLOAT32 ? 4 : 8)))
       return YQ_ERR_INVALID_ARG;
     if (rows && !col.data) return YQ_ERR_INVALID_ARG;
     P.c[c] = FmtCol{col.data, col.nulls, col.type, col.width};
-    max_line += (uint64_t)mc + 1;
+    dates += col.type == YQ_DATETIME;
   }
   if (rows == 0) return YQ_OK;
-  if ((uint64_t)rows * max_line >= (1ull << 32)) return YQ_ERR_UNSUPPORTED;  // 32-bit line offsets
+  // Offsets are 32-bit. A call is refused by 29 bytes a date, its longest text
+  // within eleven-digit years; text that passes 4 GiB all the same, through
+  // earlier dates, comes out of the 32-bit sum short by 2^32. What is left is
+  // less than the shortest text of these rows (the excess is a byte a date),
+  // which is how it is told apart below.
+  const uint64_t max_line = fmt_max_line(*batch);
+  if ((uint64_t)rows * (max_line - dates) >= (1ull << 32)) return YQ_ERR_UNSUPPORTED;
+  const bool may_wrap = (uint64_t)rows * max_line >= (1ull << 32);
+  const uint64_t min_text = (uint64_t)rows * ((uint64_t)batch->ncols * 2 + dates);  // a cell has a byte, a date two
   cudaStream_t s = as_stream(stream);
   Workspace ws;
   YQ_TRY(ws.acquire(workspace, workspace_bytes, yq_csv_format_workspace_size(rows), s));
@@ -721,6 +735,7 @@ int yq_csv_format(const yq_batch* batch, uint8_t* out, uint64_t capacity, uint64
   void* scan_ws = ws.take<uint8_t>(yq_prefix_sum_workspace_size(rows));
   P.end = end;
   P.out = out;
+  P.capacity = capacity;
   P.out_aligned4 = (reinterpret_cast<uintptr_t>(out) & 3) == 0;
   double in_bytes = 0;
   for (int c = 0; c < batch->ncols; ++c)
@@ -734,10 +749,11 @@ int yq_csv_format(const yq_batch* batch, uint8_t* out, uint64_t capacity, uint64
   // With room for the longest text of these rows the text cannot overflow: it
   // is written without waiting for its length, which is read at the end. A
   // call with less room waits first (one that lacks room writes nothing).
-  const bool fits = out && capacity >= rows * max_line;
+  const bool fits = out && !may_wrap && capacity >= rows * max_line;
   uint32_t total = 0;
   if (!fits) {
     YQ_TRY(d2h_sync(&total, end + rows - 1, sizeof(total), s));
+    if (may_wrap && total < min_text) return YQ_ERR_UNSUPPORTED;
     *bytes = total;
     if (total > capacity) return YQ_ERR_CAPACITY;
     if (!out) return YQ_ERR_INVALID_ARG;
@@ -751,6 +767,7 @@ int yq_csv_format(const yq_batch* batch, uint8_t* out, uint64_t capacity, uint64
   if (fits) {
     YQ_TRY(d2h_sync(&total, end + rows - 1, sizeof(total), s));
     *bytes = total;
+    if (total > capacity) return YQ_ERR_CAPACITY;
   }
   return YQ_OK;
 }

@@ -1245,6 +1245,19 @@ YQ_CSV_HD void put_cell(Out& o, const void* data, const uint8_t* nulls, int32_t 
   }
 }
 
+// Bytes of the longest text put_cell gives a cell of this type; -1: no text
+// form. Callers size buffers by it, so it has to hold for every value.
+YQ_CSV_HD int max_cell(int32_t type, int32_t width) {
+  switch (type) {
+    case 0: return 11;  // "-2147483648"
+    case 4: return 20;  // "-9223372036854775808"
+    case 1: return 46;  // sign, 39 integer digits, '.', 4 decimals
+    case 2: return 30;  // quotes, sign, 12-digit year (int64 seconds reach -292277022657), "-MM-DD HH:MM:SS"
+    case 3: return width + 2;
+    default: return -1;
+  }
+}
+
 // Output that only counts bytes.
 struct CountOut {
   uint32_t n = 0;

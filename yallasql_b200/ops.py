@@ -752,8 +752,6 @@ def read_csv(data: bytes, project: list[str] | None = None, text_width: int = 25
     return [schema[f] for f in fields], batch
 
 
-# Longest text of a cell by type (TEXT: its slot and two quotes).
-_CSV_MAX_CELL = {A.INT32: 11, A.INT64: 20, A.FLOAT32: 46, A.DATETIME: 29}
 _CSV_ONE_PASS_BYTES = 1 << 30
 
 
@@ -767,7 +765,7 @@ def csv_format(batch: DeviceBatch, stream=None) -> torch.Tensor:
     n = C.c_uint64(0)
     # with room for the longest text these rows can have one call counts and
     # writes; otherwise a first call only counts
-    bound = batch.rows * sum(_CSV_MAX_CELL.get(c.type, c.width + 2) + 1 for c in batch.columns)
+    bound = int(L.yq_csv_format_bound(C.byref(cols)))
     if 0 < bound <= _CSV_ONE_PASS_BYTES:
         out = torch.empty(bound, dtype=torch.uint8, device="cuda")
         _check(L.yq_csv_format(C.byref(cols), out.data_ptr(), bound, C.byref(n), None, 0, s), "yq_csv_format")
