@@ -697,6 +697,14 @@ uint64_t yq_csv_format_bound(const yq_batch* batch);
  * 4 GiB, or the text does. */
 int yq_csv_format(const yq_batch* batch, uint8_t* out, uint64_t capacity, uint64_t* bytes, void* workspace,
                   size_t workspace_bytes, void* stream);
+/* yq_csv_format into a buffer of the text's own size: once the length is known,
+ * `alloc(ctx, bytes)` is called (on this thread, not for 0 rows) for a device
+ * buffer of that many bytes, which stays the caller's; NULL from it ends the
+ * call with YQ_ERR_ALLOC. The text is stream ordered: the call waits for its
+ * length, not for the text. */
+typedef void* (*yq_alloc_fn)(void* ctx, uint64_t bytes);
+int yq_csv_format_alloc(const yq_batch* batch, yq_alloc_fn alloc, void* alloc_ctx, uint64_t* bytes, void* workspace,
+                        size_t workspace_bytes, void* stream);
 
 /* ---------------------------------------------------------------- device */
 /* Number of SMs of the current device (cached per device). */

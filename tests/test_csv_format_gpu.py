@@ -87,3 +87,36 @@ def test_text_past_32_bit_offsets(cuda, yq):
     more = ops.DeviceBatch([ops.DeviceColumn(torch.empty(143_165_577, dtype=torch.int64, device="cuda"), A.DATETIME)])
     bc, keep = more.c()  # 30 bytes a line with a date's 29: refused by its size
     assert yq.yq_csv_format(C.byref(bc), None, 0, C.byref(n), None, 0, None) == A.ERR_UNSUPPORTED
+
+
+def test_result_is_the_texts_own_size(cuda):
+    """The tensor holds the text and nothing else, and no more than the text is
+    allocated for it on the way; another stream, no rows, a failed allocation."""
+    rows = 300_000  # 7 bytes a line; the longest such line has 48 and 12
+    batch = ops.DeviceBatch([col(np.full(rows, 7, np.float32), A.FLOAT32), col(np.arange(rows, dtype=np.int32) % 10, A.INT32)])
+    want = b"".join(b"7.0000,%d\n" % (i % 10) for i in range(rows))
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    text = ops.csv_format(batch)
+    assert torch.cuda.max_memory_allocated() - before <= len(want) + 4096
+    assert text.untyped_storage().nbytes() == text.numel() == len(want)
+    assert text.cpu().numpy().tobytes() == want
+    side = torch.cuda.Stream()
+    assert ops.csv_format(batch, stream=side).cpu().numpy().tobytes() == want
+    assert ops.write_csv(["a", "b"], batch, stream=side) == b"a,b\n" + want
+    none = ops.csv_format(ops.DeviceBatch([ops.DeviceColumn(torch.empty(0, device="cuda"), A.FLOAT32)]))
+    assert none.numel() == 0 and none.is_cuda
+
+
+def test_failed_allocation_of_the_text(cuda, monkeypatch):
+    batch = ops.DeviceBatch([col(np.arange(1000, dtype=np.int32), A.INT32)])
+    want = ops.csv_format(batch).cpu()
+
+    def no_memory(*a, **k):
+        raise torch.cuda.OutOfMemoryError("no room")
+    with monkeypatch.context() as m:
+        m.setattr(ops.torch, "empty", no_memory)
+        with pytest.raises(torch.cuda.OutOfMemoryError, match="no room"):
+            ops.csv_format(batch)
+    assert torch.equal(ops.csv_format(batch).cpu(), want)

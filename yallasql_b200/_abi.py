@@ -102,6 +102,7 @@ CSV_MAX_FIELDS = 64
 
 P = C.POINTER
 vp, sz, u32, i32, u64 = C.c_void_p, C.c_size_t, C.c_uint32, C.c_int32, C.c_uint64
+ALLOC_FN = C.CFUNCTYPE(vp, vp, u64)  # yq_alloc_fn
 
 # name -> (restype, argtypes). Every symbol declared in include/yq_ops.h.
 PROTOTYPES = {
@@ -183,6 +184,7 @@ PROTOTYPES = {
     "yq_csv_format_workspace_size": (sz, [u32]),
     "yq_csv_format_bound": (u64, [P(Batch)]),
     "yq_csv_format": (C.c_int, [P(Batch), vp, u64, P(u64), vp, sz, vp]),
+    "yq_csv_format_alloc": (C.c_int, [P(Batch), ALLOC_FN, vp, P(u64), vp, sz, vp]),
     "yq_device_sm_count": (C.c_int, []),
     "yq_launch_count": (u64, []),
     "yq_workspace_trim": (i32, []),

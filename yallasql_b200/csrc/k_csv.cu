@@ -697,13 +697,18 @@ uint64_t yq_csv_format_bound(const yq_batch* batch) {
   return batch->rows * fmt_max_line(*batch);
 }
 
-int yq_csv_format(const yq_batch* batch, uint8_t* out, uint64_t capacity, uint64_t* bytes, void* workspace,
-                  size_t workspace_bytes, void* stream) {
+}  // extern "C"
+
+// `alloc` (when given) supplies `out` once the text's length is known.
+static int csv_format_impl(const yq_batch* batch, uint8_t* out, uint64_t capacity, yq_alloc_fn alloc, void* alloc_ctx,
+                           uint64_t* bytes, void* workspace, size_t workspace_bytes, void* stream) {
   if (!batch || !bytes || batch->ncols <= 0 || batch->ncols > YQ_CSV_MAX_FIELDS || !batch->columns)
     return YQ_ERR_INVALID_ARG;
   *bytes = 0;
   const uint32_t rows = batch->rows;
   FmtParams P;
+  P.out = nullptr;
+  P.capacity = 0;
   uint64_t dates = 0;
   for (int c = 0; c < batch->ncols; ++c) {
     const yq_column& col = batch->columns[c];
@@ -734,9 +739,6 @@ int yq_csv_format(const yq_batch* batch, uint8_t* out, uint64_t capacity, uint64
   uint32_t* end = ws.take<uint32_t>((size_t)rows + 1);
   void* scan_ws = ws.take<uint8_t>(yq_prefix_sum_workspace_size(rows));
   P.end = end;
-  P.out = out;
-  P.capacity = capacity;
-  P.out_aligned4 = (reinterpret_cast<uintptr_t>(out) & 3) == 0;
   double in_bytes = 0;
   for (int c = 0; c < batch->ncols; ++c)
     in_bytes += (double)rows * (batch->columns[c].width + (batch->columns[c].nulls ? 1 : 0));
@@ -755,9 +757,17 @@ int yq_csv_format(const yq_batch* batch, uint8_t* out, uint64_t capacity, uint64
     YQ_TRY(d2h_sync(&total, end + rows - 1, sizeof(total), s));
     if (may_wrap && total < min_text) return YQ_ERR_UNSUPPORTED;
     *bytes = total;
+    if (alloc) {
+      out = static_cast<uint8_t*>(alloc(alloc_ctx, total));
+      if (!out) return YQ_ERR_ALLOC;
+      capacity = total;
+    }
     if (total > capacity) return YQ_ERR_CAPACITY;
     if (!out) return YQ_ERR_INVALID_ARG;
   }
+  P.out = out;
+  P.capacity = capacity;
+  P.out_aligned4 = (reinterpret_cast<uintptr_t>(out) & 3) == 0;
   YQ_TRY(kernel_allow_smem((const void*)k_csv_format_write, kFmtSpan + 16));
   {
     ProfScope ps("csv_format_write", s, in_bytes + (double)total);
@@ -770,6 +780,19 @@ int yq_csv_format(const yq_batch* batch, uint8_t* out, uint64_t capacity, uint64
     if (total > capacity) return YQ_ERR_CAPACITY;
   }
   return YQ_OK;
+}
+
+extern "C" {
+
+int yq_csv_format(const yq_batch* batch, uint8_t* out, uint64_t capacity, uint64_t* bytes, void* workspace,
+                  size_t workspace_bytes, void* stream) {
+  return csv_format_impl(batch, out, capacity, nullptr, nullptr, bytes, workspace, workspace_bytes, stream);
+}
+
+int yq_csv_format_alloc(const yq_batch* batch, yq_alloc_fn alloc, void* alloc_ctx, uint64_t* bytes, void* workspace,
+                        size_t workspace_bytes, void* stream) {
+  if (!alloc) return YQ_ERR_INVALID_ARG;
+  return csv_format_impl(batch, nullptr, 0, alloc, alloc_ctx, bytes, workspace, workspace_bytes, stream);
 }
 
 }  // extern "C"

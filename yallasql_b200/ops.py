@@ -752,33 +752,32 @@ def read_csv(data: bytes, project: list[str] | None = None, text_width: int = 25
     return [schema[f] for f in fields], batch
 
 
-_CSV_ONE_PASS_BYTES = 1 << 30
-
-
 def csv_format(batch: DeviceBatch, stream=None) -> torch.Tensor:
-    """The rows of a device batch as CSV text on the device (uint8 tensor),
-    formatted as the reference's CsvWriter::batchToCsv formats them
-    (include/engine/operators/csv_writer.hpp:24-76), without the header line."""
+    """The rows of a device batch as CSV text on the device (uint8 tensor of
+    the text's own size), formatted as the reference's CsvWriter::batchToCsv
+    formats them (include/engine/operators/csv_writer.hpp:24-76), without the
+    header line."""
     L = lib()
     s = _stream(stream)
     cols, keep = batch.c()
     n = C.c_uint64(0)
-    # with room for the longest text these rows can have one call counts and
-    # writes; otherwise a first call only counts
-    bound = int(L.yq_csv_format_bound(C.byref(cols)))
-    if 0 < bound <= _CSV_ONE_PASS_BYTES:
-        out = torch.empty(bound, dtype=torch.uint8, device="cuda")
-        _check(L.yq_csv_format(C.byref(cols), out.data_ptr(), bound, C.byref(n), None, 0, s), "yq_csv_format")
-        out = out[: int(n.value)]
-        return out.clone() if bound > 4 * int(n.value) else out
-    st = L.yq_csv_format(C.byref(cols), None, 0, C.byref(n), None, 0, s)
-    if st not in (A.OK, A.ERR_CAPACITY):
-        _check(st, "yq_csv_format")
-    out = torch.empty(max(int(n.value), 1), dtype=torch.uint8, device="cuda")
-    if n.value:
-        _check(L.yq_csv_format(C.byref(cols), out.data_ptr(), int(n.value), C.byref(n), None, 0, s), "yq_csv_format")
+    text, failed = [], []
+
+    def alloc(_ctx, nbytes):
+        try:
+            text.append(torch.empty(nbytes, dtype=torch.uint8, device="cuda"))
+            return text[0].data_ptr()
+        except Exception as e:  # raised below: it cannot pass through the C call
+            failed.append(e)
+            return None
+    st = L.yq_csv_format_alloc(C.byref(cols), A.ALLOC_FN(alloc), None, C.byref(n), None, 0, s)
+    if failed:
+        raise failed[0]
+    _check(st, "yq_csv_format_alloc")
+    if s != _stream():  # the text belongs to the current stream: written before it is handed out
+        torch.cuda.ExternalStream(s).synchronize()
     del keep
-    return out[: int(n.value)]
+    return text[0] if text else torch.empty(0, dtype=torch.uint8, device="cuda")
 
 
 def write_csv(names: list[str], batch: DeviceBatch, stream=None) -> bytes:
