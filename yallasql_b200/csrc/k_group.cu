@@ -27,8 +27,8 @@
 //
 // Integer keys of few distinct values (up to kFewGroups) skip the sort:
 //   k_few_find        the distinct keys, through a hash table per block (a NULL
-//                     key or too many keys send the call to the sort)
-//   k_few_order       their ascending order = the group indices
+//                     key or too many keys send the call to the sort), and
+//                     their ascending order = the group indices
 //   k_few_accumulate  one pass over the input columns into accumulators that
 //                     each thread owns in shared memory
 //   k_few_finish      each group's partials folded in block order
@@ -481,16 +481,16 @@ __global__ void __launch_bounds__(kGroupThreads) k_group_span(const __grid_const
 
 // ------------------------------------------------------- few distinct keys
 // With few groups the sort, its permutation and the reads through it are most
-// of the work (32M rows, 11 groups, five aggregates: 1.63 ms of kernels, 0.25 ms here, for
-// 384 MB of input). Here the input is read once to find the keys and once to
+// of the work (32M rows, 11 groups, five aggregates: 1.63 ms of kernels, 0.25 ms
+// here, for 384 MB of input). Here the input is read once to find the keys and once to
 // accumulate. Each thread owns an accumulator per group and aggregate in
 // shared memory (element [group][thread], so a warp's 32 updates hit 32
 // banks whatever groups its rows belong to) and adds its rows in row order;
 // threads, then blocks, fold in a fixed tree. So sums need no atomics and the
 // bits do not depend on scheduling. Latency-bound on the shared-memory
 // read-modify-writes; eight rows a thread are loaded ahead.
-// The group limit is the accumulators': at 28 bytes a thread and group, 50
-// groups leave one block of 128 threads on an SM.
+// The group limit is the accumulators' (few_limit): at 28 bytes a thread and
+// group, 50 groups leave one block of 128 threads on an SM and 61 fill it.
 constexpr int kFewThreads = 128;
 constexpr int kFewItems = 8;
 constexpr uint32_t kFewGroups = 96;
@@ -498,10 +498,10 @@ constexpr uint32_t kFewSlots = 512;          // hash slots, at most a fifth full
 constexpr int kFewFindThreads = 256;
 constexpr unsigned long long kNoKey = ~0ull;  // empty slot; the key of that value has a flag of its own
 
-struct FewTable {
-  unsigned long long keys[kFewSlots];  // kNoKey on entry
-  uint32_t count, has_last, overflow, ngroups;  // zero on entry, as all below
-  uint32_t last_gid, pad;
+struct FewTable {  // all zero on entry
+  unsigned long long keys[kFewSlots];  // ~key (0, an empty slot, would be the key kNoKey's)
+  uint32_t count, has_last, overflow, ngroups;
+  uint32_t last_gid, ticket, err, pad;
   uint32_t gid[kFewSlots];
   unsigned long long group_key[kFewGroups];
 };
@@ -511,31 +511,76 @@ __device__ __forceinline__ uint32_t few_hash(unsigned long long k) {  // the top
 }
 static_assert(kFewSlots == 512, "few_hash gives nine bits");
 
-// Puts `key` into the table (empty slots hold `empty`, which is not a key to
-// put in); false when it holds too many keys.
+// Puts `value` into the table from slot h on (empty slots hold `empty`, which is
+// no value to put in); false when that makes more than `limit` values.
 template <typename K>
-__device__ __forceinline__ bool few_insert(K* keys, uint32_t* count, K key, K empty) {
-  uint32_t h = few_hash(key);
+__device__ __forceinline__ bool few_insert(K* table, uint32_t* count, K value, K empty, uint32_t h, uint32_t limit) {
   for (uint32_t n = 0; n < kFewSlots; ++n, h = (h + 1) & (kFewSlots - 1)) {
-    K cur = *reinterpret_cast<volatile K*>(keys + h);
-    if (cur == key) return true;
+    K cur = *reinterpret_cast<volatile K*>(table + h);
+    if (cur == value) return true;
     if (cur != empty) continue;
-    cur = atomicCAS(keys + h, empty, key);
-    if (cur == empty) return atomicAdd(count, 1u) < kFewGroups;
-    if (cur == key) return true;
+    cur = atomicCAS(table + h, empty, value);
+    if (cur == empty) return atomicAdd(count, 1u) < limit;
+    if (cur == value) return true;
   }
   return false;
 }
 
+// Group index of every key: ascending signed order. The keys are compacted
+// first, so that each looks at the others and not at every slot. Run by one
+// block, whose stores to T the next kernel reads.
+template <int BLOCK>
+__device__ __forceinline__ void few_order(FewTable* T, int width, uint32_t limit) {
+  __shared__ long long s_val[kFewGroups];
+  __shared__ uint32_t s_n;
+  const volatile FewTable* V = T;  // other blocks wrote it: not from L1
+  const bool has_last = V->has_last != 0u;
+  const uint32_t n = V->count + (has_last ? 1u : 0u);
+  if (V->overflow || n > limit) {
+    if (threadIdx.x == 0) T->overflow = 1u;
+    return;
+  }
+  if (threadIdx.x == 0) s_n = 0u;
+  __syncthreads();
+  auto value_of = [&](unsigned long long k) { return width == 4 ? (long long)(int32_t)(uint32_t)k : (long long)k; };
+  for (uint32_t i = threadIdx.x; i < kFewSlots; i += BLOCK) {
+    const unsigned long long k = ~V->keys[i];
+    if (k != kNoKey) s_val[atomicAdd(&s_n, 1u)] = value_of(k);
+  }
+  if (threadIdx.x == 0 && has_last) s_val[atomicAdd(&s_n, 1u)] = -1ll;  // the 8-byte key ~0
+  __syncthreads();
+  auto rank_of = [&](long long v) {
+    uint32_t r = 0;
+    for (uint32_t j = 0; j < n; ++j) r += s_val[j] < v ? 1u : 0u;
+    return r;
+  };
+  for (uint32_t i = threadIdx.x; i < kFewSlots; i += BLOCK) {
+    const unsigned long long k = ~V->keys[i];
+    if (k == kNoKey) continue;
+    const uint32_t rank = rank_of(value_of(k));
+    T->gid[i] = rank;
+    T->group_key[rank] = k;
+  }
+  if (threadIdx.x == 0) {
+    if (has_last) {
+      const uint32_t rank = rank_of(-1ll);
+      T->last_gid = rank;
+      T->group_key[rank] = kNoKey;
+    }
+    T->ngroups = n;
+  }
+}
+
+// `head` (mapped host memory): whether the table is of no use, and its groups.
 // K: the key's bits. Row 0's key is known to be there, so a block's table is
 // filled with it: empty slots need no value outside the key's own, and a probe
 // is a product, a load and a compare.
 template <typename K>
 __global__ void __launch_bounds__(kFewFindThreads) k_few_find(const K* __restrict__ keys,
                                                               const uint8_t* __restrict__ nulls, uint32_t rows,
-                                                              FewTable* T) {
+                                                              uint32_t limit, FewTable* T, uint32_t* head) {
   __shared__ K s_keys[kFewSlots];
-  __shared__ uint32_t s_count, s_over;
+  __shared__ uint32_t s_count, s_over, s_last;
   const K first = __ldg(keys);
   for (uint32_t i = threadIdx.x; i < kFewSlots; i += kFewFindThreads) s_keys[i] = first;
   if (threadIdx.x == 0) {
@@ -574,7 +619,7 @@ __global__ void __launch_bounds__(kFewFindThreads) k_few_find(const K* __restric
 #pragma unroll
       for (int q = 1; q < kFewItems; ++q)
         if (q == m) key = k[q];
-      ok = few_insert<K>(s_keys, &s_count, key, first);
+      ok = few_insert<K>(s_keys, &s_count, key, first, few_hash(key), limit);
     }
     if (!ok || over) s_over = 1u;
     // this block or another one has found too many keys: the table is not used
@@ -583,51 +628,27 @@ __global__ void __launch_bounds__(kFewFindThreads) k_few_find(const K* __restric
   __syncthreads();
   if (s_over) {
     if (threadIdx.x == 0) atomicOr(&T->overflow, 1u);
-    return;
-  }
-  for (uint32_t i = threadIdx.x; i <= kFewSlots; i += kFewFindThreads) {
-    const K key = i < kFewSlots ? s_keys[i] : first;
-    if (i < kFewSlots && key == first) continue;
-    if ((unsigned long long)key == kNoKey) atomicOr(&T->has_last, 1u);
-    else if (!few_insert<unsigned long long>(T->keys, &T->count, key, kNoKey)) atomicOr(&T->overflow, 1u);
-  }
-}
-
-// Group index of every key: ascending signed order. The keys are compacted
-// first, so that each looks at the others and not at every slot.
-__global__ void __launch_bounds__(kFewSlots) k_few_order(FewTable* T, int width) {
-  __shared__ long long s_val[kFewGroups];
-  __shared__ uint32_t s_n;
-  const uint32_t i = threadIdx.x;
-  const unsigned long long mine = T->keys[i];
-  const uint32_t n = T->count + (T->has_last ? 1u : 0u);
-  if (T->overflow || n > kFewGroups) {
-    if (i == 0) T->overflow = 1u;
-    return;
-  }
-  if (i == 0) s_n = 0u;
-  __syncthreads();
-  const long long value = width == 4 ? (long long)(int32_t)(uint32_t)mine : (long long)mine;
-  if (mine != kNoKey) s_val[atomicAdd(&s_n, 1u)] = value;
-  if (i == 0 && T->has_last) s_val[atomicAdd(&s_n, 1u)] = -1ll;  // the 8-byte key ~0
-  __syncthreads();
-  auto rank_of = [&](long long v) {
-    uint32_t r = 0;
-    for (uint32_t j = 0; j < n; ++j) r += s_val[j] < v ? 1u : 0u;
-    return r;
-  };
-  if (mine != kNoKey) {
-    const uint32_t rank = rank_of(value);
-    T->gid[i] = rank;
-    T->group_key[rank] = mine;
-  }
-  if (i == 0) {
-    if (T->has_last) {
-      const uint32_t rank = rank_of(-1ll);
-      T->last_gid = rank;
-      T->group_key[rank] = kNoKey;
+  } else {
+    for (uint32_t i = threadIdx.x; i <= kFewSlots; i += kFewFindThreads) {
+      const K key = i < kFewSlots ? s_keys[i] : first;
+      if (i < kFewSlots && key == first) continue;
+      const unsigned long long k = key;
+      if (k == kNoKey) atomicOr(&T->has_last, 1u);
+      else if (!few_insert<unsigned long long>(T->keys, &T->count, ~k, 0ull, few_hash(k), limit)) atomicOr(&T->overflow, 1u);
     }
-    T->ngroups = n;
+  }
+  // the last block to get here has every block's keys before it
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(&T->ticket, 1u) == gridDim.x - 1 ? 1u : 0u;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  few_order<kFewFindThreads>(T, (int)sizeof(K), limit);
+  if (threadIdx.x == 0) {  // its own stores, or another block's flag
+    head[0] = *reinterpret_cast<volatile uint32_t*>(&T->overflow);
+    head[1] = T->ngroups;
+    __threadfence_system();
   }
 }
 
@@ -659,6 +680,7 @@ struct FewParams {
   uint32_t rows_per_block;
   const FewTable* T;
   GPart* part;        // [blocks][groups][nagg]
+  uint32_t* host_err; // mapped host memory
   yq_column out_key;
 };
 
@@ -726,7 +748,7 @@ __global__ void __launch_bounds__(kFewThreads, 5) k_few_accumulate(const __grid_
   const uint32_t G = F.ngroups, tid = threadIdx.x;
   const size_t unit = (size_t)G * kFewThreads;  // elements of one array
   for (uint32_t i = tid; i < kFewSlots; i += kFewThreads) {
-    const unsigned long long key = F.T->keys[i];
+    const unsigned long long key = ~F.T->keys[i];
     s_slot[i].key = (K)key;
     s_slot[i].gid = key == kNoKey ? (K)kNoGroup : (K)F.T->gid[i];
   }
@@ -897,6 +919,10 @@ __global__ void __launch_bounds__(kFinishThreads) k_few_finish(const __grid_cons
     if (F.out_key.width == 4) static_cast<uint32_t*>(F.out_key.data)[g] = (uint32_t)k;
     else static_cast<unsigned long long*>(F.out_key.data)[g] = k;
     if (F.out_key.nulls) const_cast<uint8_t*>(F.out_key.nulls)[g] = 0;
+    if (g == 0) {
+      *F.host_err = *F.P.err;
+      __threadfence_system();
+    }
   }
   if (j >= F.P.nagg) return;
   const GAgg& a = F.P.a[j];
@@ -943,13 +969,14 @@ size_t few_workspace_bytes(int32_t nagg) {
   WsSize w;
   w.add<FewTable>(1);
   w.add<GPart>((size_t)sm_count() * kFewBlocksPerSm * kFewGroups * (nagg > 0 ? nagg : 1));
-  w.add<uint32_t>(4);
   return w.total();
 }
 
-// Rows from which the search for few distinct keys pays for itself when it
-// fails (a search that meets too many keys stops within its first steps, but
-// its launches and its read-back take about 25 us).
+// Rows from which the search for few distinct keys is made. One that fails
+// stops within its first steps and costs two launches and a wait, 19 us; where
+// it succeeds the call takes 76 us instead of 170 (100K rows, 11 groups, five
+// aggregates), and from 130K rows on, where the sort's path also orders its
+// tiles, 67 instead of 247.
 constexpr uint32_t kFewMinRows = 100000;
 
 // (Above 2^30 rows the sort refuses the call, and 32-bit row arithmetic ends.)
@@ -957,54 +984,16 @@ bool few_applies(const yq_column& key, uint32_t rows) {
   return rows >= kFewMinRows && rows < (1u << 30) && (key.type == YQ_INT32 || key.type == YQ_INT64 || key.type == YQ_DATETIME);
 }
 
-// The sort-free path. *done = false: the keys are too many (or one is NULL)
-// and nothing was written.
-int group_by_few(const GroupParams& P, const yq_column& key, const yq_column& out_key, uint32_t capacity,
-                 uint32_t* groups, void* few_ws, size_t few_bytes, cudaStream_t s, bool* done) {
-  *done = false;
-  Workspace ws;
-  YQ_TRY(ws.acquire(few_ws, few_bytes, few_workspace_bytes(P.nagg), s));
-  FewTable* T = ws.take<FewTable>(1);
-  GPart* part = ws.take<GPart>((size_t)sm_count() * kFewBlocksPerSm * kFewGroups * (P.nagg > 0 ? P.nagg : 1));
-  uint32_t* d_err = ws.take<uint32_t>(4);
-  YQ_TRY_CUDA(cudaMemsetAsync(T->keys, 0xff, sizeof(T->keys), s));
-  YQ_TRY_CUDA(cudaMemsetAsync(&T->count, 0, sizeof(FewTable) - sizeof(T->keys), s));
-  const unsigned step = kFewFindThreads * kFewItems;
-  unsigned grid = grid_for(P.rows, step);
-  const void* find = key.width == 4 ? (const void*)k_few_find<uint32_t> : (const void*)k_few_find<unsigned long long>;
-  const unsigned resident = (unsigned)(sm_count() * kernel_blocks_per_sm(find, kFewFindThreads, 0));
-  if (grid > resident) grid = resident;
-  {
-    ProfScope ps("group_few_find", s, (double)P.rows * key.width);
-    if (key.width == 4)
-      k_few_find<uint32_t><<<grid, kFewFindThreads, 0, s>>>(static_cast<const uint32_t*>(key.data), key.nulls, P.rows, T);
-    else
-      k_few_find<unsigned long long><<<grid, kFewFindThreads, 0, s>>>(static_cast<const unsigned long long*>(key.data),
-                                                                      key.nulls, P.rows, T);
-    YQ_CHECK_LAUNCH();
-  }
-  k_few_order<<<1, kFewSlots, 0, s>>>(T, key.width);
-  YQ_CHECK_LAUNCH();
-  uint32_t head[4];  // count, has_last, overflow, ngroups
-  YQ_TRY(d2h_sync(head, &T->count, sizeof(head), s));
-  const uint32_t G = head[3];
-  if (head[2] || G == 0) return YQ_OK;
-  FewParams F;
-  F.P = P;
-  F.P.err = d_err;
-  F.key = key;
-  F.out_key = out_key;
-  F.ngroups = G;
-  F.T = T;
-  F.part = part;
-  // arrays in descending element size, so each stays aligned
-  int off = 0;
+// The accumulators of a call's aggregates: which arrays a thread keeps per group.
+void few_layout(const GroupParams& P, FewParams& F) {
   auto value_size = [&](int j) {
     const GAgg& a = P.a[j];
     if (a.kind == YQ_AGG_COUNT || a.kind == YQ_AGG_COUNT_STAR) return 0;
     return a.kind == YQ_AGG_SUM || a.kind == YQ_AGG_AVG || a.width == 8 ? 8 : 4;
   };
-  off = 4;  // the row counts; padded to 8 with the 4-byte arrays placed first
+  // An array begins its offset times the elements of one array (a multiple of
+  // 128) into the room, so it is aligned whatever its element size.
+  int off = 4;  // the row counts
   F.ncol = 0;
   int placed = 0;
   for (int j = 0; j < P.nagg; ++j) F.acc[j] = FewAcc{0, -1, 0};
@@ -1028,22 +1017,78 @@ int group_by_few(const GroupParams& P, const yq_column& key, const yq_column& ou
       F.acc[i].cnt_off = C.cnt_off;
     }
   }
-  for (const int size : {4, 8}) {
-    for (int j = 0; j < P.nagg; ++j) {
-      if (value_size(j) != size) continue;
-      F.acc[j].val_off = off;
-      F.acc[j].val_size = size;
-      off += size;
-    }
+  for (int j = 0; j < P.nagg; ++j) {
+    if (value_size(j) == 0) continue;
+    F.acc[j].val_off = off;
+    F.acc[j].val_size = value_size(j);
+    off += value_size(j);
   }
   F.bytes = off;
-  const size_t smem = (size_t)kFewSlots * 2 * key.width + (size_t)G * kFewThreads * off;
-  if (smem > 220 * 1024) return YQ_OK;  // too many accumulators for one block
+}
+
+size_t few_smem(int key_width, uint32_t groups, int bytes) {
+  return (size_t)kFewSlots * 2 * key_width + (size_t)groups * kFewThreads * bytes;
+}
+
+// Groups whose accumulators a block has room for. The search for the keys stops
+// at it: a key of more values is known after its first rows instead of after
+// the whole column.
+constexpr size_t kFewSmem = 220 * 1024;
+uint32_t few_limit(int key_width, int bytes) {
+  const size_t n = (kFewSmem - few_smem(key_width, 0, 0)) / ((size_t)kFewThreads * bytes);
+  return n < kFewGroups ? (uint32_t)n : kFewGroups;
+}
+
+// The sort-free path. *done = false: the keys are too many (or one is NULL)
+// and nothing was written.
+int group_by_few(const GroupParams& P, const yq_column& key, const yq_column& out_key, uint32_t capacity,
+                 uint32_t* groups, void* few_ws, size_t few_bytes, cudaStream_t s, bool* done) {
+  *done = false;
+  FewParams F;
+  F.P = P;
+  few_layout(P, F);
+  const uint32_t limit = few_limit(key.width, F.bytes);
+  if (limit == 0) return YQ_OK;
+  Workspace ws;
+  YQ_TRY(ws.acquire(few_ws, few_bytes, few_workspace_bytes(P.nagg), s));
+  FewTable* T = ws.take<FewTable>(1);
+  GPart* part = ws.take<GPart>((size_t)sm_count() * kFewBlocksPerSm * kFewGroups * (P.nagg > 0 ? P.nagg : 1));
+  // one memset, and each kernel leaves the host's words itself: a search that
+  // fails costs two launches and a wait
+  MappedWords m;
+  YQ_TRY(m.acquire());
+  YQ_TRY_CUDA(cudaMemsetAsync(T, 0, sizeof(FewTable), s));
+  const unsigned step = kFewFindThreads * kFewItems;
+  unsigned grid = grid_for(P.rows, step);
+  const void* find = key.width == 4 ? (const void*)k_few_find<uint32_t> : (const void*)k_few_find<unsigned long long>;
+  const unsigned resident = (unsigned)(sm_count() * kernel_blocks_per_sm(find, kFewFindThreads, 0));
+  if (grid > resident) grid = resident;
+  {
+    ProfScope ps("group_few_find", s, (double)P.rows * key.width);
+    if (key.width == 4)
+      k_few_find<uint32_t><<<grid, kFewFindThreads, 0, s>>>(static_cast<const uint32_t*>(key.data), key.nulls, P.rows,
+                                                            limit, T, m.device);
+    else
+      k_few_find<unsigned long long><<<grid, kFewFindThreads, 0, s>>>(static_cast<const unsigned long long*>(key.data),
+                                                                      key.nulls, P.rows, limit, T, m.device);
+    YQ_CHECK_LAUNCH();
+  }
+  YQ_TRY_CUDA(cudaStreamSynchronize(s));
+  const uint32_t G = m.host[1];
+  if (m.host[0] || G == 0) return YQ_OK;
+  F.P.err = &T->err;
+  F.key = key;
+  F.out_key = out_key;
+  F.ngroups = G;
+  F.T = T;
+  F.part = part;
+  F.host_err = m.device + 2;
   if (G > capacity) {
     *groups = G;
     *done = true;
     return YQ_ERR_CAPACITY;
   }
+  const size_t smem = few_smem(key.width, G, F.bytes);
   void (*const accumulate)(FewParams) =
       key.width == 4 ? k_few_accumulate<uint32_t> : k_few_accumulate<unsigned long long>;
   YQ_TRY(kernel_allow_smem((const void*)accumulate, smem));
@@ -1053,7 +1098,6 @@ int group_by_few(const GroupParams& P, const yq_column& key, const yq_column& ou
   if (blocks > (unsigned)(sm_count() * per_sm)) blocks = (unsigned)(sm_count() * per_sm);
   F.rows_per_block = (uint32_t)align_up(((size_t)P.rows + blocks - 1) / blocks, kFewThreads * kFewItems);
   blocks = (P.rows + F.rows_per_block - 1) / F.rows_per_block;
-  YQ_TRY_CUDA(cudaMemsetAsync(d_err, 0, 4 * sizeof(uint32_t), s));
   double in_bytes = (double)P.rows * key.width;
   for (int j = 0; j < P.nagg; ++j)
     if (P.a[j].data) in_bytes += (double)P.rows * (type_width(P.a[j].type) + (P.a[j].nulls ? 1 : 0));
@@ -1064,11 +1108,10 @@ int group_by_few(const GroupParams& P, const yq_column& key, const yq_column& ou
   }
   k_few_finish<<<dim3(G, (unsigned)(P.nagg > 0 ? P.nagg : 1)), kFinishThreads, 0, s>>>(F, blocks);
   YQ_CHECK_LAUNCH();
-  uint32_t err = 0;
-  YQ_TRY(d2h_sync(&err, d_err, sizeof(err), s));
+  YQ_TRY_CUDA(cudaStreamSynchronize(s));
   *groups = G;
   *done = true;
-  return err ? YQ_ERR_INVALID_ARG : YQ_OK;
+  return m.host[2] ? YQ_ERR_INVALID_ARG : YQ_OK;
 }
 
 }  // namespace

@@ -108,6 +108,33 @@ __global__ void k_to_host(uint32_t* __restrict__ dst, const uint32_t* __restrict
   __threadfence_system();
 }
 
+int MappedWords::acquire() {
+  int d = 0;
+  YQ_TRY_CUDA(cudaGetDevice(&d));
+  if (d < 0 || d >= 64) return YQ_ERR_UNSUPPORTED;
+  {
+    std::lock_guard<std::mutex> lk(g_mapped_mu);
+    if (!g_mapped_free[d].empty()) {
+      host = g_mapped_free[d].back();
+      g_mapped_free[d].pop_back();
+    }
+  }
+  if (!host) {
+    void* h = nullptr;
+    YQ_TRY_CUDA(cudaHostAlloc(&h, kMappedBytes, cudaHostAllocMapped | cudaHostAllocPortable));
+    host = static_cast<uint32_t*>(h);
+  }
+  dev = d;
+  YQ_TRY_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void**>(&device), host, 0));
+  return YQ_OK;
+}
+
+MappedWords::~MappedWords() {
+  if (dev < 0) return;
+  std::lock_guard<std::mutex> lk(g_mapped_mu);
+  g_mapped_free[dev].push_back(host);
+}
+
 int d2h_sync(void* host_dst, const void* dev_src, size_t bytes, cudaStream_t s) {
   if (bytes == 0) return YQ_OK;
   int dev = 0;
@@ -119,35 +146,12 @@ int d2h_sync(void* host_dst, const void* dev_src, size_t bytes, cudaStream_t s) 
     YQ_TRY_CUDA(cudaStreamSynchronize(s));
     return YQ_OK;
   }
-  uint32_t* buf = nullptr;
-  {
-    std::lock_guard<std::mutex> lk(g_mapped_mu);
-    if (!g_mapped_free[dev].empty()) {
-      buf = g_mapped_free[dev].back();
-      g_mapped_free[dev].pop_back();
-    }
-  }
-  if (!buf) {
-    void* h = nullptr;
-    YQ_TRY_CUDA(cudaHostAlloc(&h, kMappedBytes, cudaHostAllocMapped | cudaHostAllocPortable));
-    buf = static_cast<uint32_t*>(h);
-  }
-  uint32_t* dptr = nullptr;
-  cudaError_t e = cudaHostGetDevicePointer(reinterpret_cast<void**>(&dptr), buf, 0);
-  if (e == cudaSuccess) {
-    k_to_host<<<1, 256, 0, s>>>(dptr, static_cast<const uint32_t*>(dev_src), (uint32_t)(bytes / 4));
-    e = cudaGetLastError();
-  }
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  if (e == cudaSuccess) memcpy(host_dst, buf, bytes);
-  {
-    std::lock_guard<std::mutex> lk(g_mapped_mu);
-    g_mapped_free[dev].push_back(buf);
-  }
-  if (e != cudaSuccess) {
-    set_cuda_error(e);
-    return YQ_ERR_CUDA;
-  }
+  MappedWords m;
+  YQ_TRY(m.acquire());
+  k_to_host<<<1, 256, 0, s>>>(m.device, static_cast<const uint32_t*>(dev_src), (uint32_t)(bytes / 4));
+  YQ_TRY_CUDA(cudaGetLastError());
+  YQ_TRY_CUDA(cudaStreamSynchronize(s));
+  memcpy(host_dst, m.host, bytes);
   return YQ_OK;
 }
 

@@ -80,6 +80,21 @@ int h2d_async(void* dst, const void* src, size_t bytes, cudaStream_t s);
 // small reads bypass the copy engines (runtime.cu).
 int d2h_sync(void* host_dst, const void* dev_src, size_t bytes, cudaStream_t s);
 
+// 64 KB of mapped pinned host memory of the current device, for words a kernel
+// leaves for the host itself (stores through `device`, then
+// __threadfence_system()): read `host` after synchronising the stream, and not
+// destroyed before that (the next call would share the buffer).
+struct MappedWords {
+  uint32_t* host = nullptr;
+  uint32_t* device = nullptr;
+  int dev = -1;
+  MappedWords() = default;
+  MappedWords(const MappedWords&) = delete;
+  MappedWords& operator=(const MappedWords&) = delete;
+  int acquire();
+  ~MappedWords();
+};
+
 int sm_count();
 
 // Per-device, thread-safe launch settings (runtime.cu): raise `kernel`'s
