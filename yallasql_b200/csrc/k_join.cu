@@ -77,7 +77,8 @@ struct JoinParams {
   unsigned long long* total;
   uint32_t* err;
   const uint32_t* counts;  // typed nested loop: matches per left row, counted up front (null: count in the kernel)
-  char* vdst[2];           // typed nested loop writing the condition's own values: left / right output (or null)
+  char* vdst[2];           // typed nested loop writing values from registers: left / right output (or null)
+  const char* vsrc;        // and the left output's column
 };
 
 
@@ -759,8 +760,8 @@ __global__ void k_join_count_sorted(const T* __restrict__ lcol, uint32_t L, cons
 // ascending) as k_join_nested.
 //
 // Each left row's matches are compacted into a shared-memory ring of two runs
-// of 512 bytes, whose entries sit where their output positions lie in a 16-byte
-// word; a full run leaves 16 bytes a lane. Storing each match as it is found
+// (512 bytes of values, 256 row ids), whose entries sit where their output
+// positions lie in a 16-byte word; a full run of values leaves 16 bytes a lane. Storing each match as it is found
 // (64 unaligned bytes a store for a comparison that half the pairs pass) held
 // the kernel to 2.3 TB/s of output: 20K x 20K INT32 rows under <, 199M pairs,
 // 677 us for the writing alone. A row's ring is looked at once for kNtUnroll
@@ -775,31 +776,110 @@ constexpr uint32_t kNtTile = (kNtBlock / 32) * kNtRows;  // left rows per block
 constexpr int kNtCountUnroll = 16;  // right values a lane loads ahead while counting,
 constexpr int kNtUnroll = 4;        // and while it writes
 
-// Outputs [pb + i0, pb + i1) of left row l: right rows rows[i0 .. i1) of a run.
-__device__ __noinline__ void write_rows(const JoinParams& J, uint32_t l, unsigned long long pb, uint32_t i0,
-                                        uint32_t i1, const uint32_t* rows) {
+// Cells [pb, pb + cells) of one output of left row l, moved in pieces of V
+// (`pieces` a cell): a lane has four loads in flight before its first store.
+// Bound by the latency of these loads where few left rows meet a long right
+// side (a warp holds four left rows): 500 x 40,000 INT32 rows under <, two other
+// 4-byte columns written, 0.74 ms; one load and store at a time, by runs of 128,
+// 2.30; every match stored as it is found 1.27. 20-byte texts 1.60, 2.5 and 2.0.
+template <typename V>
+__device__ __forceinline__ void write_cells(const char* src_, char* dst_, bool right, uint32_t pieces, uint32_t l,
+                                            unsigned long long pb, uint32_t cells, const uint32_t* rows) {
+  constexpr int K = 4;
+  const V* const src = reinterpret_cast<const V*>(src_);
+  V* const dst = reinterpret_cast<V*>(dst_) + pb * pieces;
   const uint32_t lane = threadIdx.x & 31;
-  if (pb + i1 > J.capacity) i1 = pb >= J.capacity ? 0u : (uint32_t)(J.capacity - pb);
+  V v[K];
+  if (pieces == 1) {
+    if (!right) {  // one value for all of them
+      const V mine = __ldg(src + l);
+#pragma unroll
+      for (int k = 0; k < K; ++k) v[k] = mine;
+    }
+    for (uint32_t x0 = lane; x0 < cells; x0 += 32 * K) {
+      if (right)
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+          if (x0 + 32 * k < cells) v[k] = __ldg(src + rows[x0 + 32 * k]);
+#pragma unroll
+      for (int k = 0; k < K; ++k)
+        if (x0 + 32 * k < cells) dst[x0 + 32 * k] = v[k];
+    }
+    return;
+  }
+  if constexpr (sizeof(V) == 4 || sizeof(V) == 16) {
+    // piece x of the run is piece x % pieces of cell x / pieces, kept by steps of 32
+    if (cells == 0) return;
+    const uint32_t n = cells * pieces, qs = 32u / pieces, rs = 32u - qs * pieces, width = pieces * sizeof(V);
+    uint32_t c = lane / pieces, r = lane - c * pieces;
+    auto pass = [&](uint32_t x0, auto full) {
+      constexpr bool FULL = decltype(full)::value;
+      uint32_t row[K], piece[K];
+#pragma unroll
+      for (int k = 0; k < K; ++k) {
+        row[k] = right ? rows[FULL || x0 + 32 * k < n ? c : 0u] : l;  // past the end: the first cell again
+        piece[k] = r;
+        c += qs;
+        r += rs;
+        const bool carry = r >= pieces;
+        r -= carry ? pieces : 0u;
+        c += carry ? 1u : 0u;
+      }
+#pragma unroll
+      for (int k = 0; k < K; ++k)
+        v[k] = __ldg(reinterpret_cast<const V*>(src_ + (unsigned long long)row[k] * width) + piece[k]);
+#pragma unroll
+      for (int k = 0; k < K; ++k)
+        if (FULL || x0 + 32 * k < n) dst[x0 + 32 * k] = v[k];
+    };
+    uint32_t x0 = 0;
+    for (; x0 + 32 * K <= n; x0 += 32 * K) pass(x0 + lane, std::true_type{});
+    if (x0 < n) pass(x0 + lane, std::false_type{});
+  }
+}
+
+// Outputs [pb, pb + n) of left row l: right rows rows[0 .. n).
+__device__ __forceinline__ void write_rows(const JoinParams& J, uint32_t l, unsigned long long pb, uint32_t n,
+                                           const uint32_t* rows) {
+  const uint32_t lane = threadIdx.x & 31;
+  if (pb >= J.capacity) return;
+  if (pb + n > J.capacity) n = (uint32_t)(J.capacity - pb);
   if (J.nout == 0) {
-    for (uint32_t i = i0 + lane; i < i1; i += 32) {
+    for (uint32_t i = lane; i < n; i += 32) {
       J.out_left[pb + i] = l;
       J.out_right[pb + i] = rows[i];
     }
     return;
   }
+#pragma unroll 1
   for (int o = 0; o < J.nout; ++o) {
     const JOut& w = J.out[o];
-    for (uint32_t i = i0 + lane; i < i1; i += 32) write_col(w, pb + i, w.side ? rows[i] : l);
+    const bool right = w.side != 0;
+    if (w.width == 4) write_cells<uint32_t>(w.src, w.dst, right, 1u, l, pb, n, rows);
+    else if (w.width == 8) write_cells<unsigned long long>(w.src, w.dst, right, 1u, l, pb, n, rows);
+    else if (w.width == 1) write_cells<uint8_t>(w.src, w.dst, right, 1u, l, pb, n, rows);
+    else if (((w.width | reinterpret_cast<uintptr_t>(w.dst) | reinterpret_cast<uintptr_t>(w.src)) & 15) == 0)
+      write_cells<uint4>(w.src, w.dst, right, (uint32_t)w.width / 16u, l, pb, n, rows);
+    else write_cells<uint32_t>(w.src, w.dst, right, (uint32_t)w.width / 4u, l, pb, n, rows);
+    if (!w.dst_nulls) continue;
+    if (w.src_nulls)
+      write_cells<uint8_t>(reinterpret_cast<const char*>(w.src_nulls), reinterpret_cast<char*>(w.dst_nulls), right, 1u,
+                           l, pb, n, rows);
+    else
+      for (uint32_t i = lane; i < n; i += 32) w.dst_nulls[pb + i] = 0;
   }
 }
 
-// VALUES: the outputs are the condition's own two columns (SELECT a.x, b.y ...
-// WHERE a.x < b.y), written from registers; otherwise the runs hold row ids.
+// VALUES: the outputs are the condition's right column and a left column as wide
+// (SELECT a.x, b.y ... WHERE a.x < b.y, a.x or another column of a), or one of
+// them, written from registers; otherwise the runs hold row ids. Their writer
+// stands once, behind the comparisons: called out of line from each row's place
+// it cost the kernel 128 registers a thread, 16 warps an SM.
 template <typename T, int OP, bool VALUES>
 __global__ void __launch_bounds__(kNtBlock) k_join_nested_typed(const __grid_constant__ JoinParams J) {
   using B = typename std::conditional<VALUES, T, uint32_t>::type;
   constexpr uint32_t VEC = 16 / sizeof(B);
-  constexpr uint32_t RUN = 32 * VEC;
+  constexpr uint32_t RUN = VALUES ? 32 * VEC : 256;  // row ids: what an output's set-up costs, over more cells
   constexpr uint32_t RING = RUN * (RUN < 32u * kNtUnroll ? 4 : 2);  // a batch of matches crosses less than half of it
   static_assert(RING >= RUN + 32 * kNtUnroll, "a batch must not overtake the run being written");
   __shared__ __align__(16) B s_buf[kNtBlock / 32][kNtRows][RING];
@@ -816,11 +896,15 @@ __global__ void __launch_bounds__(kNtBlock) k_join_nested_typed(const __grid_con
   const T* rcol = reinterpret_cast<const T*>(J.cond[0].r.data);
   const uint32_t l0 = tile * kNtTile + warp * kNtRows;
   T lv[kNtRows];
+  T lw[kNtRows];  // VALUES: the left output's cells
   bool lok[kNtRows];
 #pragma unroll
   for (int i = 0; i < kNtRows; ++i) {
     lok[i] = l0 + i < J.L;
     lv[i] = lok[i] ? __ldg(lcol + l0 + i) : T(0);
+    lw[i] = T(0);
+    if constexpr (VALUES)
+      if (J.vdst[0] && lok[i]) lw[i] = __ldg(reinterpret_cast<const T*>(J.vsrc) + l0 + i);
   }
   // pass 1: matches per left row (counted up front from the sorted right
   // side when J.counts is given, else here over the whole right side)
@@ -844,10 +928,14 @@ __global__ void __launch_bounds__(kNtBlock) k_join_nested_typed(const __grid_con
 #pragma unroll
         for (int i = 0; i < kNtRows; ++i) cnt[i] += nl_cmp<T, OP>(lv[i], rv[u]) ? 1u : 0u;
     }
-    for (uint32_t r = whole + lane; r < J.R; r += 32) {
-      const T rv = __ldg(rcol + r);
+    for (uint32_t r0 = whole + lane; r0 < J.R; r0 += 32 * kNtUnroll) {
+      T rv[kNtUnroll];
 #pragma unroll
-      for (int i = 0; i < kNtRows; ++i) cnt[i] += nl_cmp<T, OP>(lv[i], rv) ? 1u : 0u;
+      for (int u = 0; u < kNtUnroll; ++u) rv[u] = r0 + u * 32 < J.R ? __ldg(rcol + r0 + u * 32) : T(0);
+#pragma unroll
+      for (int u = 0; u < kNtUnroll; ++u)
+#pragma unroll
+        for (int i = 0; i < kNtRows; ++i) cnt[i] += r0 + u * 32 < J.R && nl_cmp<T, OP>(lv[i], rv[u]) ? 1u : 0u;
     }
 #pragma unroll
     for (int i = 0; i < kNtRows; ++i)
@@ -899,7 +987,7 @@ __global__ void __launch_bounds__(kNtBlock) k_join_nested_typed(const __grid_con
     any |= lok[i];
   }
   if (!any) return;
-  // entries [head, n) of row i, all within one run
+  // VALUES: entries [head, n) of row i, all within one run
   auto flush = [&](int i, uint32_t n) {
     __syncwarp();
     const uint32_t r0 = head[i] & ~(RUN - 1u);  // the run's first entry
@@ -910,22 +998,45 @@ __global__ void __launch_bounds__(kNtBlock) k_join_nested_typed(const __grid_con
         if (vl) {
           T x[VEC];
 #pragma unroll
-          for (uint32_t v = 0; v < VEC; ++v) x[v] = lv[i];
+          for (uint32_t v = 0; v < VEC; ++v) x[v] = lw[i];
           *reinterpret_cast<uint4*>(vl + pos + lane * VEC) = *reinterpret_cast<const uint4*>(x);
         }
         if (vr) *reinterpret_cast<uint4*>(vr + pos + lane * VEC) = *reinterpret_cast<const uint4*>(buf + lane * VEC);
       } else {
         for (uint32_t x = head[i] - r0 + lane; x < n - r0; x += 32)
           if (pos + x < J.capacity) {
-            if (vl) vl[pos + x] = lv[i];
+            if (vl) vl[pos + x] = lw[i];
             if (vr) vr[pos + x] = buf[x];
           }
       }
-    } else {
-      write_rows(J, l0 + i, pos, head[i] - r0, n - r0, buf);
     }
     __syncwarp();
     head[i] = n;
+  };
+  // Row ids: the runs that are full, and on the last batch all that is left.
+  auto flush_rows = [&](bool last) {
+    __syncwarp();
+    for (;;) {
+      uint32_t h = 0u, n = 0u;
+      unsigned long long p = 0ull;
+      int row = -1;
+#pragma unroll
+      for (int i = kNtRows - 1; i >= 0; --i) {
+        const uint32_t end = (head[i] | (RUN - 1u)) + 1u;
+        if (fill[i] >= end || (last && fill[i] > head[i])) {
+          row = i;
+          h = head[i];
+          n = min(fill[i], end);
+          p = p0[i];
+        }
+      }
+      if (row < 0) break;
+      write_rows(J, l0 + row, p + h, n - h, reinterpret_cast<const uint32_t*>(s_buf[warp][row]) + (h & (RING - 1u)));
+#pragma unroll
+      for (int i = 0; i < kNtRows; ++i)
+        if (i == row) head[i] = n;
+    }
+    __syncwarp();
   };
   // kNtUnroll right values a lane against every row; FULL: all of them exist
   auto batch = [&](uint32_t r0, auto full) {
@@ -947,15 +1058,28 @@ __global__ void __launch_bounds__(kNtBlock) k_join_nested_typed(const __grid_con
         }
         fill[i] += __popc(bal);
       }
-      for (uint32_t run = (before | (RUN - 1u)) + 1u; run <= fill[i]; run += RUN) flush(i, run);
+      if constexpr (VALUES)
+        for (uint32_t run = (before | (RUN - 1u)) + 1u; run <= fill[i]; run += RUN) flush(i, run);
     }
   };
   uint32_t r0 = lane;
-  for (; r0 - lane + 32 * kNtUnroll <= J.R; r0 += 32 * kNtUnroll) batch(r0, std::true_type{});
-  if (r0 - lane < J.R) batch(r0, std::false_type{});
+  for (; r0 - lane + 32 * kNtUnroll <= J.R; r0 += 32 * kNtUnroll) {
+    batch(r0, std::true_type{});
+    if constexpr (!VALUES) {
+      bool due = false;
 #pragma unroll
-  for (int i = 0; i < kNtRows; ++i)
-    if (lok[i] && fill[i] > head[i]) flush(i, fill[i]);
+      for (int i = 0; i < kNtRows; ++i) due |= fill[i] > (head[i] | (RUN - 1u));
+      if (due) flush_rows(false);
+    }
+  }
+  if (r0 - lane < J.R) batch(r0, std::false_type{});
+  if constexpr (VALUES) {
+#pragma unroll
+    for (int i = 0; i < kNtRows; ++i)
+      if (lok[i] && fill[i] > head[i]) flush(i, fill[i]);
+  } else {
+    flush_rows(true);
+  }
 }
 
 template <typename T, bool VALUES>
@@ -973,14 +1097,15 @@ static int launch_nested_typed_op(int op, unsigned grid, const JoinParams& J, cu
 
 template <typename T>
 static int launch_nested_typed(int op, unsigned grid, JoinParams J, cudaStream_t s) {
-  // the outputs are the condition's own left and right columns, each at most once
+  // a left column of the condition's width and the condition's right column, each at most once
   bool values = J.nout >= 1 && J.nout <= 2;
   J.vdst[0] = J.vdst[1] = nullptr;
   for (int o = 0; o < J.nout && values; ++o) {
     const JOut& w = J.out[o];
-    const JCol& cc = w.side ? J.cond[0].r : J.cond[0].l;
-    values = w.src == cc.data && w.width == (int)sizeof(T) && !w.dst_nulls && !J.vdst[w.side];
-    if (values) J.vdst[w.side] = w.dst;
+    values = w.width == (int)sizeof(T) && !w.dst_nulls && !J.vdst[w.side != 0] && (!w.side || w.src == J.cond[0].r.data);
+    if (!values) break;
+    J.vdst[w.side != 0] = w.dst;
+    if (!w.side) J.vsrc = w.src;
   }
   return values ? launch_nested_typed_op<T, true>(op, grid, J, s) : launch_nested_typed_op<T, false>(op, grid, J, s);
 }
