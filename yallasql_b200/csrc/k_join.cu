@@ -1358,27 +1358,36 @@ static int join_impl(const yq_batch* left, const yq_batch* right, const yq_join_
       eq_float ? kHashMaxRows : ((unsigned long long)J.L * J.R > (1ull << 32) ? kSortedMinRows : kTableRows);
   const size_t eq_sort_bytes = J.eq >= 0 && J.R > table_rows && J.cond[J.eq].r.type != YQ_BOOL
                                    ? join_sort_bytes(J.R, J.cond[J.eq].r.nulls != nullptr) : 0;
-  const bool use_sorted = eq_sort_bytes != 0;
-  const bool use_hash = J.eq >= 0 && !use_sorted && J.R <= kHashMaxRows;
-  const uint32_t nbuckets = use_hash ? pow2_at_least(J.R) : 0u;
   const JCond& t0 = J.cond[0];
-  const bool typed = !use_hash && !use_sorted && J.ncond == 1 && J.ngroups == 1 && t0.l.type == t0.r.type && !t0.l.nulls &&
-                     !t0.r.nulls && t0.l.width == t0.r.width && t0.cmp != YQ_EQ &&
-                     (t0.l.type == YQ_INT32 || t0.l.type == YQ_FLOAT32 || t0.l.type == YQ_INT64 ||
-                      t0.l.type == YQ_DATETIME || t0.l.type == YQ_FLOAT64);
-  const uint32_t ntiles = ceil_div<uint32_t>(J.L, use_hash || use_sorted ? kJoinTile : (typed ? kNtTile : kNlTile));
-  const size_t count_bytes = typed && counts_first(J.L, J.R) ? join_sort_bytes(J.R, false) : 0;
-  const bool count_first = count_bytes != 0;  // else (a right side too long to sort) the kernel counts
-  WsSize w;
-  w.add<uint32_t>(nbuckets + 1);
-  w.add<unsigned long long>(use_hash ? J.R : 1);
-  w.add<uint32_t>(use_hash ? J.R : 1);
-  w.add<unsigned long long>((size_t)ntiles + 3);
-  w.add<uint32_t>(8);
-  if (count_first) count_ws_layout(J.L, J.R, count_bytes, w);
-  if (use_sorted) sorted_ws_layout(J.R, eq_sort_bytes, w);
+  bool use_sorted = eq_sort_bytes != 0, use_hash, typed, count_first;
+  uint32_t nbuckets, ntiles;
+  size_t count_bytes;
   Workspace ws;
-  YQ_TRY(ws.acquire(workspace, workspace_bytes, w.total(), s));
+  for (;;) {
+    use_hash = J.eq >= 0 && !use_sorted && J.R <= kHashMaxRows;
+    nbuckets = use_hash ? pow2_at_least(J.R) : 0u;
+    typed = !use_hash && !use_sorted && J.ncond == 1 && J.ngroups == 1 && t0.l.type == t0.r.type && !t0.l.nulls &&
+                       !t0.r.nulls && t0.l.width == t0.r.width && t0.cmp != YQ_EQ &&
+                       (t0.l.type == YQ_INT32 || t0.l.type == YQ_FLOAT32 || t0.l.type == YQ_INT64 ||
+                        t0.l.type == YQ_DATETIME || t0.l.type == YQ_FLOAT64);
+    ntiles = ceil_div<uint32_t>(J.L, use_hash || use_sorted ? kJoinTile : (typed ? kNtTile : kNlTile));
+    count_bytes = typed && counts_first(J.L, J.R) ? join_sort_bytes(J.R, false) : 0;
+    count_first = count_bytes != 0;  // else (a right side too long to sort) the kernel counts
+    WsSize w;
+    w.add<uint32_t>(nbuckets + 1);
+    w.add<unsigned long long>(use_hash ? J.R : 1);
+    w.add<uint32_t>(use_hash ? J.R : 1);
+    w.add<unsigned long long>((size_t)ntiles + 3);
+    w.add<uint32_t>(8);
+    if (count_first) count_ws_layout(J.L, J.R, count_bytes, w);
+    if (use_sorted) sorted_ws_layout(J.R, eq_sort_bytes, w);
+    const int st = ws.acquire(workspace, workspace_bytes, w.total(), s);
+    if (st == YQ_OK) break;
+    // no room for the sorted table (up to 70 bytes a right row): the forms that
+    // need a few words a tile give the same pairs
+    if (!use_sorted || !(workspace ? workspace_bytes < w.total() : st == YQ_ERR_ALLOC)) return st;
+    use_sorted = false;
+  }
   uint32_t* d_bstart = ws.take<uint32_t>(nbuckets + 1);
   unsigned long long* d_hkeys = ws.take<unsigned long long>(use_hash ? J.R : 1);
   uint32_t* d_hrows = ws.take<uint32_t>(use_hash ? J.R : 1);

@@ -161,9 +161,11 @@ int d2h_sync(void* host_dst, const void* dev_src, size_t bytes, cudaStream_t s) 
 // next synchronisation, so each call that ends with a read-back had its
 // workspace mapped anew: 0.44 ms for a 16K-row filter + aggregate that runs
 // 40 us on the GPU, 13 ms for a 32M-row GROUP BY's 1 GB. This pool keeps up to
-// 1/64 of the device's memory (2.8 GB of 180) across synchronisations, hands
-// back what is above that, and everything when the device runs out or
-// yq_workspace_trim is called. The driver orders reuse between streams.
+// 1/64 of the device's memory (2.8 GB of 180) across synchronisations and hands
+// back what is above that, and all that no call uses when yq_workspace_trim is
+// called. Another allocation of the process that finds the device full gets a
+// pool's idle memory from the driver (tests/test_workspace_pool_gpu.py). The
+// driver orders reuse between streams.
 namespace {
 constexpr size_t kPoolShare = 64;
 std::mutex g_pool_mu;
@@ -208,6 +210,7 @@ int pool_alloc(void** p, size_t bytes, cudaStream_t s) {
   }
   if (e != cudaSuccess) {
     set_cuda_error(e);
+    cudaGetLastError();  // reported here: a later launch check must not find it
     return YQ_ERR_ALLOC;
   }
   return YQ_OK;
