@@ -1147,9 +1147,10 @@ static bool hashable(int t) {
   return t == YQ_INT32 || t == YQ_INT64 || t == YQ_DATETIME || t == YQ_FLOAT32 || t == YQ_FLOAT64 || t == YQ_BOOL;
 }
 
+// (2^31, the greatest there is, for more: sizes are asked for any row count)
 static uint32_t pow2_at_least(uint32_t x) {
   uint32_t p = 16;
-  while (p < x) p <<= 1;
+  while (p < x && p < (1u << 31)) p <<= 1;
   return p;
 }
 
@@ -1507,7 +1508,8 @@ size_t yq_join_workspace_size(uint32_t left_rows, uint32_t right_rows) {
   w.add<uint32_t>(8);
   WsSize sorted = w;
   if (counts_first(left_rows, right_rows)) count_ws_layout(left_rows, right_rows, join_sort_bytes(right_rows, false), w);
-  if (right_rows > kSortedMinRows) sorted_ws_layout(right_rows, join_sort_bytes(right_rows, true), sorted);
+  const size_t eq_sort_bytes = right_rows > kSortedMinRows ? join_sort_bytes(right_rows, true) : 0;
+  if (eq_sort_bytes) sorted_ws_layout(right_rows, eq_sort_bytes, sorted);  // (0: more rows than the sort takes)
   return w.total() > sorted.total() ? w.total() : sorted.total();
 }
 
