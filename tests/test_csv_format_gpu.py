@@ -1,6 +1,7 @@
 """CSV writer at the limits of its one-pass form: a buffer of exactly the bound,
 the longest cell of every type, and text past the 32-bit offsets."""
 import ctypes as C
+import json
 
 import numpy as np
 import pytest
@@ -120,3 +121,22 @@ def test_failed_allocation_of_the_text(cuda, monkeypatch):
         with pytest.raises(torch.cuda.OutOfMemoryError, match="no room"):
             ops.csv_format(batch)
     assert torch.equal(ops.csv_format(batch).cpu(), want)
+
+
+def test_profiled_bytes_hold_the_text(cuda, yq):
+    """The write kernel's profiled bytes are the cells in and the text out, also
+    where the text's length is read after the launch."""
+    rows = 1000
+    batch = ops.DeviceBatch([col(np.full(rows, 123456, np.int32), A.INT32)])
+    bc, keep = batch.c()
+    bound = int(yq.yq_csv_format_bound(C.byref(bc)))
+    for room in (bound, rows * 7):  # one pass; the length first
+        yq.yq_profile_enable(1)
+        yq.yq_profile_read(None, 0, 1)
+        st, n, text, _ = format_into(yq, batch, room)
+        buf = C.create_string_buffer(1 << 14)
+        yq.yq_profile_read(buf, len(buf), 1)
+        yq.yq_profile_enable(0)
+        assert (st, n) == (A.OK, rows * 7)
+        got = json.loads(buf.value.decode())["csv_format_write"]
+        assert got["launches"] == 1 and got["units"] == rows * 4 + rows * 7

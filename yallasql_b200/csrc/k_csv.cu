@@ -777,6 +777,7 @@ static int csv_format_impl(const yq_batch* batch, uint8_t* out, uint64_t capacit
   if (fits) {
     YQ_TRY(d2h_sync(&total, end + rows - 1, sizeof(total), s));
     *bytes = total;
+    prof_add("csv_format_write", (double)total);  // its length was not known at the launch
     if (total > capacity) return YQ_ERR_CAPACITY;
   }
   return YQ_OK;

@@ -262,6 +262,16 @@ void prof_end(cudaStream_t s) {
   cudaEventRecord(r.b, s);
 }
 
+void prof_add(const char* tag, double units) {
+  std::lock_guard<std::mutex> lk(g_prof_mu);
+  if (!g_prof_on) return;
+  for (size_t i = g_prof.size(); i-- > 0;)
+    if (g_prof[i].tag == tag) {
+      g_prof[i].units += units;
+      return;
+    }
+}
+
 int sm_count() {
   static std::atomic<int> cached[64] = {};
   int dev = 0;

@@ -38,6 +38,7 @@ void count_launch(int n = 1);
 // event pair on the launch stream around each tagged launch.
 void prof_begin(const char* tag, cudaStream_t s, double units);
 void prof_end(cudaStream_t s);
+void prof_add(const char* tag, double units);  // to the latest record of this tag
 struct ProfScope {
   cudaStream_t s;
   ProfScope(const char* tag, cudaStream_t st, double units = 0.0) : s(st) { prof_begin(tag, st, units); }
