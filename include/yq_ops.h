@@ -674,7 +674,7 @@ size_t yq_csv_parse_workspace_size(uint32_t records);
  * dropped, order kept (csv-parser's IGNORE_ROW policy); *rows = rows kept.
  * Synchronises `stream`. Cells that fail to convert: YQ_ERR_INVALID_ARG with
  * *error filled, every other cell still converted. Dropping rows allocates
- * stream-ordered temporaries (cudaMallocAsync) even with a workspace. */
+ * stream-ordered temporaries even with a workspace. */
 int yq_csv_parse(const uint8_t* data, uint64_t nbytes, const uint32_t* record_starts, uint32_t records,
                  const int32_t* field_column, int32_t nfields, yq_column* out, int32_t ncols, uint32_t* rows,
                  yq_csv_error* error, void* workspace, size_t workspace_bytes, void* stream);
@@ -710,8 +710,9 @@ int yq_csv_format_alloc(const yq_batch* batch, yq_alloc_fn alloc, void* alloc_ct
 /* Number of SMs of the current device (cached per device). */
 int yq_device_sm_count(void);
 /* Gives the memory that the current device's workspace pool keeps and no call
- * uses back to the driver (the library does so itself when an allocation
- * fails; a host that allocates elsewhere calls it when it runs out). */
+ * uses back to the driver: blocks whose stream-ordered free has been reached.
+ * Other allocations of the process that find the device full get such blocks
+ * from the driver without this call; other processes do not. */
 int yq_workspace_trim(void);
 /* Kernel launches issued by this library on this process (for accounting). */
 uint64_t yq_launch_count(void);

@@ -764,12 +764,12 @@ static std::unique_ptr<Batch> collect_runs(Operator* child, CacheManager& cache,
 }
 
 // ----------------------------------------------------------- OrderOperator
-// Every child batch becomes a run; yq_order_by sorts the runs (segmented radix
-// sort), merges them pairwise by merge path until one remains and gathers the
-// rows (OrderOperator::firstPass / merge_all_sorted, order_operator.hpp:89-193).
+// Every child batch becomes a run; yq_order_by gives the order of the runs
+// sorted and merged, by one stable sort of all of them, and gathers the rows
+// (OrderOperator::firstPass / merge_all_sorted, order_operator.hpp:89-193).
 // The reference sorts by its first ORDER BY key only (`orders[0]`,
 // order_operator.hpp:277); here every key counts: with more than one key (or a
-// text key longer than the merge path's 32-byte key) the concatenated runs are
+// text key beyond yq_order_by's 32 bytes) the concatenated runs are
 // sorted at once by all keys (stable LSD over the keys, yq_sort_indices_multi)
 // and gathered.
 class OrderOperator final : public Operator {
@@ -806,7 +806,7 @@ class OrderOperator final : public Operator {
     yq_batch ib{av.data(), (int32_t)av.size(), (uint32_t)total};
     yq_batch ob{rv.data(), (int32_t)rv.size(), (uint32_t)total};
     int st = YQ_ERR_UNSUPPORTED;
-    if (keys_.size() == 1)  // sort every run, merge (key words, row id) level by level, gather once
+    if (keys_.size() == 1)  // one stable sort of all runs, every column gathered once
       st = yq_order_by(&ib, keys_[0], desc_[0], nulls_first_[0], offs.data(), (int32_t)offs.size() - 1, &ob, nullptr,
                        0, s);
     if (st == YQ_ERR_UNSUPPORTED) {

@@ -12,8 +12,8 @@
 //   ProjectionOperator (projection_operator.hpp)      ProjectionOperator -> yq_filter_project
 //   AggregateOperator (aggregate_operator.hpp)        AggregateOperator -> yq_filter_aggregate
 //                                                     (absorbs a child FilterOperator's predicate)
-//   OrderOperator (order_operator.hpp/.cpp)           OrderOperator -> yq_sort_segments + yq_gather
-//                                                     + yq_merge_pass per level
+//   OrderOperator (order_operator.hpp/.cpp)           OrderOperator -> yq_order_by (one key),
+//                                                     yq_sort_indices_multi + yq_gather (several)
 //   JoinOperator (join_operator.hpp)                  JoinOperator -> yq_join_project
 //   CrossProductOperator (cross_product_operator.hpp) CrossProductOperator -> yq_join_project (no condition)
 #pragma once

@@ -542,8 +542,9 @@ class OrderByRuns:
     (the order that sorted and merged runs would have), then every column
     gathered once by the sorted row ids (OrderOperator::firstPass +
     merge_all_sorted, order_operator.hpp:89-193 / order_operator.cpp:14-220).
-    The workspace is allocated once and reused across calls; `two_level`
-    sizes it for the packed rows through which large tables are gathered."""
+    The workspace is allocated once and reused across calls; `two_level` (pack,
+    then gather) sizes it for the packed rows through which large tables are
+    gathered."""
 
     def __init__(self, batch: DeviceBatch, key: int, offsets: list[int], two_level: bool = True):
         self.key, self.offsets, self.n = key, list(offsets), batch.rows

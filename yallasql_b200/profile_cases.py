@@ -4,10 +4,11 @@
     python -m yallasql_b200.profile_cases join     # 30M-row fact table joined to the 2,556-row date table + SUM
     python -m yallasql_b200.profile_cases order    # 16M rows (key f32, id, 16-byte txt, date), 116,480-row runs
     python -m yallasql_b200.profile_cases cross    # 20K x 20K cross product with < (198M output pairs)
+    python -m yallasql_b200.profile_cases columns  # 10K x 10K under <, another column of each side written (50M pairs)
     python -m yallasql_b200.profile_cases csv      # 4M-row sales table as CSV text (~205 MB): index + parse + write
     python -m yallasql_b200.profile_cases group    # 16M sales rows GROUP BY discount: COUNT(*), SUM, AVG, MIN, MAX
 
-An optional second argument sets the row count (rows per side for cross).
+An optional second argument sets the row count (rows per side for cross and columns).
 
 The inputs are larger than L2 (so DRAM counters mean something) and hold a few
 GB of device memory at most; every case runs its operators once and exits.
@@ -78,6 +79,15 @@ def cross_case(rows: int = 20_000) -> None:
     torch.cuda.synchronize()
 
 
+def columns_case(rows: int = 10_000) -> None:
+    x, y = datagen.cross_tables(rows, seed=2)
+    ids = np.arange(rows, dtype=np.int32)
+    ops.join_project(ops.DeviceBatch([_dev(x, A.INT32), _dev(ids, A.INT32)]),
+                     ops.DeviceBatch([_dev(y, A.INT32), _dev(ids, A.INT32)]), [(0, 0, A.LT)], [(0, 1), (1, 1)],
+                     capacity=rows * rows * 3 // 5)
+    torch.cuda.synchronize()
+
+
 def csv_case(rows: int = 4_000_000) -> None:
     _, body = datagen.sales_csv(rows, seed=0)
     text = torch.from_numpy(body).cuda()
@@ -94,7 +104,8 @@ def group_case(rows: int = 16_000_000) -> None:
     torch.cuda.synchronize()
 
 
-CASES = {"filter": filter_case, "join": join_case, "order": order_case, "cross": cross_case, "csv": csv_case,
+CASES = {"filter": filter_case, "join": join_case, "order": order_case, "cross": cross_case,
+         "columns": columns_case, "csv": csv_case,
          "group": group_case}
 
 if __name__ == "__main__":
