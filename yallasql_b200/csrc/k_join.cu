@@ -399,6 +399,7 @@ struct SortedJoin {
   uint4* slots;          // {key, first sorted position (kNoSlot: empty), run}
   uint32_t nslots;       // power of two, >= 1.5 R
   uint32_t rows;         // R
+  uint32_t tile_rows;    // left rows a block takes, at most kJoinTile
 };
 constexpr uint32_t kNoSlot = 0xffffffffu;
 constexpr uint32_t kOneRow = 0x80000000u;  // run field: the key's only row (row ids are below 2^30)
@@ -450,27 +451,28 @@ __global__ void __launch_bounds__(256) k_join_sorted_build(const __grid_constant
   }
 }
 
-// Matches of a thread's kJoinItems consecutive left rows: the number of rows of
+// Matches of a thread's ITEMS consecutive left rows: the number of rows of
 // each one's key, and where they are (a sorted position, or kOneRow and the
 // row). The first probe of every row goes out before any is looked at.
+template <int ITEMS>
 __device__ __forceinline__ void sorted_matches(const SortedJoin& S, const JCol& key, uint32_t l0, uint32_t L,
-                                               uint32_t (&where)[kJoinItems], uint32_t (&run)[kJoinItems]) {
-  uint64_t k[kJoinItems];
-  uint32_t h[kJoinItems], joins = 0u;
-  uint4 at[kJoinItems];
+                                               uint32_t (&where)[ITEMS], uint32_t (&run)[ITEMS]) {
+  uint64_t k[ITEMS];
+  uint32_t h[ITEMS], joins = 0u;
+  uint4 at[ITEMS];
 #pragma unroll
-  for (int i = 0; i < kJoinItems; ++i) {
+  for (int i = 0; i < ITEMS; ++i) {
     const uint32_t l = l0 + i < L ? l0 + i : L - 1u;
     if (l0 + i < L && key_joins(key, l)) joins |= 1u << i;
     k[i] = hash_key(key, l);
   }
 #pragma unroll
-  for (int i = 0; i < kJoinItems; ++i) {
+  for (int i = 0; i < ITEMS; ++i) {
     h[i] = hash_bucket(k[i], S.nslots);
     at[i] = __ldg(S.slots + h[i]);
   }
 #pragma unroll
-  for (int i = 0; i < kJoinItems; ++i) {
+  for (int i = 0; i < ITEMS; ++i) {
     where[i] = run[i] = 0u;
     if (!(joins >> i & 1u)) continue;
     auto mine = [&](const uint4& e) { return e.x == (uint32_t)k[i] && e.y == (uint32_t)(k[i] >> 32); };
@@ -503,10 +505,7 @@ __device__ __forceinline__ void write_col(const JOut& w, unsigned long long pos,
 
 constexpr uint32_t kSortedChunk = 2048;  // outputs resolved to (left, right) rows at a time
 
-// EQ_ONLY: the equality is the only condition, so a left row's matches are its
-// key's run. Otherwise the run's rows are candidates: a lane tests a short run
-// itself, the whole warp a long one.
-template <bool EQ_ONLY>
+// The equality is the only condition: a left row's matches are its key's run.
 __global__ void __launch_bounds__(kJoinBlock) k_join_sorted(const __grid_constant__ JoinParams J,
                                                             const __grid_constant__ SortedJoin S) {
   __shared__ uint32_t s_tile;
@@ -518,38 +517,15 @@ __global__ void __launch_bounds__(kJoinBlock) k_join_sorted(const __grid_constan
   if (threadIdx.x == 0) s_tile = atomicAdd(J.tile_counter, 1u);
   __syncthreads();
   const uint32_t tile = s_tile;
-  const uint32_t base = tile * kJoinTile;
-  const JCond& ec = J.cond[J.eq];
+  const uint32_t base = tile * S.tile_rows, end = min(J.L, base + S.tile_rows);
   const int lane = threadIdx.x & 31;
-  uint32_t first[kJoinItems], run[kJoinItems], cnt[kJoinItems], sum = 0;
-  sorted_matches(S, ec.l, base + threadIdx.x * kJoinItems, J.L, first, run);
-#pragma unroll
-  for (int k = 0; k < kJoinItems; ++k) cnt[k] = run[k];
-  if constexpr (!EQ_ONLY) {
-#pragma unroll 1
-    for (int k = 0; k < kJoinItems; ++k) {
-      const uint32_t l = base + threadIdx.x * kJoinItems + k;
-      cnt[k] = 0;
-      if (run[k] <= 32)
-        for (uint32_t x = 0; x < run[k]; ++x) cnt[k] += all_conds(J, l, match_row(S, first[k], x), J.eq) ? 1u : 0u;
-      for (uint32_t todo = __ballot_sync(0xffffffffu, run[k] > 32); todo; todo &= todo - 1) {
-        const int src = __ffs(todo) - 1;
-        const uint32_t n = __shfl_sync(0xffffffffu, run[k], src), f = __shfl_sync(0xffffffffu, first[k], src);
-        const uint32_t wl = __shfl_sync(0xffffffffu, l, src);
-        uint32_t c = 0;
-        for (uint32_t x = lane; x < ((n + 31u) & ~31u); x += 32) {
-          const bool m = x < n && all_conds(J, wl, match_row(S, f, x), J.eq);
-          c += __popc(__ballot_sync(0xffffffffu, m));
-        }
-        if (lane == src) cnt[k] = c;
-      }
-    }
-  }
+  uint32_t first[kJoinItems], run[kJoinItems], sum = 0;
+  sorted_matches<kJoinItems>(S, J.cond[J.eq].l, base + threadIdx.x * kJoinItems, end, first, run);
   unsigned long long wide = 0;  // the tile's pairs may exceed 32 bits (a hot key on both sides)
 #pragma unroll
   for (int k = 0; k < kJoinItems; ++k) {
-    wide += cnt[k];
-    sum += cnt[k];
+    wide += run[k];
+    sum += run[k];
   }
   const int huge = __syncthreads_or(wide > 0xfffffu);  // 256 sums below 2^20 fit a 32-bit scan
   unsigned long long total;
@@ -572,13 +548,13 @@ __global__ void __launch_bounds__(kJoinBlock) k_join_sorted(const __grid_constan
   const unsigned long long prefix = s_prefix;
   if (tile == gridDim.x - 1 && threadIdx.x == 0) *J.total = prefix + total;
   if (prefix >= J.capacity || total == 0) return;  // nothing of this tile is stored
-  if (EQ_ONLY && !huge) {
+  if (!huge) {
     uint32_t at = (uint32_t)excl;
 #pragma unroll
     for (int k = 0; k < kJoinItems; ++k) {
       s_off[threadIdx.x * kJoinItems + k] = at;
       s_first[threadIdx.x * kJoinItems + k] = first[k];
-      at += cnt[k];
+      at += run[k];
     }
     if (threadIdx.x == 0) s_off[kJoinTile] = (uint32_t)total;
     const unsigned long long room = J.capacity - prefix;
@@ -587,7 +563,7 @@ __global__ void __launch_bounds__(kJoinBlock) k_join_sorted(const __grid_constan
       const uint32_t n = min(kSortedChunk, n_out - c0);
       __syncthreads();
       for (uint32_t i = threadIdx.x; i < n; i += kJoinBlock) {
-        uint32_t lo = 0, hi = kJoinTile;  // the left row whose outputs hold position c0 + i
+        uint32_t lo = 0, hi = S.tile_rows;  // the left row whose outputs hold position c0 + i
         while (lo + 1 < hi) {
           const uint32_t mid = (lo + hi) >> 1;
           if (s_off[mid] <= c0 + i) lo = mid;
@@ -617,27 +593,106 @@ __global__ void __launch_bounds__(kJoinBlock) k_join_sorted(const __grid_constan
 #pragma unroll 1
   for (int k = 0; k < kJoinItems; ++k) {
     const uint32_t l = base + threadIdx.x * kJoinItems + k;
-    if (run[k] <= 32) {
-      for (uint32_t x = 0; x < run[k]; ++x) {
-        const uint32_t r = match_row(S, first[k], x);
-        if (EQ_ONLY || all_conds(J, l, r, J.eq)) emit_pair(J, pos++, l, r);
-      }
-    }
+    if (run[k] <= 32)
+      for (uint32_t x = 0; x < run[k]; ++x) emit_pair(J, pos++, l, match_row(S, first[k], x));
     for (uint32_t todo = __ballot_sync(0xffffffffu, run[k] > 32); todo; todo &= todo - 1) {
       const int src = __ffs(todo) - 1;
       const uint32_t n = __shfl_sync(0xffffffffu, run[k], src), f = __shfl_sync(0xffffffffu, first[k], src);
       const uint32_t wl = __shfl_sync(0xffffffffu, l, src);
-      unsigned long long wp = __shfl_sync(0xffffffffu, pos, src);
-      for (uint32_t x = lane; x < ((n + 31u) & ~31u); x += 32) {
-        const uint32_t r = x < n ? match_row(S, f, x) : 0u;
-        const bool m = x < n && (EQ_ONLY || all_conds(J, wl, r, J.eq));
-        const uint32_t bal = __ballot_sync(0xffffffffu, m);
-        if (m) emit_pair(J, wp + __popc(bal & lanemask_lt()), wl, r);
-        wp += __popc(bal);
-      }
-      if (lane == src) pos = wp;
+      const unsigned long long wp = __shfl_sync(0xffffffffu, pos, src);
+      for (uint32_t x = lane; x < n; x += 32) emit_pair(J, wp + x, wl, match_row(S, f, x));
+      if (lane == src) pos = wp + n;
     }
   }
+}
+
+// With further conditions the rows of a key's run are candidates. A block's
+// candidates form one sequence (left row by left row, right rows ascending, the
+// order of the output), cut into eight equal parts for its warps, so that a key
+// with many rows on both sides is shared by all of them: 3,000 left rows to
+// 20,000 right ones of one key and two more conditions took 246 ms with a warp
+// going through the long runs of its 128 left rows one after the other, 9.4 in
+// the nested loop.
+__global__ void __launch_bounds__(kJoinBlock) k_join_sorted_conds(const __grid_constant__ JoinParams J,
+                                                                  const __grid_constant__ SortedJoin S) {
+  constexpr int NW = kJoinBlock / 32;
+  __shared__ uint32_t s_tile;
+  __shared__ unsigned long long s_off[kJoinBlock + 1];  // first candidate of every left row
+  __shared__ uint32_t s_where[kJoinBlock];
+  __shared__ unsigned long long s_scan[2 * (NW + 1)];
+  __shared__ unsigned long long s_cnt[NW];
+  __shared__ unsigned long long s_prefix;
+  if (threadIdx.x == 0) s_tile = atomicAdd(J.tile_counter, 1u);
+  __syncthreads();
+  const uint32_t tile = s_tile;
+  const uint32_t base = tile * S.tile_rows, end = min(J.L, base + S.tile_rows);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned long long candidates;
+  {
+    uint32_t where[1], run[1];
+    sorted_matches<1>(S, J.cond[J.eq].l, base + threadIdx.x, end, where, run);
+    unsigned long long first = run[0], zero = 0, tz;
+    block_exclusive_sum2<kJoinBlock>(first, zero, s_scan, candidates, tz);
+    s_off[threadIdx.x] = first;
+    s_where[threadIdx.x] = where[0];
+    if (threadIdx.x == 0) s_off[kJoinBlock] = candidates;
+  }
+  __syncthreads();
+  const unsigned long long part = ((candidates + NW - 1) / NW + 31) & ~31ull;
+  const unsigned long long x0 = min(candidates, part * warp), x1 = min(candidates, x0 + part);
+  // The last row whose first candidate is at or before x (it has candidates: x is one), from row `lo` on.
+  auto row_of = [&](unsigned long long x, uint32_t lo) {
+    uint32_t hi = S.tile_rows;
+    while (lo + 1 < hi) {
+      const uint32_t mid = (lo + hi) >> 1;
+      if (s_off[mid] <= x) lo = mid;
+      else hi = mid;
+    }
+    return lo;
+  };
+  // f(matches of 32 candidates, left row, right row), in order
+  auto sweep = [&](auto f) {
+    if (x0 >= x1) return;
+    uint32_t row = row_of(x0, 0u);
+    for (unsigned long long x = x0; x < x1; x += 32) {
+      const unsigned long long mine = min(x + lane, x1 - 1), last = min(x + 31, x1 - 1);
+      const uint32_t at = last < s_off[row + 1] ? row : row_of(mine, row);
+      const uint32_t l = base + at, r = match_row(S, s_where[at], (uint32_t)(mine - s_off[at]));
+      const bool m = x + lane < x1 && all_conds(J, l, r, J.eq);
+      f(__ballot_sync(0xffffffffu, m), m, l, r);
+      row = __shfl_sync(0xffffffffu, at, 31);
+    }
+  };
+  unsigned long long count = 0;
+  sweep([&](uint32_t bal, bool, uint32_t, uint32_t) { count += __popc(bal); });
+  if (lane == 0) s_cnt[warp] = count;
+  __syncthreads();
+  unsigned long long total = 0, before = 0;
+#pragma unroll
+  for (int w = 0; w < NW; ++w) {
+    before += w < warp ? s_cnt[w] : 0ull;
+    total += s_cnt[w];
+  }
+  if (threadIdx.x < 32) {
+    const unsigned long long p = tile_lookback(J.status, tile, total, J.err);
+    if (threadIdx.x == 0) s_prefix = p;
+  }
+  __syncthreads();
+  if (tile == gridDim.x - 1 && threadIdx.x == 0) *J.total = s_prefix + total;
+  unsigned long long pos = s_prefix + before;
+  if (count == 0 || pos >= J.capacity) return;  // nothing of this warp is stored
+  const uint32_t lt = lanemask_lt();
+  sweep([&](uint32_t bal, bool m, uint32_t l, uint32_t r) {
+    if (m) emit_pair(J, pos + __popc(bal & lt), l, r);
+    pos += __popc(bal);
+  });
+}
+
+// Left rows a block of the sorted join takes: few enough that four blocks an SM
+// have some, as one row may have any number of matches.
+static uint32_t sorted_tile_rows(uint32_t L, bool eq_only) {
+  const uint32_t most = eq_only ? kJoinTile : kJoinBlock, rows = ceil_div<uint32_t>(L, (uint32_t)sm_count() * 4u);
+  return rows < 1u ? 1u : (rows < most ? rows : most);
 }
 
 // ------------------------------------------------------------ nested loop
@@ -1375,7 +1430,8 @@ static int join_impl(const yq_batch* left, const yq_batch* right, const yq_join_
                        !t0.r.nulls && t0.l.width == t0.r.width && t0.cmp != YQ_EQ &&
                        (t0.l.type == YQ_INT32 || t0.l.type == YQ_FLOAT32 || t0.l.type == YQ_INT64 ||
                         t0.l.type == YQ_DATETIME || t0.l.type == YQ_FLOAT64);
-    ntiles = ceil_div<uint32_t>(J.L, use_hash || use_sorted ? kJoinTile : (typed ? kNtTile : kNlTile));
+    const uint32_t tile_rows = use_sorted ? sorted_tile_rows(J.L, J.ncond == 1) : (use_hash ? kJoinTile : (typed ? kNtTile : kNlTile));
+    ntiles = ceil_div<uint32_t>(J.L, tile_rows);
     count_bytes = typed && counts_first(J.L, J.R) ? join_sort_bytes(J.R, false) : 0;
     count_first = count_bytes != 0;  // else (a right side too long to sort) the kernel counts
     WsSize w;
@@ -1435,6 +1491,7 @@ static int join_impl(const yq_batch* left, const yq_batch* right, const yq_join_
     S.perm = perm;
     S.rows = J.R;
     S.nslots = sorted_slots(J.R);
+    S.tile_rows = sorted_tile_rows(J.L, J.ncond == 1);
     S.slots = ws.take<uint4>(S.nslots);
     const yq_column rc{const_cast<char*>(ec.r.data), ec.r.nulls, ec.r.type, ec.r.width};
     KeyJob j{rc, 0, 0};
@@ -1455,8 +1512,8 @@ static int join_impl(const yq_batch* left, const yq_batch* right, const yq_join_
       YQ_CHECK_LAUNCH();
     }
     ProfScope ps("join_sorted_probe", s, (double)J.L * ec.l.width);
-    if (J.ncond == 1) k_join_sorted<true><<<ntiles, kJoinBlock, 0, s>>>(J, S);
-    else k_join_sorted<false><<<ntiles, kJoinBlock, 0, s>>>(J, S);
+    if (J.ncond == 1) k_join_sorted<<<ntiles, kJoinBlock, 0, s>>>(J, S);
+    else k_join_sorted_conds<<<ntiles, kJoinBlock, 0, s>>>(J, S);
     YQ_CHECK_LAUNCH();
   } else {
     ProfScope ps("join_nested_loop", s, (double)J.L * J.R * 0.0);
@@ -1503,7 +1560,11 @@ extern "C" {
 
 size_t yq_join_workspace_size(uint32_t left_rows, uint32_t right_rows) {
   const uint32_t nb = pow2_at_least(right_rows);
-  const uint32_t ntiles = ceil_div<uint32_t>(left_rows, kNtTile < kNlTile ? kNtTile : kNlTile);
+  uint32_t ntiles = ceil_div<uint32_t>(left_rows, kNtTile < kNlTile ? kNtTile : kNlTile);
+  for (const bool eq_only : {false, true}) {
+    const uint32_t sorted = ceil_div<uint32_t>(left_rows, sorted_tile_rows(left_rows, eq_only));
+    if (sorted > ntiles) ntiles = sorted;
+  }
   WsSize w;
   w.add<uint32_t>(nb + 1);
   w.add<unsigned long long>(right_rows ? right_rows : 1);
