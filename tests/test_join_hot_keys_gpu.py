@@ -69,3 +69,22 @@ def test_one_key_and_a_condition_takes_no_longer_than_the_nested_loop(cuda, yq, 
             assert (st, n.value) == (A.OK, 0)
             ms[name] = min(ms.get(name, 1e9), a.elapsed_time(b))
     assert ms["sorted"] < 1.5 * ms["nested"], ms
+
+
+def test_a_row_with_millions_of_matches(cuda):
+    """More pairs in a tile than its 32-bit offsets hold: three left rows, one of
+    them without a match, to 1.5M right rows of two keys."""
+    rows = 1_500_000
+    rk = (torch.arange(rows, device="cuda", dtype=torch.int32) % 5 == 0).int()  # 1 for every fifth row
+    rv = torch.arange(rows, device="cuda", dtype=torch.int32)
+    lk = torch.tensor([0, 9, 0, 1], device="cuda", dtype=torch.int32)
+    lb = ops.DeviceBatch([ops.DeviceColumn(lk, A.INT32), ops.DeviceColumn(lk * 100, A.INT32)])
+    rb = ops.DeviceBatch([ops.DeviceColumn(rk, A.INT32), ops.DeviceColumn(rv, A.INT32)])
+    zero, one = (rk == 0).nonzero().flatten().int(), (rk == 1).nonzero().flatten().int()
+    wl = torch.cat([torch.full_like(zero, 0), torch.full_like(zero, 2), torch.full_like(one, 3)])
+    wr = torch.cat([zero, zero, one])
+    gl, gr = ops.join_pairs(lb, rb, [(0, 0, A.EQ)], capacity=len(wl))
+    assert torch.equal(gl, wl) and torch.equal(gr, wr)
+    out = ops.join_project(lb, rb, [(0, 0, A.EQ)], [(1, 1), (0, 1)], capacity=len(wl))
+    assert torch.equal(out.columns[0].data, rv[wr.long()])
+    assert torch.equal(out.columns[1].data, (lk * 100)[wl.long()])

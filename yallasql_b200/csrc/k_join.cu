@@ -513,12 +513,12 @@ __global__ void __launch_bounds__(kJoinBlock) k_join_sorted(const __grid_constan
   __shared__ unsigned long long s_prefix;
   __shared__ uint32_t s_off[kJoinTile + 1];
   __shared__ uint32_t s_first[kJoinTile];
-  __shared__ uint32_t s_l[kSortedChunk], s_r[kSortedChunk];
+  __shared__ __align__(8) uint32_t s_l[kSortedChunk];
+  __shared__ uint32_t s_r[kSortedChunk];
   if (threadIdx.x == 0) s_tile = atomicAdd(J.tile_counter, 1u);
   __syncthreads();
   const uint32_t tile = s_tile;
   const uint32_t base = tile * S.tile_rows, end = min(J.L, base + S.tile_rows);
-  const int lane = threadIdx.x & 31;
   uint32_t first[kJoinItems], run[kJoinItems], sum = 0;
   sorted_matches<kJoinItems>(S, J.cond[J.eq].l, base + threadIdx.x * kJoinItems, end, first, run);
   unsigned long long wide = 0;  // the tile's pairs may exceed 32 bits (a hot key on both sides)
@@ -589,20 +589,28 @@ __global__ void __launch_bounds__(kJoinBlock) k_join_sorted(const __grid_constan
     }
     return;
   }
-  unsigned long long pos = prefix + excl;
-#pragma unroll 1
+  // A tile of more pairs than 32 bits count: the same by 64-bit offsets, pair by
+  // pair (one row with 3M matches, two columns written: 12 ms; 92 when a warp
+  // wrote each such row).
+  static_assert(kJoinTile * 8 <= sizeof(s_l), "64-bit offsets in the place of the chunk's left rows");
+  unsigned long long* const s_wide_off = reinterpret_cast<unsigned long long*>(s_l);
+  unsigned long long at = excl;
+#pragma unroll
   for (int k = 0; k < kJoinItems; ++k) {
-    const uint32_t l = base + threadIdx.x * kJoinItems + k;
-    if (run[k] <= 32)
-      for (uint32_t x = 0; x < run[k]; ++x) emit_pair(J, pos++, l, match_row(S, first[k], x));
-    for (uint32_t todo = __ballot_sync(0xffffffffu, run[k] > 32); todo; todo &= todo - 1) {
-      const int src = __ffs(todo) - 1;
-      const uint32_t n = __shfl_sync(0xffffffffu, run[k], src), f = __shfl_sync(0xffffffffu, first[k], src);
-      const uint32_t wl = __shfl_sync(0xffffffffu, l, src);
-      const unsigned long long wp = __shfl_sync(0xffffffffu, pos, src);
-      for (uint32_t x = lane; x < n; x += 32) emit_pair(J, wp + x, wl, match_row(S, f, x));
-      if (lane == src) pos = wp + n;
+    s_wide_off[threadIdx.x * kJoinItems + k] = at;
+    s_first[threadIdx.x * kJoinItems + k] = first[k];
+    at += run[k];
+  }
+  __syncthreads();
+  const unsigned long long n_out = min(total, J.capacity - prefix);
+  for (unsigned long long i = threadIdx.x; i < n_out; i += kJoinBlock) {
+    uint32_t lo = 0, hi = S.tile_rows;
+    while (lo + 1 < hi) {
+      const uint32_t mid = (lo + hi) >> 1;
+      if (s_wide_off[mid] <= i) lo = mid;
+      else hi = mid;
     }
+    emit_pair(J, prefix + i, base + lo, match_row(S, s_first[lo], (uint32_t)(i - s_wide_off[lo])));
   }
 }
 
