@@ -85,3 +85,27 @@ def test_room_for_a_part(cuda, yq, room, first):
         assert np.array_equal(host[:room], b[rows]) and (host[room:] == 0x5a).all(), (s, c)
         nb = nul.cpu().numpy()
         assert not nb[:room].any() and (nb[room:] == 0x5a).all()
+
+
+@pytest.mark.parametrize("kind", [A.INT32, A.FLOAT32, A.INT64, A.FLOAT64])
+@pytest.mark.parametrize("L,R", [(1, 1), (255, 24), (257, 25), (5000, 5), (150_001, 3), (40_000, 33), (200_003, 40), (410_001, 26)])
+def test_few_right_rows(cuda, kind, L, R):
+    """Right sides around the 24 rows up to which every right row is a candidate
+    of every left row (NaN meets nothing but under <>, -0.0 equals 0.0)."""
+    rng = np.random.default_rng(L + R + kind)
+    dt = {A.INT32: np.int32, A.FLOAT32: np.float32, A.INT64: np.int64, A.FLOAT64: np.float64}[kind]
+    x, y = rng.integers(-40, 40, L).astype(dt), rng.integers(-40, 40, R).astype(dt)
+    if kind in (A.FLOAT32, A.FLOAT64):
+        x[::7], y[::5] = np.nan, -0.0
+    wide = rng.integers(0, 256, (L, 20), dtype=np.uint8)
+    dev = lambda v, t: ops.DeviceColumn(torch.from_numpy(np.ascontiguousarray(v)).cuda(), t)
+    lb = ops.DeviceBatch([dev(x, kind), dev(wide, A.TEXT)])
+    rb = ops.DeviceBatch([dev(y, kind), dev(np.arange(R, dtype=np.int64), A.INT64)])
+    for cmp, f in ((A.LT, np.less), (A.LE, np.less_equal), (A.GT, np.greater), (A.GE, np.greater_equal),
+                   (A.NE, np.not_equal)):
+        wl, wr = np.nonzero(f(x[:, None], y[None, :]))
+        gl, gr = ops.join_pairs(lb, rb, [(0, 0, cmp)], capacity=max(1, len(wl)))
+        assert np.array_equal(gl.cpu().numpy(), wl) and np.array_equal(gr.cpu().numpy(), wr), cmp
+        out = ops.join_project(lb, rb, [(0, 0, cmp)], [(0, 1), (1, 1)], capacity=max(1, len(wl)))
+        assert np.array_equal(out.columns[0].data.cpu().numpy(), wide[wl]) and \
+            np.array_equal(out.columns[1].data.cpu().numpy(), wr), cmp

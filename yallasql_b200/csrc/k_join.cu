@@ -621,8 +621,14 @@ __global__ void __launch_bounds__(kJoinBlock) k_join_sorted(const __grid_constan
 // 20,000 right ones of one key and two more conditions took 246 ms with a warp
 // going through the long runs of its 128 left rows one after the other, 9.4 in
 // the nested loop.
-__global__ void __launch_bounds__(kJoinBlock) k_join_sorted_conds(const __grid_constant__ JoinParams J,
-                                                                  const __grid_constant__ SortedJoin S) {
+// ALL: no equality and a right side of a few rows, every one of which is a
+// candidate of every left row. (A block of the typed nested loop takes 16 left
+// rows, and its counter, look-back and waits are most of its work then: 1M left
+// rows to 5 right ones under <, pairs, 980 us there and 127 here; to 20, 978 and
+// 269; 40,000 to 60, four columns, 101 and 94, but its own two columns 62 and 77.)
+template <bool ALL>
+__global__ void __launch_bounds__(kJoinBlock) k_join_candidates(const __grid_constant__ JoinParams J,
+                                                                const __grid_constant__ SortedJoin S) {
   constexpr int NW = kJoinBlock / 32;
   __shared__ uint32_t s_tile;
   __shared__ unsigned long long s_off[kJoinBlock + 1];  // first candidate of every left row
@@ -636,7 +642,9 @@ __global__ void __launch_bounds__(kJoinBlock) k_join_sorted_conds(const __grid_c
   const uint32_t base = tile * S.tile_rows, end = min(J.L, base + S.tile_rows);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   unsigned long long candidates;
-  {
+  if constexpr (ALL) {
+    candidates = (unsigned long long)(end - base) * J.R;
+  } else {
     uint32_t where[1], run[1];
     sorted_matches<1>(S, J.cond[J.eq].l, base + threadIdx.x, end, where, run);
     unsigned long long first = run[0], zero = 0, tz;
@@ -661,14 +669,21 @@ __global__ void __launch_bounds__(kJoinBlock) k_join_sorted_conds(const __grid_c
   // f(matches of 32 candidates, left row, right row), in order
   auto sweep = [&](auto f) {
     if (x0 >= x1) return;
-    uint32_t row = row_of(x0, 0u);
+    uint32_t row = ALL ? 0u : row_of(x0, 0u);
     for (unsigned long long x = x0; x < x1; x += 32) {
       const unsigned long long mine = min(x + lane, x1 - 1), last = min(x + 31, x1 - 1);
-      const uint32_t at = last < s_off[row + 1] ? row : row_of(mine, row);
-      const uint32_t l = base + at, r = match_row(S, s_where[at], (uint32_t)(mine - s_off[at]));
+      uint32_t at, r;
+      if constexpr (ALL) {  // (at most kJoinBlock * kSmallRight candidates)
+        at = (uint32_t)mine / J.R;
+        r = (uint32_t)mine - at * J.R;
+      } else {
+        at = last < s_off[row + 1] ? row : row_of(mine, row);
+        r = match_row(S, s_where[at], (uint32_t)(mine - s_off[at]));
+      }
+      const uint32_t l = base + at;
       const bool m = x + lane < x1 && all_conds(J, l, r, J.eq);
       f(__ballot_sync(0xffffffffu, m), m, l, r);
-      row = __shfl_sync(0xffffffffu, at, 31);
+      if constexpr (!ALL) row = __shfl_sync(0xffffffffu, at, 31);
     }
   };
   unsigned long long count = 0;
@@ -695,6 +710,8 @@ __global__ void __launch_bounds__(kJoinBlock) k_join_sorted_conds(const __grid_c
     pos += __popc(bal);
   });
 }
+
+constexpr uint32_t kSmallRight = 24;  // right rows up to which all of them are candidates
 
 // Left rows a block of the sorted join takes: few enough that four blocks an SM
 // have some, as one row may have any number of matches.
@@ -1427,7 +1444,7 @@ static int join_impl(const yq_batch* left, const yq_batch* right, const yq_join_
   const size_t eq_sort_bytes = J.eq >= 0 && J.R > table_rows && J.cond[J.eq].r.type != YQ_BOOL
                                    ? join_sort_bytes(J.R, J.cond[J.eq].r.nulls != nullptr) : 0;
   const JCond& t0 = J.cond[0];
-  bool use_sorted = eq_sort_bytes != 0, use_hash, typed, count_first;
+  bool use_sorted = eq_sort_bytes != 0, use_hash, typed, small, count_first;
   uint32_t nbuckets, ntiles;
   size_t count_bytes;
   Workspace ws;
@@ -1438,7 +1455,11 @@ static int join_impl(const yq_batch* left, const yq_batch* right, const yq_join_
                        !t0.r.nulls && t0.l.width == t0.r.width && t0.cmp != YQ_EQ &&
                        (t0.l.type == YQ_INT32 || t0.l.type == YQ_FLOAT32 || t0.l.type == YQ_INT64 ||
                         t0.l.type == YQ_DATETIME || t0.l.type == YQ_FLOAT64);
-    const uint32_t tile_rows = use_sorted ? sorted_tile_rows(J.L, J.ncond == 1) : (use_hash ? kJoinTile : (typed ? kNtTile : kNlTile));
+    small = typed && J.R <= kSmallRight;
+    const uint32_t tile_rows = use_sorted ? sorted_tile_rows(J.L, J.ncond == 1)
+                               : use_hash ? kJoinTile
+                               : small    ? sorted_tile_rows(J.L, false)
+                               : typed    ? kNtTile : kNlTile;
     ntiles = ceil_div<uint32_t>(J.L, tile_rows);
     count_bytes = typed && counts_first(J.L, J.R) ? join_sort_bytes(J.R, false) : 0;
     count_first = count_bytes != 0;  // else (a right side too long to sort) the kernel counts
@@ -1521,12 +1542,17 @@ static int join_impl(const yq_batch* left, const yq_batch* right, const yq_join_
     }
     ProfScope ps("join_sorted_probe", s, (double)J.L * ec.l.width);
     if (J.ncond == 1) k_join_sorted<<<ntiles, kJoinBlock, 0, s>>>(J, S);
-    else k_join_sorted_conds<<<ntiles, kJoinBlock, 0, s>>>(J, S);
+    else k_join_candidates<false><<<ntiles, kJoinBlock, 0, s>>>(J, S);
     YQ_CHECK_LAUNCH();
   } else {
     ProfScope ps("join_nested_loop", s, (double)J.L * J.R * 0.0);
     const JCond& c0 = J.cond[0];
-    if (typed) {
+    if (small) {
+      SortedJoin S{};
+      S.rows = J.R;
+      S.tile_rows = sorted_tile_rows(J.L, false);
+      k_join_candidates<true><<<ntiles, kJoinBlock, 0, s>>>(J, S);
+    } else if (typed) {
       if (count_first) {
         switch (c0.l.type) {
           case YQ_INT32: YQ_TRY(count_matches_typed<int32_t>(J, cw, s)); break;
