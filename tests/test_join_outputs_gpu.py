@@ -88,21 +88,28 @@ def test_room_for_a_part(cuda, yq, room, first):
 
 
 @pytest.mark.parametrize("kind", [A.INT32, A.FLOAT32, A.INT64, A.FLOAT64])
-@pytest.mark.parametrize("L,R", [(1, 1), (255, 24), (257, 25), (5000, 5), (150_001, 3), (40_000, 33), (200_003, 40), (410_001, 26)])
+@pytest.mark.parametrize("L,R", [(1, 1), (255, 40), (257, 41), (5000, 5), (150_001, 3), (40_000, 33), (200_003, 40), (499_999, 41), (500_000, 72),
+                                 (500_001, 73)])
 def test_few_right_rows(cuda, kind, L, R):
-    """Right sides around the 24 rows up to which every right row is a candidate
-    of every left row (NaN meets nothing but under <>, -0.0 equals 0.0)."""
+    """Right sides around the 40 rows (72 from 500,000 left rows on) up to which
+    every right row is a candidate of every left row (NaN meets nothing but under
+    <>, -0.0 equals 0.0)."""
     rng = np.random.default_rng(L + R + kind)
     dt = {A.INT32: np.int32, A.FLOAT32: np.float32, A.INT64: np.int64, A.FLOAT64: np.float64}[kind]
     x, y = rng.integers(-40, 40, L).astype(dt), rng.integers(-40, 40, R).astype(dt)
+    if L * R > 10_000_000:  # few pairs
+        x[:] = 39
+        x[::1000] = rng.integers(-40, 40, len(x[::1000]))
+        y[:] = 39
+        y[::9] = 38
     if kind in (A.FLOAT32, A.FLOAT64):
         x[::7], y[::5] = np.nan, -0.0
     wide = rng.integers(0, 256, (L, 20), dtype=np.uint8)
     dev = lambda v, t: ops.DeviceColumn(torch.from_numpy(np.ascontiguousarray(v)).cuda(), t)
     lb = ops.DeviceBatch([dev(x, kind), dev(wide, A.TEXT)])
     rb = ops.DeviceBatch([dev(y, kind), dev(np.arange(R, dtype=np.int64), A.INT64)])
-    for cmp, f in ((A.LT, np.less), (A.LE, np.less_equal), (A.GT, np.greater), (A.GE, np.greater_equal),
-                   (A.NE, np.not_equal)):
+    few = ((A.LT, np.less), (A.GT, np.greater), (A.NE, np.not_equal))
+    for cmp, f in few if L * R > 10_000_000 else few + ((A.LE, np.less_equal), (A.GE, np.greater_equal)):
         wl, wr = np.nonzero(f(x[:, None], y[None, :]))
         gl, gr = ops.join_pairs(lb, rb, [(0, 0, cmp)], capacity=max(1, len(wl)))
         assert np.array_equal(gl.cpu().numpy(), wl) and np.array_equal(gr.cpu().numpy(), wr), cmp

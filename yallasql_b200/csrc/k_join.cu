@@ -614,6 +614,12 @@ __global__ void __launch_bounds__(kJoinBlock) k_join_sorted(const __grid_constan
   }
 }
 
+// Right rows up to which all of them are candidates of every left row (below), and
+// the same with very many left rows. The general comparison costs more than the
+// typed one from there on: 200,000 x 66 rows, the condition's columns, 215 us
+// against 157; 1M x 66, pairs, 488 against 1,008; 1M x 250, 1,432 against 890.
+constexpr uint32_t kSmallRight = 40, kSmallRightMany = 72, kManyLeft = 500000;
+
 // With further conditions the rows of a key's run are candidates. A block's
 // candidates form one sequence (left row by left row, right rows ascending, the
 // order of the output), cut into eight equal parts for its warps, so that a key
@@ -624,8 +630,8 @@ __global__ void __launch_bounds__(kJoinBlock) k_join_sorted(const __grid_constan
 // ALL: no equality and a right side of a few rows, every one of which is a
 // candidate of every left row. (A block of the typed nested loop takes 16 left
 // rows, and its counter, look-back and waits are most of its work then: 1M left
-// rows to 5 right ones under <, pairs, 980 us there and 127 here; to 20, 978 and
-// 269; 40,000 to 60, four columns, 101 and 94, but its own two columns 62 and 77.)
+// rows to 5 right ones under <, pairs, 980 us there and 112 here.) Which of them
+// match is kept as bits for the second sweep (1M x 24 rows: 246 us, 320 without).
 template <bool ALL>
 __global__ void __launch_bounds__(kJoinBlock) k_join_candidates(const __grid_constant__ JoinParams J,
                                                                 const __grid_constant__ SortedJoin S) {
@@ -636,6 +642,7 @@ __global__ void __launch_bounds__(kJoinBlock) k_join_candidates(const __grid_con
   __shared__ unsigned long long s_scan[2 * (NW + 1)];
   __shared__ unsigned long long s_cnt[NW];
   __shared__ unsigned long long s_prefix;
+  __shared__ uint32_t s_bits[ALL ? kJoinBlock * kSmallRightMany / 32 : 1];  // which candidates match
   if (threadIdx.x == 0) s_tile = atomicAdd(J.tile_counter, 1u);
   __syncthreads();
   const uint32_t tile = s_tile;
@@ -666,28 +673,40 @@ __global__ void __launch_bounds__(kJoinBlock) k_join_candidates(const __grid_con
     }
     return lo;
   };
-  // f(matches of 32 candidates, left row, right row), in order
+  // f(candidates, left row, right row, whether this lane has one), 32 at a time in order
   auto sweep = [&](auto f) {
-    if (x0 >= x1) return;
-    uint32_t row = ALL ? 0u : row_of(x0, 0u);
-    for (unsigned long long x = x0; x < x1; x += 32) {
-      const unsigned long long mine = min(x + lane, x1 - 1), last = min(x + 31, x1 - 1);
-      uint32_t at, r;
-      if constexpr (ALL) {  // (at most kJoinBlock * kSmallRight candidates)
-        at = (uint32_t)mine / J.R;
-        r = (uint32_t)mine - at * J.R;
-      } else {
-        at = last < s_off[row + 1] ? row : row_of(mine, row);
-        r = match_row(S, s_where[at], (uint32_t)(mine - s_off[at]));
+    if constexpr (ALL) {
+      uint32_t at = ((uint32_t)x0 + lane) / J.R, r = (uint32_t)x0 + lane - at * J.R;
+      for (uint32_t x = (uint32_t)x0; x < (uint32_t)x1; x += 32) {
+        f(x, base + at, r, x + lane < (uint32_t)x1);
+        if (J.R >= 32u) {
+          r += 32u;
+          if (r >= J.R) {
+            r -= J.R;
+            ++at;
+          }
+        } else {
+          at = (x + 32u + lane) / J.R;
+          r = x + 32u + lane - at * J.R;
+        }
       }
-      const uint32_t l = base + at;
-      const bool m = x + lane < x1 && all_conds(J, l, r, J.eq);
-      f(__ballot_sync(0xffffffffu, m), m, l, r);
-      if constexpr (!ALL) row = __shfl_sync(0xffffffffu, at, 31);
+    } else {
+      if (x0 >= x1) return;
+      uint32_t row = row_of(x0, 0u);
+      for (unsigned long long x = x0; x < x1; x += 32) {
+        const unsigned long long mine = min(x + lane, x1 - 1), last = min(x + 31, x1 - 1);
+        const uint32_t at = last < s_off[row + 1] ? row : row_of(mine, row);
+        f(0u, base + at, match_row(S, s_where[at], (uint32_t)(mine - s_off[at])), x + lane < x1);
+        row = __shfl_sync(0xffffffffu, at, 31);
+      }
     }
   };
   unsigned long long count = 0;
-  sweep([&](uint32_t bal, bool, uint32_t, uint32_t) { count += __popc(bal); });
+  sweep([&](uint32_t x, uint32_t l, uint32_t r, bool in) {
+    const uint32_t bal = __ballot_sync(0xffffffffu, in && all_conds(J, l, r, J.eq));
+    if (ALL && lane == 0) s_bits[x >> 5] = bal;  // kept for the second sweep
+    count += __popc(bal);
+  });
   if (lane == 0) s_cnt[warp] = count;
   __syncthreads();
   unsigned long long total = 0, before = 0;
@@ -705,13 +724,13 @@ __global__ void __launch_bounds__(kJoinBlock) k_join_candidates(const __grid_con
   unsigned long long pos = s_prefix + before;
   if (count == 0 || pos >= J.capacity) return;  // nothing of this warp is stored
   const uint32_t lt = lanemask_lt();
-  sweep([&](uint32_t bal, bool m, uint32_t l, uint32_t r) {
-    if (m) emit_pair(J, pos + __popc(bal & lt), l, r);
+  sweep([&](uint32_t x, uint32_t l, uint32_t r, bool in) {
+    const uint32_t bal = ALL ? s_bits[x >> 5] : __ballot_sync(0xffffffffu, in && all_conds(J, l, r, J.eq));
+    if (bal >> lane & 1u) emit_pair(J, pos + __popc(bal & lt), l, r);
     pos += __popc(bal);
   });
 }
 
-constexpr uint32_t kSmallRight = 24;  // right rows up to which all of them are candidates
 
 // Left rows a block of the sorted join takes: few enough that four blocks an SM
 // have some, as one row may have any number of matches.
@@ -1455,7 +1474,7 @@ static int join_impl(const yq_batch* left, const yq_batch* right, const yq_join_
                        !t0.r.nulls && t0.l.width == t0.r.width && t0.cmp != YQ_EQ &&
                        (t0.l.type == YQ_INT32 || t0.l.type == YQ_FLOAT32 || t0.l.type == YQ_INT64 ||
                         t0.l.type == YQ_DATETIME || t0.l.type == YQ_FLOAT64);
-    small = typed && J.R <= kSmallRight;
+    small = typed && J.R <= (J.L >= kManyLeft ? kSmallRightMany : kSmallRight);
     const uint32_t tile_rows = use_sorted ? sorted_tile_rows(J.L, J.ncond == 1)
                                : use_hash ? kJoinTile
                                : small    ? sorted_tile_rows(J.L, false)
